@@ -195,8 +195,6 @@ static int ctx_create(int device, bool use_given_stream, void *stream, fnn_cuda_
     if (e == cudaSuccess) e = cudaMemset(ctx->err_flag, 0, 2 * sizeof(int));
     if (e == cudaSuccess) e = cudaHostAlloc((void **)&ctx->err_host, sizeof(int), cudaHostAllocDefault);
     if (e == cudaSuccess) *ctx->err_host = 0;
-    if (e == cudaSuccess) e = cudaMalloc((void **)&ctx->sk_flags, 2048 * sizeof(unsigned));
-    if (e == cudaSuccess) e = cudaMemset(ctx->sk_flags, 0, 2048 * sizeof(unsigned));
     if (e != cudaSuccess) {
         if (ctx->owns_stream) cudaStreamDestroy(ctx->stream);
         delete ctx;
@@ -233,7 +231,6 @@ int fnn_cuda_ctx_destroy(fnn_cuda_ctx *ctx) {
     for (void *p : ctx->retired_scratch) cudaFree(p);
     if (ctx->err_flag) cudaFree(ctx->err_flag);
     if (ctx->err_host) cudaFreeHost(ctx->err_host);
-    if (ctx->sk_flags) cudaFree(ctx->sk_flags);
     if (ctx->owns_stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
     return FNN_OK;

@@ -68,7 +68,6 @@ struct fnn_cuda_ctx {
                               // the fused GEMM + all-gather
     int *err_host = nullptr;  // pinned host copy of err_flag[0], refreshed by fnn_cuda_sync
     bool overlap_launches = true;   // programmatic dependent launch (fnn_cuda_ctx_set_overlap)
-    unsigned *sk_flags = nullptr;   // 2 x 1024 zeroed counters of the tcgen05 kernel's split-K hand-over
 };
 
 struct fnn_cuda_arena {
@@ -222,6 +221,26 @@ inline cudaError_t launch_pdl(void (*kern)(KArgs...), int grid, int block, size_
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = ctx->overlap_launches ? 1 : 0;   // without it every kernel waits for the one before it
+    return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
+}
+// The same with thread-block clusters of `cluster` consecutive blocks.
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_pdl_cluster(void (*kern)(KArgs...), int grid, int cluster, int block, size_t smem,
+                                      const fnn_cuda_ctx *ctx, Args &&...args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = ctx->stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)cluster;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = ctx->overlap_launches ? 2 : 1;
     return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
 }
 #endif
