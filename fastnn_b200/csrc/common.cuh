@@ -398,6 +398,17 @@ int prepare_qmm_tc(fnn_cuda_ctx *ctx, fnn_cuda_qweight *w);
 static inline bool auto_uses_mma(const fnn_cuda_qweight *w) { return w->K >= 512 && w->N >= 64; }
 bool qmm_tc_supported(const fnn_cuda_qweight *w, size_t M);
 int launch_qmm_tc(fnn_cuda_ctx *ctx, const QmmArgs &args);
+// large batches: two SMs per tile
+struct PairTiling {
+    int Mb = 0, m_tiles = 0;   // batch rows per tile, tiles over the batch
+    int terms = 0;             // narrow terms per activation
+    bool sum = false;          // the terms accumulate into the same columns
+    double cost = 0;           // estimated microseconds of the main loops and the last epilogue
+};
+PairTiling pair_tiling(int fmt, int M, int N, int K, int sm_count);
+double tc_single_cost(const fnn_cuda_ctx *ctx, const fnn_cuda_qweight *w, size_t M);   // of the single-SM kernel
+bool qmm_tc_uses_pair(const fnn_cuda_ctx *ctx, const fnn_cuda_qweight *w, size_t M);
+int launch_qmm_tc_pair(fnn_cuda_ctx *ctx, const QmmArgs &args);
 void free_qweight_aux(fnn_cuda_qweight *w);
 
 int ensure_scratch(fnn_cuda_ctx *ctx, size_t bytes);

@@ -798,23 +798,27 @@ namespace {
 // A cluster lives inside one GPC, so fewer of the larger ones run at once (74, 45, 33, 26, 22 of 2 .. 6 on a
 // B200, and only 15 of 8); a cluster that has to wait for a second round costs more than the split gains
 // (48 tiles in 3 parts: 19.9 us against 11.8 in 2).
-int split_parts(const fnn_cuda_ctx *ctx, int tiles, int kblocks, int cols, int wf) {
+struct Split {
+    int parts;
+    double cost;   // estimated microseconds of the main loops
+};
+Split split_parts(const fnn_cuda_ctx *ctx, int tiles, int kblocks, int cols, int wf) {
     static const int kActive[] = {0, 148, 74, 45, 33, 26, 22};   // of 148 SMs
     const double t_step = (wf == WF_CB) ? 0.8 : 0.15 + 0.25 * cols / 256.0;
     const double t_part = 0.8 + 0.4 * cols / 128.0;
-    int best = 1;
-    double best_cost = kblocks * t_step;
+    const int waves = (tiles + ctx->sm_count - 1) / ctx->sm_count;
+    Split best{1, waves * kblocks * t_step};
     for (int q = 2; q <= 6 && q <= kblocks; ++q) {
         if (tiles > kActive[q] * ctx->sm_count / 148) break;
         const bool crowded = 4 * tiles * q > 3 * ctx->sm_count;
         const double cost = (kblocks + q - 1) / q * t_step + t_part * (q - 1) + (crowded ? 1.5 : 0.0);
-        if (cost < best_cost) {
-            best_cost = cost;
-            best = q;
-        }
+        if (cost < best.cost) best = {q, cost};
     }
     return best;
 }
+
+// batch rows per tile: T * Mb is the MMA N (multiple of 16, at most 256)
+int batch_rows(int terms, int M) { return std::min(terms == 1 ? 256 : terms == 2 ? 128 : 80, (M + 15) & ~15); }
 
 // Scratch of one call: the rewritten activations Bq[T][Mpad][Kp], then dq[Mpad] and rowsum[Mpad].
 // `fixed_scratch` null: the context's growable buffer; otherwise a caller-supplied region of
@@ -827,9 +831,7 @@ int launch_tc(fnn_cuda_ctx *ctx, const QmmArgs &a, uint8_t *fixed_scratch = null
     const int M = (int)a.M, N = (int)w->N, K = (int)w->K;
     const int Kbytes = K * ES;
     const int Kp = (Kbytes + 15) & ~15;  // row bytes; TMA strides are multiples of 16 bytes
-    // batch rows per tile: T*Mb is the MMA N (multiple of 16, at most 256)
-    const int mb_max = (T == 1) ? 256 : (T == 2) ? 128 : 80;
-    int Mb = std::min(mb_max, (M + 15) & ~15);
+    const int Mb = batch_rows(T, M);
     const int m_tiles = (M + Mb - 1) / Mb;
     const int Mpad = m_tiles * Mb;
 
@@ -839,7 +841,7 @@ int launch_tc(fnn_cuda_ctx *ctx, const QmmArgs &a, uint8_t *fixed_scratch = null
     const int n_tiles = (N + kTileN - 1) / kTileN;
     const int kblocks = (Kbytes + kKBlockBytes * ATOMS - 1) / (kKBlockBytes * ATOMS);
     const int tiles = n_tiles * m_tiles;
-    const int parts = split_parts(ctx, tiles, kblocks, T * Mb, WF);
+    const int parts = split_parts(ctx, tiles, kblocks, T * Mb, WF).parts;
     int rc = FNN_OK;
     uint8_t *bq;
     if (fixed_scratch) {
@@ -930,6 +932,13 @@ int launch_tc(fnn_cuda_ctx *ctx, const QmmArgs &a, uint8_t *fixed_scratch = null
 
 int dispatch_tc(fnn_cuda_ctx *ctx, const QmmArgs &a, uint8_t *fixed, size_t fixed_bytes);
 
+double tc_single_cost(const fnn_cuda_ctx *ctx, const fnn_cuda_qweight *w, size_t M) {
+    const bool cb = w->fmt == FNN_FMT_I4CB, f8 = w->fmt == FNN_FMT_F8 || w->fmt == FNN_FMT_F4;
+    const int terms = cb ? 1 : f8 && M < 128 ? 3 : 2, Mb = batch_rows(terms, (int)M);
+    const int tiles = (int)(div_ceil(w->N, (size_t)kTileN) * div_ceil(M, (size_t)Mb));
+    return split_parts(ctx, tiles, (int)div_ceil(w->K, (size_t)kKBlockBytes), terms * Mb, cb ? WF_CB : WF_TMA).cost;
+}
+
 bool qmm_tc_supported(const fnn_cuda_qweight *w, size_t M) {
     (void)M;
     // I8 / FP8 / FP4 codes are operands as stored; I4 and the codebook format are widened in shared
@@ -963,6 +972,7 @@ int dispatch_tc(fnn_cuda_ctx *ctx, const QmmArgs &a, uint8_t *fixed, size_t fixe
 
 int launch_qmm_tc(fnn_cuda_ctx *ctx, const QmmArgs &a) {
     FNN_REQUIRE(a.M < (1u << 24), FNN_ERR_DISPATCH, "qmatmul: M=%zu too large for the tcgen05 path", a.M);
+    if (!a.allgather && qmm_tc_uses_pair(ctx, a.w, a.M)) return launch_qmm_tc_pair(ctx, a);
     return dispatch_tc(ctx, a, nullptr, 0);
 }
 

@@ -1,0 +1,545 @@
+// tcgen05 kernel for large batches: two SMs of a cluster work on one tile (cta_group::2).
+//
+// Bound by the tensor pipe.  A single-SM tile of 128 output channels x 256 accumulator columns moves
+// 16 KB of weights and 32 KB of activations through L2 and shared memory for every 512 cycles of
+// MMA (94 B per cycle and SM, 27 TB/s over the chip at the full 8-bit rate), which L2 cannot feed.  Here the
+// pair computes 256 channels: each SM holds its own 128 weight rows and half of the activation tile,
+// and the tensor cores of both read both halves, so the activation traffic of an SM halves.
+//
+// Two forms, by how the narrow activation terms (see qmm_tc.cu) meet:
+//   SUM   (FP8, FP4: two e4m3 terms of the same scale) both terms accumulate into the same columns, two MMAs
+//         per K step: a tile is 256 channels x up to 256 batch rows and the weight tile is read once
+//         for both terms (48 B per cycle and SM)
+//   !SUM  (I8, I4: hi and lo bytes, whose int32 sums have different weights; codebook: one fp16 term)
+//         one MMA over the (term, batch row) columns; for two terms the first SM holds the hi plane
+//         and the second the lo plane of 128 batch rows (64 B per cycle and SM)
+//
+// Weight formats, warp roles, TMEM double buffering and the epilogue arithmetic are those of qmm_tc.cu.
+// Differences: the MMA issuer runs in the pair's first CTA only; the operand copies of both CTAs
+// report to that CTA's `full` barrier; commits arrive at both CTAs' `empty` and `tfull` barriers.
+// Every mbarrier wait is bounded; both CTAs meet at a cluster barrier before either exits, so no
+// arrival can reach the shared memory of a CTA that is gone.
+#include "tc_common.cuh"
+
+#include <algorithm>
+
+namespace fnn {
+
+namespace {
+
+using namespace tc;
+
+constexpr int kPairRows = 2 * kTileN;   // output channels per pair tile
+
+// ---- PTX wrappers of the two-SM forms -----------------------------------------------------------
+
+// Arrival at the first CTA's barrier.  What it announces is never read through the generic proxy by the
+// waiting thread: TMEM columns that tcgen05.ld has finished reading, operand tiles handed to the
+// async proxy by fence.proxy.async.  Waits therefore acquire at CTA scope: an acquire at cluster scope also
+// invalidates L1, and in the step loop that cost more than the step (0.6 us against 0.25).
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+// Copies into this CTA's shared memory that report to a barrier of either CTA of the pair.
+__device__ __forceinline__ void tma_load_2d_pair(void *dst, const CUtensorMap *map, uint32_t bar, int c0, int c1) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+        ::"r"(smem_u32(dst)), "l"(map), "r"(bar), "r"(c0), "r"(c1)
+        : "memory");
+}
+__device__ __forceinline__ void tma_load_3d_pair(void *dst, const CUtensorMap *map, uint32_t bar, int c0, int c1,
+                                                 int c2) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+        ::"r"(smem_u32(dst)), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2)
+        : "memory");
+}
+// Arrives at the barrier of this offset in both CTAs once the MMAs issued so far have finished.
+__device__ __forceinline__ void tc_commit_pair(uint64_t *bar) {
+    asm volatile(
+        "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
+            smem_u32(bar)),
+        "h"((uint16_t)3)
+        : "memory");
+}
+template <int KIND>
+__device__ __forceinline__ void tc_mma_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
+                                            uint32_t accumulate) {
+    if (KIND == KIND_I8) {
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+            "tcgen05.mma.cta_group::2.kind::i8 [%0], %1, %2, %3, p;\n\t}"
+            ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+            : "memory");
+    } else if (KIND == KIND_F8) {
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+            "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}"
+            ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+            : "memory");
+    } else {
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+            "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+            ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+            : "memory");
+    }
+}
+
+struct PairParams {
+    const float *scales;
+    const float *zeros;
+    const float *bias;
+    const float *dq;
+    const float *rowsum;
+    const float *codebook;   // WF_CB: 16 centroids
+    float *out;
+    int *err_flag;
+    int M, N;
+    int Mb;        // batch rows per tile
+    int n_tiles, m_tiles;   // tiles of 256 channels, of Mb batch rows
+    int kblocks;
+    int a_fmt;
+    float acc_scale;
+    int stages;
+    int epilogue;
+};
+
+template <int KIND, int T, bool SUM, int WF>
+__global__ void __launch_bounds__((2 + kEpiWarps + xf_warps(WF)) * 32, 1)
+qmm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a,
+                   const __grid_constant__ CUtensorMap map_s, PairParams p) {
+    constexpr int ATOMS = (KIND == KIND_F16) ? 2 : 1;
+    constexpr int TA = SUM ? 1 : T;                                    // accumulators per batch row
+    constexpr int kRawBytes = (WF == WF_TMA) ? 0 : kTileN * 64;        // packed nibbles: 64 bytes per row
+    constexpr int kScBytes = (WF == WF_CB) ? kTileN * 16 : 0;          // four block scales per row
+    constexpr int kXf0 = 2 + kEpiWarps;                                // first transform warp
+    constexpr int kXfArrivals = 2 * xf_warps(WF);     // of both CTAs
+    constexpr int a_atom = kTileN * kKBlockBytes, a_bytes = ATOMS * a_atom;
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    // both CTAs of the pair lay their shared memory out alike: an MMA names one offset for both
+    unsigned char *smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+    const int acc_cols = TA * p.Mb;                        // accumulator columns of a tile
+    const int mma_cols = SUM ? p.Mb : T * p.Mb;            // MMA N
+    const int b_rows = T * p.Mb / 2;                       // activation rows this CTA holds per K block
+    const int b_atom = b_rows * kKBlockBytes;              // (b_rows is a multiple of 8)
+    const int b_bytes = ATOMS * b_atom;
+    unsigned char *s_a = smem;
+    unsigned char *s_b = s_a + (size_t)p.stages * a_bytes;
+    unsigned char *s_raw = s_b + (size_t)p.stages * b_bytes;
+    uint64_t *bars = reinterpret_cast<uint64_t *>(s_raw + (size_t)p.stages * (kRawBytes + kScBytes));
+    uint64_t *full = bars, *empty = bars + p.stages, *rawfull = bars + 2 * p.stages;
+    uint64_t *tfull = bars + 3 * p.stages, *tempty = tfull + 2;
+    uint32_t *s_tmem = reinterpret_cast<uint32_t *>(tempty + 2);
+    volatile int *s_abort = reinterpret_cast<volatile int *>(s_tmem + 1);
+    float *s_cb = table_after(s_tmem + 2);                                // [16]
+
+    const int warp = __shfl_sync(0xFFFFFFFFu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+    const uint32_t rank = blockIdx.x & 1;   // clusters are pairs of consecutive blocks (a uniform value)
+    pdl_launch_dependents();
+    uint32_t ncols = 32;
+    while ((int)ncols < 2 * acc_cols) ncols <<= 1;
+    const int total_tiles = p.n_tiles * p.m_tiles;
+    const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+
+    if (threadIdx.x == 0) {
+        prefetch_tensormap(&map_w);
+        prefetch_tensormap(&map_a);
+        if (WF == WF_CB) prefetch_tensormap(&map_s);
+        for (int s = 0; s < p.stages; ++s) {
+            mbar_init(&full[s], 1 + kXfArrivals);   // (the first CTA's is the one in use)
+            mbar_init(&empty[s], 1);
+            mbar_init(&rawfull[s], 1);
+        }
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(&tfull[i], 1);
+            mbar_init(&tempty[i], 2 * kEpiWarps);   // (the first CTA's is the one in use)
+        }
+        *s_abort = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (WF == WF_CB && threadIdx.x >= 64 && threadIdx.x < 80) s_cb[threadIdx.x - 64] = p.codebook[threadIdx.x - 64];
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(s_tmem)),
+                     "r"(ncols)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    }
+    __syncwarp();
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync();   // the other CTA's barriers exist
+    tc_fence_after();
+    const uint32_t tmem_base = *s_tmem;
+
+    if (warp == 0) {
+        // ---------------- TMA producer (one in each CTA, for its own halves) ----------------
+        if (elect_one()) {
+            int s = 0;
+            uint32_t phase = 0;
+            bool ok = true;
+            // bytes that both CTAs' copies of a stage report to the first CTA's barrier (the unpacking
+            // 4-bit tensor-map type counts the packed source bytes)
+            const uint32_t full_tx = 2u * (uint32_t)((WF == WF_TMA ? (p.a_fmt == kFmtE2M1 ? a_bytes / 2 : a_bytes) : 0) + b_bytes);
+            auto load_w = [&](int st, int nt, int kb) {
+                const int n0 = nt * kPairRows + (int)rank * kTileN;
+                if (WF == WF_TMA) {
+                    const uint32_t bar = mapa(&full[st], 0);
+#pragma unroll
+                    for (int at = 0; at < ATOMS; ++at)
+                        tma_load_2d_pair(s_a + (size_t)st * a_bytes + at * a_atom, &map_w, bar,
+                                         (kb * ATOMS + at) * kKBlockBytes, n0);
+                } else {
+                    unsigned char *raw = s_raw + (size_t)st * (kRawBytes + kScBytes);
+                    mbar_expect_tx(&rawfull[st], (uint32_t)(kRawBytes + kScBytes));
+                    tma_load_2d(raw, &map_w, &rawfull[st], kb * 64, n0);
+                    if (WF == WF_CB) tma_load_2d(raw + kRawBytes, &map_s, &rawfull[st], kb * 16, n0);
+                }
+            };
+            auto load_b = [&](int st, int mt, int kb) {
+                const uint32_t bar = mapa(&full[st], 0);
+                // SUM: rows [rank * Mb / 2, + Mb / 2) of both planes.  Otherwise this CTA's half of the
+                // (term, batch row) columns: plane `rank` for two terms, half of the rows for one.
+                const int row = mt * p.Mb + ((SUM || T == 1) ? (int)rank * (p.Mb / 2) : 0);
+                const int plane = (SUM || T == 1) ? 0 : (int)rank;
+#pragma unroll
+                for (int at = 0; at < ATOMS; ++at)
+                    tma_load_3d_pair(s_b + (size_t)st * b_bytes + at * b_atom, &map_a, bar,
+                                     (kb * ATOMS + at) * kKBlockBytes, row, plane);
+            };
+            // the first ring of weight tiles does not depend on the kernel before this one
+            int head = 0;
+            if (pair < total_tiles) {
+                head = min(p.stages, p.kblocks);
+                for (int i = 0; i < head; ++i) {
+                    if (rank == 0) mbar_expect_tx(&full[i], full_tx);
+                    load_w(i, pair / p.m_tiles, i);
+                }
+            }
+            pdl_wait();
+            for (int i = 0; i < head; ++i) load_b(i, pair % p.m_tiles, i);
+            s = head;
+            if (s == p.stages) {
+                s = 0;
+                phase = 1;
+            }
+            for (int tile = pair; tile < total_tiles && ok; tile += pairs) {
+                const int nt = tile / p.m_tiles, mt = tile - nt * p.m_tiles;
+                for (int kb = (tile == pair ? head : 0); kb < p.kblocks; ++kb) {
+                    if (!mbar_wait(&empty[s], phase ^ 1, s_abort, p.err_flag, 0x10)) {
+                        ok = false;
+                        break;
+                    }
+                    if (rank == 0) mbar_expect_tx(&full[s], full_tx);
+                    load_w(s, nt, kb);
+                    load_b(s, mt, kb);
+                    if (++s == p.stages) {
+                        s = 0;
+                        phase ^= 1;
+                    }
+                }
+            }
+            if (!ok) {  // let copies already in flight land before the CTA can exit
+                for (int i = 0; i < 64; ++i) __nanosleep(1000);
+            }
+        }
+    } else if (warp == 1) {
+        // ---------------- MMA issuer (first CTA) ----------------
+        if (rank == 0) if (elect_one()) {
+            const uint32_t idesc = make_idesc(KIND, mma_cols, p.a_fmt, kPairRows);
+            int s = 0;
+            uint32_t phase = 0;
+            int as = 0;
+            uint32_t aphase = 0;
+            bool ok = true;
+            for (int tile = pair; tile < total_tiles && ok; tile += pairs) {
+                if (!mbar_wait(&tempty[as], aphase ^ 1, s_abort, p.err_flag, 0x20)) break;
+                tc_fence_after();
+                const uint32_t d_tmem = tmem_base + (uint32_t)(as * acc_cols);
+                for (int kb = 0; kb < p.kblocks; ++kb) {
+                    if (!mbar_wait(&full[s], phase, s_abort, p.err_flag, 0x40)) {
+                        ok = false;
+                        break;
+                    }
+                    tc_fence_after();
+#pragma unroll
+                    for (int at = 0; at < ATOMS; ++at) {
+                        const uint64_t da = make_desc_sw128(smem_u32(s_a + (size_t)s * a_bytes + at * a_atom));
+                        const uint64_t db = make_desc_sw128(smem_u32(s_b + (size_t)s * b_bytes + at * b_atom));
+#pragma unroll
+                        for (int t = 0; t < (SUM ? T : 1); ++t) {
+                            // the second term's rows follow the first's
+                            const uint64_t dbt = db + (uint64_t)((t * (p.Mb / 2) * kKBlockBytes) >> 4);
+#pragma unroll
+                            for (int k = 0; k < kKBlockBytes / 32; ++k)
+                                tc_mma_pair<KIND>(d_tmem, da + (uint64_t)(k * 2), dbt + (uint64_t)(k * 2), idesc,
+                                                  (kb > 0 || at > 0 || t > 0 || k > 0) ? 1u : 0u);
+                        }
+                    }
+                    tc_commit_pair(&empty[s]);
+                    if (++s == p.stages) {
+                        s = 0;
+                        phase ^= 1;
+                    }
+                }
+                if (!ok) break;
+                tc_commit_pair(&tfull[as]);
+                if (++as == 2) {
+                    as = 0;
+                    aphase ^= 1;
+                }
+            }
+        }
+    } else if (WF != WF_TMA && warp >= kXf0) {
+        // ---------------- transform warps (each CTA widens its own weight rows) ----------------
+        const int xt = threadIdx.x - kXf0 * 32;
+        int s = 0;
+        uint32_t phase = 0;
+        bool ok = true;
+        for (int tile = pair; tile < total_tiles && ok; tile += pairs) {
+            for (int kb = 0; kb < p.kblocks; ++kb) {
+                if (!mbar_wait(&rawfull[s], phase, s_abort, p.err_flag, 0x200)) {
+                    ok = false;
+                    break;
+                }
+                const unsigned char *raw = s_raw + (size_t)s * (kRawBytes + kScBytes);
+                unsigned char *dst = s_a + (size_t)s * a_bytes;
+#pragma unroll
+                for (int it = 0; it < (WF == WF_TMA ? 0 : (kTileN * 4) / (xf_warps(WF == WF_TMA ? WF_I4 : WF) * 32)); ++it) {
+                    // a 16-byte unit of a row -> its place in the 128-byte-swizzled operand tile
+                    const int item = xt + it * xf_warps(WF) * 32, row = item >> 2, c = item & 3;
+                    const uint4 w = *reinterpret_cast<const uint4 *>(raw + row * 64 + ((c ^ ((row >> 1) & 3)) << 4));
+                    uint32_t o[16];
+                    if (WF == WF_I4)
+                        widen_i4(w, o);
+                    else
+                        widen_cb(w, *reinterpret_cast<const float *>(raw + kRawBytes + row * 16 + c * 4), smem_u32(s_cb), o);
+                    unsigned char *r = dst + (WF == WF_CB ? (c >> 1) * a_atom : 0) + row * 128;
+                    constexpr int kUnits = (WF == WF_CB) ? 4 : 2;   // 16-byte chunks the unit widens to
+#pragma unroll
+                    for (int u = 0; u < kUnits; ++u)
+                        *reinterpret_cast<uint4 *>(r + ((((c * kUnits + u) & 7) ^ (row & 7)) << 4)) =
+                            make_uint4(o[4 * u], o[4 * u + 1], o[4 * u + 2], o[4 * u + 3]);
+                }
+                fence_proxy_async();   // these stores are read by the tensor cores (async proxy)
+                __syncwarp();
+                if (lane == 0) mbar_arrive_cluster(mapa(&full[s], 0));
+                if (++s == p.stages) {
+                    s = 0;
+                    phase ^= 1;
+                }
+            }
+        }
+    } else if (warp < kXf0) {
+        // ---------------- epilogue (each CTA: its own 128 channels) ----------------
+        pdl_wait();   // dq, rowsum and the output buffer belong to kernels before this one
+        const int quad = warp & 3;
+        const int chunk0 = ((warp - 2) >> 2) * 16;
+        constexpr int kStep = 16 * (kEpiWarps / 4);
+        int as = 0;
+        uint32_t aphase = 0;
+        const bool has_zero = p.zeros != nullptr;
+        const int row = quad * 32 + lane;
+        auto load_rowfac = [&](int mt, int c0) -> float {
+            const int j = lane & 15, m = mt * p.Mb + c0 + j;
+            const bool want = c0 + j < p.Mb && m < p.M && (lane < 16 || has_zero);
+            return want ? (lane < 16 ? p.dq : p.rowsum)[m] : 0.0f;
+        };
+        for (int tile = pair; tile < total_tiles; tile += pairs) {
+            const int nt = tile / p.m_tiles, mt = tile - nt * p.m_tiles;
+            const int n = nt * kPairRows + (int)rank * kTileN + row;
+            const bool n_ok = n < p.N;
+            const float scale = n_ok ? (p.scales ? __ldg(p.scales + n) : 1.0f) : 0.0f;
+            const float zero = (n_ok && has_zero) ? __ldg(p.zeros + n) : 0.0f;
+            const float bias = (n_ok && p.bias) ? p.bias[n] : 0.0f;
+            float fac = load_rowfac(mt, chunk0);
+            if (!mbar_wait(&tfull[as], aphase, s_abort, p.err_flag, 0x80)) break;
+            tc_fence_after();
+            const uint32_t t_base = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(as * acc_cols);
+            for (int c0 = chunk0; c0 < p.Mb; c0 += kStep) {
+                uint32_t r[TA][16];
+#pragma unroll
+                for (int t = 0; t < TA; ++t) tmem_ld16(t_base + (uint32_t)(t * p.Mb + c0), r[t]);
+                const float fac_next = load_rowfac(mt, c0 + kStep);
+                tmem_ld_wait();
+                float v[16];
+                switch (p.epilogue) {
+                case FNN_EPI_RELU:
+                    finish_chunk<KIND, TA, FNN_EPI_RELU>(r, fac, scale, zero, bias, p.bias != nullptr, p.acc_scale, v);
+                    break;
+                case FNN_EPI_GELU:
+                    finish_chunk<KIND, TA, FNN_EPI_GELU>(r, fac, scale, zero, bias, p.bias != nullptr, p.acc_scale, v);
+                    break;
+                case FNN_EPI_SILU:
+                    finish_chunk<KIND, TA, FNN_EPI_SILU>(r, fac, scale, zero, bias, p.bias != nullptr, p.acc_scale, v);
+                    break;
+                default:
+                    finish_chunk<KIND, TA, FNN_EPI_NONE>(r, fac, scale, zero, bias, p.bias != nullptr, p.acc_scale, v);
+                    break;
+                }
+                const int m0 = mt * p.Mb + c0;
+                const int jmax = n_ok ? min(16, min(p.Mb - c0, p.M - m0)) : 0;   // rows of this chunk that exist
+                float *dst = p.out + (size_t)m0 * p.N + n;   // a warp writes 32 consecutive n
+#pragma unroll
+                for (int j = 0; j < 16; ++j)
+                    if (j < jmax) dst[(size_t)j * p.N] = v[j];
+                fac = fac_next;
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(mapa(&tempty[as], 0));
+            if (++as == 2) {
+                as = 0;
+                aphase ^= 1;
+            }
+        }
+    }
+
+    __syncwarp();
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync();   // nothing more arrives at this CTA's barriers, and the MMAs that read its operands are done
+    if (warp == 1) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(ncols) : "memory");
+    }
+}
+
+template <int KIND, int T, bool SUM, int WF>
+int launch_pair(fnn_cuda_ctx *ctx, const QmmArgs &a, const PairTiling &tl) {
+    const fnn_cuda_qweight *w = a.w;
+    constexpr int ES = (KIND == KIND_F16) ? 2 : 1;
+    constexpr int ATOMS = (KIND == KIND_F16) ? 2 : 1;
+    constexpr int TA = SUM ? 1 : T;
+    const int M = (int)a.M, N = (int)w->N, K = (int)w->K;
+    const int Kbytes = K * ES;
+    const int Kp = (Kbytes + 15) & ~15;
+    const int n_tiles = (N + kPairRows - 1) / kPairRows;
+    const int pairs = ctx->sm_count / 2;
+    const int kblocks = (Kbytes + kKBlockBytes * ATOMS - 1) / (kKBlockBytes * ATOMS);
+    const int Mb = tl.Mb, m_tiles = tl.m_tiles, Mpad = m_tiles * Mb;
+
+    const size_t bq_bytes = (size_t)T * Mpad * Kp;
+    const size_t bq_al = (bq_bytes + 255) & ~(size_t)255;
+    int rc = ensure_scratch(ctx, bq_al + (size_t)Mpad * 8 + 256);
+    if (rc != FNN_OK) return rc;
+    uint8_t *bq = (uint8_t *)ctx->scratch;
+    float *dq = (float *)(bq + bq_al);
+    float *rowsum = dq + Mpad;
+    rc = launch_act_prep(ctx, a, KIND, T, WF == WF_I4, Kp, Mpad, bq, dq, rowsum);
+    if (rc != FNN_OK) return rc;
+
+    CUtensorMap map_w, map_a, map_s;
+    rc = encode_weight_map(&map_w, w);
+    if (rc != FNN_OK) return rc;
+    {
+        cuuint64_t dims[3] = {(cuuint64_t)Kp, (cuuint64_t)Mpad, (cuuint64_t)T};
+        cuuint64_t strides[2] = {(cuuint64_t)Kp, (cuuint64_t)Kp * Mpad};
+        // one CTA's half of the activation tile (see load_b)
+        cuuint32_t box[3] = {(cuuint32_t)kKBlockBytes, (cuuint32_t)((SUM || T == 1) ? Mb / 2 : Mb), SUM ? (cuuint32_t)T : 1u};
+        rc = encode_map(&map_a, bq, 3, dims, strides, box);
+        if (rc != FNN_OK) return rc;
+    }
+    if (WF == WF_CB) {
+        rc = encode_block_scale_map(&map_s, w);
+        if (rc != FNN_OK) return rc;
+    } else {
+        map_s = map_a;   // unused
+    }
+    PairParams p{};
+    p.scales = (w->fmt == FNN_FMT_I4CB) ? nullptr : w->scales;
+    p.zeros = w->zeros;
+    p.bias = a.bias;
+    p.dq = dq;
+    p.rowsum = rowsum;
+    p.codebook = w->codebook;
+    p.out = a.out;
+    p.err_flag = ctx->err_flag;
+    p.M = M;
+    p.N = N;
+    p.Mb = Mb;
+    p.n_tiles = n_tiles;
+    p.m_tiles = m_tiles;
+    p.kblocks = kblocks;
+    p.a_fmt = (w->fmt == FNN_FMT_F4) ? kFmtE2M1 : kFmtE4M3;
+    p.acc_scale = (WF == WF_I4) ? 0.0625f : 1.0f;
+    p.epilogue = a.epilogue;
+    const int stage_bytes = ATOMS * (kTileN + T * Mb / 2) * kKBlockBytes +
+                            ((WF == WF_TMA) ? 0 : kTileN * 64 + (WF == WF_CB ? kTileN * 16 : 0));
+    const size_t tail = (3 * 8 + 4) * 8 + 8 + kTableBytes;
+    p.stages = (int)std::min<size_t>(8, (kMaxSmem - 1024 - tail) / stage_bytes);
+    const size_t smem = 1024 + (size_t)p.stages * stage_bytes + tail;
+    const int grid = 2 * std::min(n_tiles * m_tiles, pairs);
+    const int threads = (2 + kEpiWarps + xf_warps(WF)) * 32;
+    auto kern = qmm_tc_pair_kernel<KIND, T, SUM, WF>;
+    FNN_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+                   FNN_ERR_DISPATCH);
+    FNN_CUDA_CHECK(launch_pdl_cluster(kern, grid, 2, threads, smem, ctx, map_w, map_a, map_s, p), FNN_ERR_DISPATCH);
+    ctx->launches++;
+    ctx->last_path = "tc";
+    return FNN_OK;
+}
+
+}  // namespace
+
+// Batch rows per pair tile and how the terms meet.  All pairs run whole tiles, so the time is waves x K blocks x the
+// MMAs of a K block, plus the epilogue of the last tile, which nothing hides (about 0.02 us per batch row).
+// An MMA takes max(90, columns / 2) cycles.  The accumulators of two tiles share the 512 TMEM columns.
+// Among the first tile heights that cover M the cheapest is taken: I8, M = 512, N = 11008 is 172
+// tiles of 128 rows (three waves of 128 on 74 pairs) or 215 tiles of 112 (three waves of 112).
+PairTiling pair_tiling(int fmt, int M, int N, int K, int sm_count) {
+    const bool f8 = fmt == FNN_FMT_F8 || fmt == FNN_FMT_F4, cb = fmt == FNN_FMT_I4CB;
+    const int n_tiles = (N + kPairRows - 1) / kPairRows, pairs = std::max(1, sm_count / 2);
+    const int kblocks = (K + kKBlockBytes - 1) / kKBlockBytes;
+    const int terms = cb ? 1 : (f8 && M < 128) ? 3 : 2;
+    PairTiling best{};
+    double best_cost = 0;
+    for (int sum = 0; sum < 2; ++sum) {
+        if (sum ? !f8 : terms == 3) continue;   // three terms do not split into two halves of planes
+        const int mb_max = (sum || cb) ? 256 : 128, gran = (sum || cb) ? 32 : 16;
+        for (int q = (M + mb_max - 1) / mb_max, i = 0; i < 8; ++i, ++q) {
+            const int rows = (M + q - 1) / q;
+            const int Mb = std::min(mb_max, (rows + gran - 1) / gran * gran);
+            const int m_tiles = (M + Mb - 1) / Mb;
+            const long long waves = ((long long)n_tiles * m_tiles + pairs - 1) / pairs;
+            const int mmas = sum ? 4 * terms : cb ? 8 : 4, cols = sum || cb ? Mb : 2 * Mb;
+            double t_block = mmas * std::max(90, cols / 2) / 1850.0;   // microseconds
+            t_block = std::max(t_block, cb ? 0.75 : fmt == FNN_FMT_I4 ? 0.25 : 0.0);   // widening the weights
+            const double cost = (double)waves * kblocks * t_block + 0.02 * Mb;
+            if (best.Mb == 0 || cost < best_cost) {
+                best_cost = cost;
+                best = {Mb, m_tiles, terms, sum != 0, cost};
+            }
+        }
+    }
+    return best;
+}
+
+// From 65 batch rows on (codebook: 161, its lookups bound both kernels alike below), unless the single-SM kernel gets
+// further by splitting K: the estimates of both, with 1.5 us for the single-SM kernel's longer last epilogue.
+// Measured, us single / pair: I8 K=4096 N=4096 M=64 13.5 (11 split) / 12.5, M=96 13.7 split / 11.9; I8 N=11008 M=96
+// 18.3 / 16.7, M=256 32.7 / 24.9; I4 N=11008 M=96 20.7 / 17.3; I4 M=128 K=14336 N=4096 25.5 split / 36.6.
+bool qmm_tc_uses_pair(const fnn_cuda_ctx *ctx, const fnn_cuda_qweight *w, size_t M) {
+    if (M <= (w->fmt == FNN_FMT_I4CB ? 160u : 64u)) return false;
+    const PairTiling tl = pair_tiling(w->fmt, (int)M, (int)w->N, (int)w->K, ctx->sm_count);
+    return tl.cost < tc_single_cost(ctx, w, M) + 1.5;
+}
+
+int launch_qmm_tc_pair(fnn_cuda_ctx *ctx, const QmmArgs &a) {
+    const PairTiling tl = pair_tiling(a.w->fmt, (int)a.M, (int)a.w->N, (int)a.w->K, ctx->sm_count);
+    switch (a.w->fmt) {
+    case FNN_FMT_I8:
+        return launch_pair<KIND_I8, 2, false, WF_TMA>(ctx, a, tl);
+    case FNN_FMT_I4:
+        return launch_pair<KIND_I8, 2, false, WF_I4>(ctx, a, tl);
+    case FNN_FMT_F8:
+    case FNN_FMT_F4:
+        if (tl.terms == 3) return launch_pair<KIND_F8, 3, true, WF_TMA>(ctx, a, tl);
+        return tl.sum ? launch_pair<KIND_F8, 2, true, WF_TMA>(ctx, a, tl) : launch_pair<KIND_F8, 2, false, WF_TMA>(ctx, a, tl);
+    case FNN_FMT_I4CB:
+        return launch_pair<KIND_F16, 1, false, WF_CB>(ctx, a, tl);
+    }
+    return set_error(FNN_ERR_UNSUPPORTED, "qmatmul: tcgen05 path does not cover format %d", a.w->fmt);
+}
+
+}  // namespace fnn

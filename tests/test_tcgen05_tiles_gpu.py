@@ -44,3 +44,10 @@ def check(backend, fmt, k, n, ms):
 @pytest.mark.parametrize("kn", [(1280, 130), (2176, 24), (3000, 257), (8192, 100), (14336, 48)])
 def test_k_shares_of_a_cluster(backend, fmt, kn):
     check(backend, fmt, *kn, [5, 8, 17, 64])
+
+
+# around one pair tile (256 channels) and one CTA's half of it; around the heights of a tile in batch rows
+@pytest.mark.parametrize("fmt", list(orc.FMT_NAMES))
+@pytest.mark.parametrize("kn", [(128, 256), (520, 129), (777, 513), (1152, 1100)])
+def test_two_sm_tiles(backend, fmt, kn):
+    check(backend, fmt, *kn, [65, 127, 128, 129, 161, 257, 530])
