@@ -78,6 +78,80 @@ row_norm_kernel(const float *in, const float *res, const float *__restrict__ w, 
     }
 }
 
+// The same for rows of a multiple of four and at most 8192 elements with full-length weights, everything on 16 bytes (every
+// layer of a real model): a thread keeps its elements in registers, so the row is read once and with all
+// loads in flight together.  Bound by latency (one trip to L2, two block barriers).
+constexpr int kRowHold = 8;   // float4 a thread can hold
+__device__ __forceinline__ float4 ld_after_wait4(const float *p) {   // (volatile: stays behind griddepcontrol.wait)
+    float4 v;
+    asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                 : "l"(p)
+                 : "memory");
+    return v;
+}
+template <int KIND>
+__global__ void __launch_bounds__(kRowThreads)
+row_norm_regs_kernel(const float *in, const float *res, const float *__restrict__ w, const float *__restrict__ b,
+                     int row_size, float eps, float *out) {   // out may be in (in-place plan slot)
+    __shared__ float s_red[kRowThreads / 32];
+    pdl_launch_dependents();
+    pdl_wait();
+    const float *x = in + (size_t)blockIdx.x * row_size;
+    const float *r = res ? res + (size_t)blockIdx.x * row_size : nullptr;
+    float *y = out + (size_t)blockIdx.x * row_size;
+    float v[kRowHold][4], sm = 0.0f;
+#pragma unroll
+    for (int i = 0; i < kRowHold; ++i) {
+        const int k = (threadIdx.x + i * kRowThreads) * 4;
+        float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (k < row_size) t = ld_after_wait4(x + k);
+        v[i][0] = t.x; v[i][1] = t.y; v[i][2] = t.z; v[i][3] = t.w;
+    }
+    if (r) {
+#pragma unroll
+        for (int i = 0; i < kRowHold; ++i) {
+            const int k = (threadIdx.x + i * kRowThreads) * 4;
+            if (k >= row_size) continue;
+            const float4 t = ld_after_wait4(r + k);
+            v[i][0] = __fadd_rn(v[i][0], t.x); v[i][1] = __fadd_rn(v[i][1], t.y);
+            v[i][2] = __fadd_rn(v[i][2], t.z); v[i][3] = __fadd_rn(v[i][3], t.w);
+        }
+    }
+    float mean = 0.0f;
+    if (KIND == 1) {
+#pragma unroll
+        for (int i = 0; i < kRowHold; ++i) sm += (v[i][0] + v[i][1]) + (v[i][2] + v[i][3]);   // (zero past the row)
+        mean = __fdiv_rn(block_sum(sm, s_red), (float)row_size);
+    }
+    float sq = 0.0f;
+#pragma unroll
+    for (int i = 0; i < kRowHold; ++i) {
+        if ((threadIdx.x + i * kRowThreads) * 4 >= row_size) continue;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) sq = fmaf(v[i][j] - mean, v[i][j] - mean, sq);
+    }
+    sq = block_sum(sq, s_red);
+    const float denom = sqrtf(__fadd_rn(__fdiv_rn(sq, (float)row_size), eps));
+    const float inv_std = __fdiv_rn(1.0f, denom);
+#pragma unroll
+    for (int i = 0; i < kRowHold; ++i) {
+        const int k = (threadIdx.x + i * kRowThreads) * 4;
+        if (k >= row_size) continue;
+        const float4 w4 = *reinterpret_cast<const float4 *>(w + k);
+        const float wi[4] = {w4.x, w4.y, w4.z, w4.w};
+        float4 b4 = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (KIND == 1) b4 = *reinterpret_cast<const float4 *>(b + k);
+        const float bi[4] = {b4.x, b4.y, b4.z, b4.w};
+        float o[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            o[j] = KIND == 0 ? __fmul_rn(__fdiv_rn(v[i][j], denom), wi[j])
+                             : __fadd_rn(__fmul_rn(__fmul_rn(v[i][j] - mean, inv_std), wi[j]), bi[j]);
+        *reinterpret_cast<float4 *>(y + k) = make_float4(o[0], o[1], o[2], o[3]);
+    }
+}
+
 __global__ void __launch_bounds__(kRowThreads)
 softmax_kernel(const float *in, size_t axis_dim, size_t stride, float *out) {   // out may be in
     __shared__ float s_red[kRowThreads / 32];
@@ -144,10 +218,16 @@ int fnn_cuda_row_norm(fnn_cuda_ctx *ctx, fnn_cuda_arena *arena, int kind, size_t
     FNN_REQUIRE(rows <= 0x7FFFFFFFu, FNN_ERR_DISPATCH, "row_norm: too many rows (%zu)", rows);
     const float *in = (const float *)(arena->base + in_offset);
     float *out = (float *)(arena->base + out_offset);
-    cudaError_t e = kind == 0 ? launch_pdl(row_norm_kernel<0>, (int)rows, kRowThreads, 0, ctx, in, res, w,
-                                           wn, b, bn, row_size, eps, out)
-                              : launch_pdl(row_norm_kernel<1>, (int)rows, kRowThreads, 0, ctx, in, res, w,
-                                           wn, b, bn, row_size, eps, out);
+    auto on16 = [](const float *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };   // (null is)
+    const bool regs = row_size % 4 == 0 && row_size <= (size_t)kRowHold * kRowThreads * 4 && on16(in) && on16(out) &&
+                      on16(res) && on16(w) && wn >= row_size && (kind == 0 || (on16(b) && bn >= row_size));
+    cudaError_t e;
+    if (regs)
+        e = launch_pdl(kind == 0 ? row_norm_regs_kernel<0> : row_norm_regs_kernel<1>, (int)rows, kRowThreads, 0, ctx, in, res,
+                       w, b, (int)row_size, eps, out);
+    else
+        e = launch_pdl(kind == 0 ? row_norm_kernel<0> : row_norm_kernel<1>, (int)rows, kRowThreads, 0, ctx, in, res, w, wn, b,
+                       bn, row_size, eps, out);
     FNN_CUDA_CHECK(e, FNN_ERR_DISPATCH);
     ctx->launches++;
     return FNN_OK;
