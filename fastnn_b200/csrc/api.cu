@@ -322,6 +322,26 @@ int fnn_cuda_arena_free(fnn_cuda_arena *a) {
     return FNN_OK;
 }
 
+static int launch_copy2d(fnn_cuda_ctx *ctx, unsigned char *dst, size_t dpitch, const unsigned char *src, size_t spitch,
+                         size_t width, size_t rows);
+
+// Device address of [host, host + bytes) if all of it is pinned host memory, else null.
+static unsigned char *pinned_device_ptr(void *host, size_t bytes) {
+    cudaPointerAttributes first{}, last{};
+    if (cudaPointerGetAttributes(&first, host) != cudaSuccess ||
+        cudaPointerGetAttributes(&last, (unsigned char *)host + bytes - 1) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return nullptr;
+    }
+    if (first.type != cudaMemoryTypeHost || last.type != cudaMemoryTypeHost || !first.devicePointer) return nullptr;
+    const bool whole = (unsigned char *)last.devicePointer - (unsigned char *)first.devicePointer == (ptrdiff_t)bytes - 1;
+    return whole ? (unsigned char *)first.devicePointer : nullptr;
+}
+// Recorded transfers up to this size are kernels that read or write the pinned memory themselves: a copy-engine
+// node starts several microseconds after the kernel before it and the kernel after it as late again.  Larger ones
+// stay on the copy engines, whose rate does not depend on how many loads a few blocks keep in flight.
+constexpr size_t kHostCopyKernelMax = (size_t)256 << 10;
+
 static int arena_copy(fnn_cuda_arena *a, size_t offset, void *host, size_t bytes, bool to_device,
                       bool async) {
     clear_error();
@@ -336,6 +356,14 @@ static int arena_copy(fnn_cuda_arena *a, size_t offset, void *host, size_t bytes
     }
     if (bytes == 0) return rc;
     cudaStream_t s = a->ctx->stream;
+    if (async && a->ctx->capturing && bytes <= kHostCopyKernelMax) {
+        if (unsigned char *pinned = pinned_device_ptr(host, bytes)) {
+            unsigned char *dev = a->base + offset;
+            const int crc = to_device ? launch_copy2d(a->ctx, dev, bytes, pinned, bytes, bytes, 1)
+                                      : launch_copy2d(a->ctx, pinned, bytes, dev, bytes, bytes, 1);
+            return crc != FNN_OK ? crc : rc;
+        }
+    }
     cudaError_t e;
     if (to_device)
         e = cudaMemcpyAsync(a->base + offset, host, bytes, cudaMemcpyHostToDevice, s);
