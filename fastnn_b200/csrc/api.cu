@@ -1,6 +1,7 @@
 // Context, arena, plan-instruction kernels, replay and timing entry points of the C ABI.
 #include "common.cuh"
 
+#include <algorithm>
 #include <stdarg.h>
 #include <stdio.h>
 #include <string.h>
@@ -418,18 +419,34 @@ static int qmatmul_impl(fnn_cuda_ctx *ctx, fnn_cuda_qweight *w, const float *a, 
     QmmArgs args{w, a, out, bias, M, epilogue};
     switch (path) {
     case FNN_PATH_AUTO:
-        // Measured crossover.  The 8-bit fragment kernel wins up to 8 batch rows (beyond that it runs
-        // 16-row groups at twice the time and the tcgen05 sequence, about 14.5 us at K=4096 N=11008, is
-        // ahead); FP8, which rides the fp16 fragment kernel, up to 4.  Layers with tiles for at most a
-        // quarter of the SMs keep the fragment kernels longer (12 and 8 rows): there the tcgen05
-        // kernel is bound by its fixed cost of about 18 us.
+        // Measured crossovers.  FP8 rides the fp16 fragment kernel up to 4 batch rows (8 on layers with tiles for at most a
+        // quarter of the SMs), the codebook format the 8-bit fragment kernel up to 8 (12): there the tcgen05 kernel's
+        // operands are narrower.  The other formats are as exact on the tcgen05 kernel, whose time does not depend
+        // on the number of rows below 16; us fragment / tcgen05:
+        //   I8   K=4096 N=11008  M=4 12.8 / 12.2, M=8 13.8 / 12.1;  K=11008 N=4096 M=4 13.5 / 13.9, M=8 16.1 / 14.0;
+        //        K=1024 N=2048 M=8 5.0 / 5.4 (5 rows on, from 8 MB of weights)
+        //   FP4  K=8192 N=28672 (117 MB) M=1 30.4 / 30.8, M=2 32.1 / 30.4, M=4 36.5 / 31.4, M=8 43.5 / 31.4;
+        //        K=4096 N=11008 (22 MB) M=3 11.1 / 10.4;  K=4096 N=4096 (8 MB) M=2 6.9 / 8.4, M=4 7.4 / 8.5, M=8 8.6 / 8.7
+        //   I4   K=4096 N=4096 M=8 7.6 / 8.0, N=28672 18.3 / 19.3;  K=8192 N=8192 M=8 16.9 / 13.0, K=14336 N=4096 M=4
+        //        17.5 / 14.2: where the staged rows no longer fit beside the ring
         {
             const bool frag_ok = qmm_mma_supported(w, M) && auto_uses_mma(w);
             const size_t tiles128 = div_ceil(w->N, (size_t)128);
             const bool narrow = tiles128 * 4 <= (size_t)ctx->sm_count;
-            const size_t frag_max =
-                !frag_ok ? 0 : (w->fmt == FNN_FMT_F8 ? (narrow ? 8 : 4) : (narrow ? 12 : 8));
-            if (qmm_tc_supported(w, M) && M > frag_max && M > 4) return launch_qmm_tc(ctx, args);
+            const size_t mb = (w->N * w->words_per_row * 4) >> 20;   // packed weights
+            size_t frag_max;
+            switch (w->fmt) {
+            case FNN_FMT_F8: frag_max = narrow ? 8 : 4; break;
+            case FNN_FMT_I4CB: frag_max = narrow ? 12 : 8; break;
+            case FNN_FMT_I8: frag_max = mb >= 8 ? 4 : 8; break;
+            case FNN_FMT_F4: frag_max = mb >= 64 ? 1 : mb >= 16 ? 2 : mb >= 8 ? 4 : 8; break;
+            default: frag_max = std::max<size_t>(1, std::min<size_t>(8, ((size_t)48 << 10) / w->K)); break;
+            }
+            // a capture that finds the scratch buffer too small stays on the kernels that need none, as far as they go
+            const bool no_room = ctx->capturing && ctx->scratch_bytes < qmm_tc_scratch_bytes(w, M);
+            if (!frag_ok) frag_max = 4;
+            else if (no_room && M <= (narrow ? 12u : 8u)) frag_max = narrow ? 12 : 8;
+            if (qmm_tc_supported(w, M) && M > frag_max) return launch_qmm_tc(ctx, args);
         }
         // tiny layers stay on the row kernel: a 16-row x 128-k fragment tile would be mostly padding
         if (qmm_mma_supported(w, M) && auto_uses_mma(w)) return launch_qmm_mma(ctx, args);

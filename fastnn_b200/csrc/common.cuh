@@ -398,6 +398,7 @@ int prepare_qmm_tc(fnn_cuda_ctx *ctx, fnn_cuda_qweight *w);
 static inline bool auto_uses_mma(const fnn_cuda_qweight *w) { return w->K >= 512 && w->N >= 64; }
 bool qmm_tc_supported(const fnn_cuda_qweight *w, size_t M);
 int launch_qmm_tc(fnn_cuda_ctx *ctx, const QmmArgs &args);
+size_t qmm_tc_scratch_bytes(const fnn_cuda_qweight *w, size_t M);   // of the single-SM kernel
 // large batches: two SMs per tile
 struct PairTiling {
     int Mb = 0, m_tiles = 0;   // batch rows per tile, tiles over the batch

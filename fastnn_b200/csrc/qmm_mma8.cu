@@ -18,6 +18,7 @@
 // Epilogue as everywhere:  out = act(dq*acc*scale[n] + zero[n]*sum_k a[m,k] + bias[n])
 // (src/backend/cpu/microkernels/gemm.rs:2048-2087, src/backend/cpu/matmul.rs:61-71).
 #include "frag_common.cuh"
+#include "tc_common.cuh"
 
 namespace fnn {
 
@@ -140,6 +141,10 @@ struct P8 {
     int KB, ntiles, tiles_per_group;
     int Kc;      // activations staged per pass (multiple of KBLK)
     int epilogue;
+    // several rows: the activations already rewritten (byte planes [2][M][Kp], row factors and sums), or null
+    const uint8_t *planes;
+    const float *dq, *rowsum;
+    int Kp;
     int gather_on;
     GatherArgs g;
 };
@@ -277,12 +282,21 @@ qmm_mma8_kernel(P8 p) {
         for (int i = 0; i < kS8 - 1; ++i) issue_next();
 
         if (k0 == 0) {   // under the first weight loads: the per-row scan of the activations
+            if (CB && kCanHold)   // columns of a single row that hold nothing (its own two are written as it is staged)
+                for (int i = tid; i < kc_len / 32 * 8 * CG; i += NT)
+                    if ((i & (8 * CG - 1)) >= 2) s_boff[i] = 0;
             // everything above (scales, the first weight copies) is independent of the kernel before
             // this one on the stream; the activations and the gather counters are not
             pdl_wait();
             if (p.gather_on) gc = gather_begin(p.g, blockIdx.x * NT + tid);
             // ---- per-row step and sum: max |a| over the whole row first ---------------------
-            if (kCanHold && vec_ok && p.K % 8 == 0 && p.K <= NT * 8 * kHeld && kc_len >= Kpad) {
+            if (MULTI && !CB && p.planes) {
+                // written by the kernel before this one: read through L2, after the wait
+                if (tid < p.M) {
+                    s_dq[tid] = __ldcg(p.dq + tid);
+                    s_rs[tid] = __ldcg(p.rowsum + tid);
+                }
+            } else if (kCanHold && vec_ok && p.K % 8 == 0 && p.K <= NT * 8 * kHeld && kc_len >= Kpad) {
                 // A single batch row that is staged in one pass: every thread keeps its groups of eight
                 // consecutive activations in registers between the scan and the rewrite, so the row is
                 // read once.
@@ -328,7 +342,7 @@ qmm_mma8_kernel(P8 p) {
             } else {
                 frag::scan_rows<NT, MULTI ? 4 : 1>(p.act, p.M, p.K, vec_ok, s_part, s_mx, s_rs);
             }
-            if (tid < p.M) {
+            if (tid < p.M && !(MULTI && !CB && p.planes)) {
                 const float bm = s_mx[tid];
                 s_dq[tid] = (bm > 0.0f && isfinite(bm)) ? bm / 16256.0f : 1.0f;
             }   // (published by the barrier below)
@@ -339,7 +353,17 @@ qmm_mma8_kernel(P8 p) {
 
         __syncthreads();  // previous pass fully consumed
         // ---- stage the activation bytes of [k0, k0 + kc_len) --------------------------------
-        if (MULTI && vec_ok && (p.K % 8 == 0)) {
+        if (MULTI && !CB && p.planes) {
+            // copies of the rewritten rows, sixteen bytes at a time
+            const int pieces = kc_len / 16;
+            for (int i = tid; i < 2 * p.M * pieces; i += NT) {
+                const int r = i / pieces, k = (i - r * pieces) * 16;   // plane-major rows, as staged
+                const bool in = k0 + k < p.Kp;
+                frag::cp_async16(s_act + (size_t)r * RS + k, p.planes + (in ? (size_t)r * p.Kp + k0 + k : 0), in ? 16 : 0);
+            }
+            cp_async_commit();
+            cp_async_wait<0>();
+        } else if (MULTI && vec_ok && (p.K % 8 == 0)) {
             // eight activations of four rows per thread and step: two 16-byte loads per row in flight,
             // one 8-byte store per (row, plane)
             const int n8 = kc_len / 8;
@@ -400,6 +424,19 @@ qmm_mma8_kernel(P8 p) {
                 const int gp = group_pos8<FMT>(g8 * 8);
                 *reinterpret_cast<uint2 *>(s_act + gp) = make_uint2(hi[0], hi[1]);
                 *reinterpret_cast<uint2 *>(s_act + (size_t)RS + gp) = make_uint2(lo[0], lo[1]);
+                if (CB) {
+                    // the block sums of the pass below while the bytes are still in registers: four
+                    // consecutive threads hold one 32-element block (whole half-warps are active here)
+                    int sh = __dp4a((int)hi[0], 0x01010101, __dp4a((int)hi[1], 0x01010101, 0));
+                    int sl = __dp4a((int)lo[0], 0x01010101, __dp4a((int)lo[1], 0x01010101, 0));
+                    const unsigned half = 0xFFFFu << (lane & 16);
+                    sh += __shfl_xor_sync(half, sh, 1);
+                    sl += __shfl_xor_sync(half, sl, 1);
+                    sh += __shfl_xor_sync(half, sh, 2);
+                    sl += __shfl_xor_sync(half, sl, 2);
+                    if ((lane & 3) == 0)
+                        *reinterpret_cast<int2 *>(s_boff + (g8 >> 2) * 8 * CG) = make_int2(-kCbHalf * sh, -kCbHalf * sl);
+                }
             }
         } else
         for (int m = 0; m < p.M; ++m) {
@@ -441,7 +478,7 @@ qmm_mma8_kernel(P8 p) {
             }
         }
         __syncthreads();
-        if (CB) {
+        if (CB && !(kCanHold && held)) {
             // -8192 * sum of each 32-element block of every staged column: the centroids are carried
             // with an offset of 8192, which the second MMA of a block takes back through its C operand
             const int nblk = kc_len / 32;
@@ -639,6 +676,28 @@ int launch8(fnn_cuda_ctx *ctx, const QmmArgs &a, int blocks_per_sm = 1) {
     p.epilogue = a.epilogue;
     p.gather_on = a.gather != nullptr;
     if (a.gather) p.g = *a.gather;
+    // Several rows: every block scans and rewrites all of them, which costs more than a kernel that does it once
+    // as soon as there is enough to rewrite.  us in the blocks / once: I4 K=4096 N=4096 M=2 6.3 / 6.3, M=4 7.3 / 6.7,
+    // M=8 10.4 / 7.6; I8 K=11008 N=4096 M=2 13.6 / 12.8, M=4 16.3 / 13.5; I8 K=1024 N=2048 M=4 4.1 / 4.6, M=8 5.7 / 5.0;
+    // I4 K=4096 N=28672 M=4 15.3 / 15.8.  (The codebook format stages groups of eight bytes: slower this way.)
+    const size_t elems = a.M * w->K;
+    if (MULTI && !TT::codebook && !a.gather && (elems > 16384 || (a.M > 4 && elems >= 8192))) {
+        const int Kp = (p.K + 15) & ~15;
+        // (a capture that finds the scratch buffer too small keeps to the blocks)
+        const size_t plane_bytes = ((size_t)2 * p.M * Kp + 255) & ~(size_t)255;
+        if (!ctx->capturing || ctx->scratch_bytes >= plane_bytes + (size_t)p.M * 8) {
+            int rc = ensure_scratch(ctx, plane_bytes + (size_t)p.M * 8);
+            if (rc != FNN_OK) return rc;
+            uint8_t *planes = (uint8_t *)ctx->scratch;
+            float *dq = (float *)(planes + plane_bytes), *rowsum = dq + p.M;
+            rc = tc::launch_act_prep(ctx, a, tc::KIND_I8, 2, FMT == FNN_FMT_I4, Kp, p.M, planes, dq, rowsum);
+            if (rc != FNN_OK) return rc;
+            p.planes = planes;
+            p.dq = dq;
+            p.rowsum = rowsum;
+            p.Kp = Kp;
+        }
+    }
     const int cols = 2 * p.M;   // int8 pairs
     constexpr int MR = 4 * CG;
     const size_t ring = (size_t)kG8 * kW8 * kS8 * kU8 * 2 * (512 + (TT::codebook ? 128 : 0));

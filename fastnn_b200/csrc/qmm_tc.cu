@@ -7,8 +7,7 @@
 //   FP4   kind::f8f6f4 with an e2m1 A operand: the 4-bit tensor-map type unpacks sixteen packed
 //         codes (8 bytes) into each 16-byte slot of the swizzled tile; again no ALU
 //   I4    TMA brings the packed nibbles (64 bytes per row and K block); transform warps widen them
-//         in shared memory to int8 holding 16*q (two logic operations per eight weights) for
-//         kind::i8
+//         into TMEM as int8 holding 16*q (two logic operations per eight weights) for kind::i8
 //   I4CB  TMA brings the nibbles and the block scales; transform warps write fp16 of
 //         block scale x centroid (one rounding) for kind::f16
 //
@@ -24,7 +23,7 @@
 // (src/backend/cpu/microkernels/gemm.rs:2048-2087, src/backend/cpu/matmul.rs:61-71).
 //
 // Warp roles: warp 0 = TMA producer and TMEM owner, warp 1 = MMA issuer, warps 2-9 = epilogue (a TMEM
-// lane quadrant each, two warps per quadrant), warps 10-17 = transform (I4 / I4CB only).  Every
+// lane quadrant each, two warps per quadrant), from warp 10 on = transform (I4: 8, I4CB: 16).  Every
 // mbarrier wait is bounded: a wait that runs out raises the context's error flag, every role leaves
 // its loop, TMEM is freed and the kernel returns.
 #include "tc_common.cuh"
@@ -932,17 +931,28 @@ int launch_tc(fnn_cuda_ctx *ctx, const QmmArgs &a, uint8_t *fixed_scratch = null
 
 int dispatch_tc(fnn_cuda_ctx *ctx, const QmmArgs &a, uint8_t *fixed, size_t fixed_bytes);
 
+namespace {
+int terms_of(const fnn_cuda_qweight *w, size_t M) {
+    return w->fmt == FNN_FMT_I4CB ? 1 : (w->fmt == FNN_FMT_F8 || w->fmt == FNN_FMT_F4) && M < 128 ? 3 : 2;
+}
+}  // namespace
+
+size_t qmm_tc_scratch_bytes(const fnn_cuda_qweight *w, size_t M) {
+    const int terms = terms_of(w, M), Mb = batch_rows(terms, (int)M);
+    const size_t Mpad = div_ceil(M, (size_t)Mb) * Mb, Kp = (w->K * (w->fmt == FNN_FMT_I4CB ? 2 : 1) + 15) & ~(size_t)15;
+    return (((size_t)terms * Mpad * Kp + 255) & ~(size_t)255) + Mpad * 8 + 256;
+}
+
 double tc_single_cost(const fnn_cuda_ctx *ctx, const fnn_cuda_qweight *w, size_t M) {
-    const bool cb = w->fmt == FNN_FMT_I4CB, f8 = w->fmt == FNN_FMT_F8 || w->fmt == FNN_FMT_F4;
-    const int terms = cb ? 1 : f8 && M < 128 ? 3 : 2, Mb = batch_rows(terms, (int)M);
+    const bool cb = w->fmt == FNN_FMT_I4CB;
+    const int terms = terms_of(w, M), Mb = batch_rows(terms, (int)M);
     const int tiles = (int)(div_ceil(w->N, (size_t)kTileN) * div_ceil(M, (size_t)Mb));
     return split_parts(ctx, tiles, (int)div_ceil(w->K, (size_t)kKBlockBytes), terms * Mb, cb ? WF_CB : WF_TMA).cost;
 }
 
 bool qmm_tc_supported(const fnn_cuda_qweight *w, size_t M) {
     (void)M;
-    // I8 / FP8 / FP4 codes are operands as stored; I4 and the codebook format are widened in shared
-    // memory.  The codebook format becomes fp16 of block scale x centroid (only when those stay inside
+    // I8 / FP8 / FP4 codes are operands as stored; I4 and the codebook format are widened on the way.  The codebook format becomes fp16 of block scale x centroid (only when those stay inside
     // the fp16 range) and its block scales travel by TMA, four per row and stage (K a multiple of 128).
     if (w->fmt == FNN_FMT_I4CB && (!w->fp16_ok || w->K % 128 != 0)) return false;
     return w->K >= 128 && w->N >= 1 && w->N < (1u << 30) && w->K < (1u << 29);
