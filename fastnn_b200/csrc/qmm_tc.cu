@@ -147,7 +147,9 @@ act_prep_kernel(const float *act, int M, int K, int Kp, int Mpad, uint8_t *bq, f
 // step with all loads in flight together, stays in registers between the scan and the rewrite, and
 // every plane is written eight bytes at a time.
 constexpr int kPrepHold = 8;   // units of eight elements a thread can hold
-template <int KIND, int T, bool PERM8>
+// HOLD: 2, 4 or 8 units, the smallest that covers the row: fewer registers (more rows at once on an SM, and room beside
+// the main kernel before it) and less code to fetch, which a kernel of two microseconds notices.
+template <int KIND, int T, bool PERM8, int HOLD>
 __global__ void __launch_bounds__(256)
 act_prep_regs_kernel(const float *act, int M, int K, int Kp, int Mpad, uint8_t *bq, float *dq, float *rowsum) {
     __shared__ float s_max[8], s_sum[8];
@@ -156,9 +158,9 @@ act_prep_regs_kernel(const float *act, int M, int K, int Kp, int Mpad, uint8_t *
     const int m = blockIdx.x, tid = threadIdx.x;
     const float4 *row4 = reinterpret_cast<const float4 *>(act + (size_t)m * K);
     const int units = K >> 3;
-    float v[kPrepHold][8];
+    float v[HOLD][8];
 #pragma unroll
-    for (int i = 0; i < kPrepHold; ++i) {
+    for (int i = 0; i < HOLD; ++i) {
         const int u = tid + i * 256;
         float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
         if (u < units) {
@@ -170,7 +172,7 @@ act_prep_regs_kernel(const float *act, int M, int K, int Kp, int Mpad, uint8_t *
     }
     float mx = 0.0f, sum = 0.0f;
 #pragma unroll
-    for (int i = 0; i < kPrepHold; ++i)
+    for (int i = 0; i < HOLD; ++i)
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
             mx = fmaxf(mx, fabsf(v[i][j]));
@@ -204,7 +206,7 @@ act_prep_regs_kernel(const float *act, int M, int K, int Kp, int Mpad, uint8_t *
         }
         uint4 *dst = reinterpret_cast<uint4 *>(bq + (size_t)m * Kp);   // Kp = 2 K bytes here
 #pragma unroll
-        for (int i = 0; i < kPrepHold; ++i) {
+        for (int i = 0; i < HOLD; ++i) {
             const int u = tid + i * 256;
             if (u >= units) continue;
             uint32_t h[4];
@@ -230,7 +232,7 @@ act_prep_regs_kernel(const float *act, int M, int K, int Kp, int Mpad, uint8_t *
         }
     }
 #pragma unroll
-    for (int i = 0; i < kPrepHold; ++i) {
+    for (int i = 0; i < HOLD; ++i) {
         const int u = tid + i * 256;
         if (u >= units) continue;
         uint32_t w[T][2];
@@ -764,7 +766,10 @@ int launch_prep(fnn_cuda_ctx *ctx, const QmmArgs &a, int Kp, int Mpad, uint8_t *
     // same shared-memory carve-out as the main kernel: alternating carve-outs between consecutive
     // kernels makes every SM reconfigure (and drain) twice per call
     const bool regs_ok = K % 8 == 0 && K <= kPrepHold * 256 * 8 && (reinterpret_cast<uintptr_t>(a.a) & 15) == 0;
-    auto prep = regs_ok ? act_prep_regs_kernel<KIND, T, PERM8> : act_prep_kernel<KIND, T, PERM8>;
+    auto prep = !regs_ok             ? act_prep_kernel<KIND, T, PERM8>
+                : K <= 2 * 256 * 8 ? act_prep_regs_kernel<KIND, T, PERM8, 2>
+                : K <= 4 * 256 * 8 ? act_prep_regs_kernel<KIND, T, PERM8, 4>
+                                   : act_prep_regs_kernel<KIND, T, PERM8, kPrepHold>;
     FNN_CUDA_CHECK(cudaFuncSetAttribute(prep, cudaFuncAttributePreferredSharedMemoryCarveout,
                                         cudaSharedmemCarveoutMaxShared),
                    FNN_ERR_DISPATCH);
