@@ -141,7 +141,7 @@ struct P8 {
     int KB, ntiles, tiles_per_group;
     int Kc;      // activations staged per pass (multiple of KBLK)
     int epilogue;
-    // several rows: the activations already rewritten (byte planes [2][M][Kp], row factors and sums), or null
+    // PLANES: the activations already rewritten (byte planes [2][M][Kp], row factors and sums)
     const uint8_t *planes;
     const float *dq, *rowsum;
     int Kp;
@@ -151,7 +151,9 @@ struct P8 {
 
 // MULTI: more than one batch row (all rows scanned and staged together); the single-row instantiation
 // keeps the shortest prologue.  CG 8-column groups hold the (term, batch row) columns: up to 4 * CG rows.
-template <int FMT, int CG, int kG8, bool MULTI>
+// PLANES: the rows arrive rewritten (p.planes); its own instantiation, since the branch and the longer code cost the
+// smallest calls 2 %.
+template <int FMT, int CG, int kG8, bool MULTI, bool PLANES>
 __global__ void __launch_bounds__(kG8 * kW8 * 32, (kG8 == 1 && CG == 1 && !MULTI && !T8<FMT>::codebook) ? 3 : 1)
 qmm_mma8_kernel(P8 p) {
     using TT = T8<FMT>;
@@ -290,7 +292,7 @@ qmm_mma8_kernel(P8 p) {
             pdl_wait();
             if (p.gather_on) gc = gather_begin(p.g, blockIdx.x * NT + tid);
             // ---- per-row step and sum: max |a| over the whole row first ---------------------
-            if (MULTI && !CB && p.planes) {
+            if (PLANES) {
                 // written by the kernel before this one: read through L2, after the wait
                 if (tid < p.M) {
                     s_dq[tid] = __ldcg(p.dq + tid);
@@ -342,7 +344,7 @@ qmm_mma8_kernel(P8 p) {
             } else {
                 frag::scan_rows<NT, MULTI ? 4 : 1>(p.act, p.M, p.K, vec_ok, s_part, s_mx, s_rs);
             }
-            if (tid < p.M && !(MULTI && !CB && p.planes)) {
+            if (!PLANES && tid < p.M) {
                 const float bm = s_mx[tid];
                 s_dq[tid] = (bm > 0.0f && isfinite(bm)) ? bm / 16256.0f : 1.0f;
             }   // (published by the barrier below)
@@ -353,7 +355,7 @@ qmm_mma8_kernel(P8 p) {
 
         __syncthreads();  // previous pass fully consumed
         // ---- stage the activation bytes of [k0, k0 + kc_len) --------------------------------
-        if (MULTI && !CB && p.planes) {
+        if (PLANES) {
             // copies of the rewritten rows, sixteen bytes at a time
             const int pieces = kc_len / 16;
             for (int i = tid; i < 2 * p.M * pieces; i += NT) {
@@ -716,7 +718,9 @@ int launch8(fnn_cuda_ctx *ctx, const QmmArgs &a, int blocks_per_sm = 1) {
                 "qmatmul: shared memory budget exceeded for M=%d on the 8-bit fragment kernel", p.M);
     p.tiles_per_group = sz.tiles_per_group;
     p.Kc = sz.Kc;
-    auto kern = qmm_mma8_kernel<FMT, CG, kG8, MULTI>;
+    auto kern = qmm_mma8_kernel<FMT, CG, kG8, MULTI, false>;
+    if constexpr (MULTI && !TT::codebook)
+        if (p.planes) kern = qmm_mma8_kernel<FMT, CG, kG8, MULTI, true>;
     FNN_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sz.smem),
                    FNN_ERR_DISPATCH);
     FNN_CUDA_CHECK(launch_pdl(kern, sz.grid, kG8 * kW8 * 32, sz.smem, ctx, p), FNN_ERR_DISPATCH);
