@@ -808,7 +808,10 @@ struct Split {
 };
 Split split_parts(const fnn_cuda_ctx *ctx, int tiles, int kblocks, int cols, int wf) {
     static const int kActive[] = {0, 148, 74, 45, 33, 26, 22};   // of 148 SMs
-    const double t_step = (wf == WF_CB) ? 0.8 : 0.15 + 0.25 * cols / 256.0;
+    // (codebook: 1.1 at 256 columns; below 128 the lookups bound a block and 0.8 is what the split was fitted with)
+    const double t_step = (wf != WF_CB)  ? 0.15 + 0.25 * cols / 256.0
+                          : cols <= 128 ? 0.8
+                                        : 0.8 + 0.35 * (cols - 128) / 128.0;
     const double t_part = 0.8 + 0.4 * cols / 128.0;
     const int waves = (tiles + ctx->sm_count - 1) / ctx->sm_count;
     Split best{1, waves * kblocks * t_step};

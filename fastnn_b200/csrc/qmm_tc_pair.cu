@@ -504,7 +504,8 @@ PairTiling pair_tiling(int fmt, int M, int N, int K, int sm_count) {
             const long long waves = ((long long)n_tiles * m_tiles + pairs - 1) / pairs;
             const int mmas = sum ? 4 * terms : cb ? 8 : 4, cols = sum || cb ? Mb : 2 * Mb;
             double t_block = mmas * std::max(90, cols / 2) / 1850.0;   // microseconds
-            t_block = std::max(t_block, cb ? 0.75 : fmt == FNN_FMT_I4 ? 0.25 : 0.0);   // widening the weights
+            // widening the weights (codebook: and three stages of 74 KB)
+            t_block = std::max(t_block, cb ? std::max(0.75, Mb / 256.0) : fmt == FNN_FMT_I4 ? 0.25 : 0.0);
             const double cost = (double)waves * kblocks * t_block + 0.02 * Mb;
             if (best.Mb == 0 || cost < best_cost) {
                 best_cost = cost;
@@ -519,8 +520,10 @@ PairTiling pair_tiling(int fmt, int M, int N, int K, int sm_count) {
 // further by splitting K: the estimates of both, with 1.5 us for the single-SM kernel's longer last epilogue.
 // Measured, us single / pair: I8 K=4096 N=4096 M=64 13.5 (11 split) / 12.5, M=96 13.7 split / 11.9; I8 N=11008 M=96
 // 18.3 / 16.7, M=256 32.7 / 24.9; I4 N=11008 M=96 20.7 / 17.3; I4 M=128 K=14336 N=4096 25.5 split / 36.6.
+// Codebook: M=512 K=4096 N=14336 89.3 / 78.3, M=4096 569 / 476, K=2048 N=8192 188 / 156; short K is the epilogue's (M=674 K=512
+// N=8320 30.3 / 35.8: below 2048 never).
 bool qmm_tc_uses_pair(const fnn_cuda_ctx *ctx, const fnn_cuda_qweight *w, size_t M) {
-    if (M <= (w->fmt == FNN_FMT_I4CB ? 160u : 64u)) return false;
+    if (M <= (w->fmt == FNN_FMT_I4CB ? 160u : 64u) || (w->fmt == FNN_FMT_I4CB && w->K < 2048)) return false;
     const PairTiling tl = pair_tiling(w->fmt, (int)M, (int)w->N, (int)w->K, ctx->sm_count);
     return tl.cost < tc_single_cost(ctx, w, M) + 1.5;
 }
