@@ -808,10 +808,7 @@ struct Split {
 };
 Split split_parts(const fnn_cuda_ctx *ctx, int tiles, int kblocks, int cols, int wf) {
     static const int kActive[] = {0, 148, 74, 45, 33, 26, 22};   // of 148 SMs
-    // (codebook: 1.1 at 256 columns; below 128 the lookups bound a block and 0.8 is what the split was fitted with)
-    const double t_step = (wf != WF_CB)  ? 0.15 + 0.25 * cols / 256.0
-                          : cols <= 128 ? 0.8
-                                        : 0.8 + 0.35 * (cols - 128) / 128.0;
+    const double t_step = (wf == WF_CB) ? 0.8 : 0.15 + 0.25 * cols / 256.0;
     const double t_part = 0.8 + 0.4 * cols / 128.0;
     const int waves = (tiles + ctx->sm_count - 1) / ctx->sm_count;
     Split best{1, waves * kblocks * t_step};
@@ -824,8 +821,13 @@ Split split_parts(const fnn_cuda_ctx *ctx, int tiles, int kblocks, int cols, int
     return best;
 }
 
-// batch rows per tile: T * Mb is the MMA N (multiple of 16, at most 256)
-int batch_rows(int terms, int M) { return std::min(terms == 1 ? 256 : terms == 2 ? 128 : 80, (M + 15) & ~15); }
+// Batch rows per tile: T * Mb is the MMA N (multiple of 16, at most 256), tiles of equal height.  The codebook format stops at
+// 128: two accumulator buffers then fit beside the widened operands, and the epilogue of a tile runs under the
+// next (M=674 K=512 N=8320, where the epilogue is the bound: 34.5 us with one buffer of 256).
+int batch_rows(int terms, int M) {
+    const int most = terms == 3 ? 80 : 128, tiles = (M + most - 1) / most;
+    return ((M + tiles - 1) / tiles + 15) & ~15;
+}
 
 // Scratch of one call: the rewritten activations Bq[T][Mpad][Kp], then dq[Mpad] and rowsum[Mpad].
 // `fixed_scratch` null: the context's growable buffer; otherwise a caller-supplied region of
