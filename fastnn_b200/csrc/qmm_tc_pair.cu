@@ -516,14 +516,14 @@ PairTiling pair_tiling(int fmt, int M, int N, int K, int sm_count) {
     return best;
 }
 
-// From 65 batch rows on (codebook: 161, its lookups bound both kernels alike below), unless the single-SM kernel gets
+// From 65 batch rows on (codebook: 129, its lookups bound both kernels alike below), unless the single-SM kernel gets
 // further by splitting K: the estimates of both, with 1.5 us for the single-SM kernel's longer last epilogue.
 // Measured, us single / pair: I8 K=4096 N=4096 M=64 13.5 (11 split) / 12.5, M=96 13.7 split / 11.9; I8 N=11008 M=96
 // 18.3 / 16.7, M=256 32.7 / 24.9; I4 N=11008 M=96 20.7 / 17.3; I4 M=128 K=14336 N=4096 25.5 split / 36.6.
 // Codebook: M=512 K=4096 N=14336 89.3 / 78.3, M=4096 569 / 476, K=2048 N=8192 188 / 156; short K is the epilogue's (M=674 K=512
 // N=8320 30.3 / 35.8: below 2048 never).
 bool qmm_tc_uses_pair(const fnn_cuda_ctx *ctx, const fnn_cuda_qweight *w, size_t M) {
-    if (M <= (w->fmt == FNN_FMT_I4CB ? 160u : 64u) || (w->fmt == FNN_FMT_I4CB && w->K < 2048)) return false;
+    if (M <= (w->fmt == FNN_FMT_I4CB ? 128u : 64u) || (w->fmt == FNN_FMT_I4CB && w->K < 2048)) return false;
     const PairTiling tl = pair_tiling(w->fmt, (int)M, (int)w->N, (int)w->K, ctx->sm_count);
     return tl.cost < tc_single_cost(ctx, w, M) + 1.5;
 }
