@@ -208,6 +208,23 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 __device__ __forceinline__ void pdl_launch_dependents() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
+// Loads of what an earlier kernel on the stream may have written: activations, a bias or a norm's weights that are
+// inputs of the plan.  They belong behind pdl_wait().  A load through `const __restrict__` or __ldg counts as
+// invariant for the compiler, which may then move it above the wait, and takes the non-coherent path, which is only
+// for data that nobody writes while the kernel lives; volatile asm keeps its place behind the (volatile asm) wait.
+__device__ __forceinline__ float ld_after_wait(const float *p) {
+    float v;
+    asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ float4 ld_after_wait(const float4 *p) {
+    float4 v;
+    asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                 : "l"(p)
+                 : "memory");
+    return v;
+}
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_pdl(void (*kern)(KArgs...), int grid, int block, size_t smem, const fnn_cuda_ctx *ctx,
                               Args &&...args) {

@@ -40,8 +40,8 @@ __device__ __forceinline__ void group_barrier(int group) {
 // warps' partials are folded by one thread per row in a fixed order, so the sums do not depend on
 // scheduling.  s_part holds [NW][rows rounded up to R][2] floats.  Ends with a block barrier.
 template <int NT, int R>
-__device__ __forceinline__ void scan_rows(const float *__restrict__ act, int M, int K, bool vec_ok,
-                                          float *s_part, float *s_mx, float *s_sum) {
+__device__ __forceinline__ void scan_rows(const float *act, int M, int K, bool vec_ok, float *s_part, float *s_mx,
+                                          float *s_sum) {
     constexpr int NW = NT / 32;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int Mr = (M + R - 1) / R * R;
@@ -54,7 +54,7 @@ __device__ __forceinline__ void scan_rows(const float *__restrict__ act, int M, 
 #pragma unroll
                 for (int m = 0; m < R; ++m) {
                     if (mb + m < M) {
-                        const float4 v = __ldg(reinterpret_cast<const float4 *>(act + (size_t)(mb + m) * K) + i);
+                        const float4 v = ld_after_wait(reinterpret_cast<const float4 *>(act + (size_t)(mb + m) * K) + i);
                         mx[m] = fmaxf(fmaxf(mx[m], fmaxf(fabsf(v.x), fabsf(v.y))), fmaxf(fabsf(v.z), fabsf(v.w)));
                         sum[m] += (v.x + v.y) + (v.z + v.w);
                     }
@@ -65,7 +65,7 @@ __device__ __forceinline__ void scan_rows(const float *__restrict__ act, int M, 
 #pragma unroll
                 for (int m = 0; m < R; ++m) {
                     if (mb + m < M) {
-                        const float a = __ldg(act + (size_t)(mb + m) * K + k);
+                        const float a = ld_after_wait(act + (size_t)(mb + m) * K + k);
                         mx[m] = fmaxf(mx[m], fabsf(a));
                         sum[m] += a;
                     }
@@ -98,6 +98,19 @@ __device__ __forceinline__ void scan_rows(const float *__restrict__ act, int M, 
         s_sum[tid] = bs;
     }
     __syncthreads();
+}
+
+// The bias of a group's rows (tiles gg, gg + GG, ...), into the third word of their entries in `meta`.  A bias can be
+// an input that the kernel before this one writes, so it is read behind pdl_wait(), unlike the scales and
+// zero points of the weight, and not through the non-coherent path.  Asynchronous copies, issued behind the
+// barrier that publishes the staged rows: they belong to the next group of the weight ring and have landed when the ring is drained, so nobody
+// waits for them and no register holds them (loaded ahead of the staging they cost 0.1 to 0.2 us of a call of 8).
+__device__ __forceinline__ void copy_bias(const float *bias, int N, int gtid, int tiles, int gg, int GG, float *meta) {
+#pragma unroll 1
+    for (int i = gtid; i < tiles * 16; i += kWarpsPerGroup * 32) {
+        const int n = (gg + (i >> 4) * GG) * 16 + (i & 15);
+        if (n < N) cp_async4(meta + i * 3 + 2, bias + n, 4);
+    }
 }
 
 // Launch sizing shared by both kernels.  One block per SM whenever the per-group accumulators of

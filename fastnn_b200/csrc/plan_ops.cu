@@ -43,9 +43,8 @@ __device__ __forceinline__ float block_max(float v, float *s_red) {
 // KIND 0: rms_norm, KIND 1: layer_norm (population variance); x = in (+ res when given).
 template <int KIND>
 __global__ void __launch_bounds__(kRowThreads)
-row_norm_kernel(const float *in, const float *res, const float *__restrict__ w, size_t w_len,
-                const float *__restrict__ b, size_t b_len, size_t row_size, float eps,
-                float *out) {   // out may be in (in-place plan slot)
+row_norm_kernel(const float *in, const float *res, const float *w, size_t w_len, const float *b, size_t b_len,
+                size_t row_size, float eps, float *out) {   // out may be in (in-place plan slot)
     __shared__ float s_red[kRowThreads / 32];
     pdl_launch_dependents();
     pdl_wait();
@@ -82,18 +81,10 @@ row_norm_kernel(const float *in, const float *res, const float *__restrict__ w, 
 // layer of a real model): a thread keeps its elements in registers, so the row is read once and with all
 // loads in flight together.  Bound by latency (one trip to L2, two block barriers).
 constexpr int kRowHold = 8;   // float4 a thread can hold
-__device__ __forceinline__ float4 ld_after_wait4(const float *p) {   // (volatile: stays behind griddepcontrol.wait)
-    float4 v;
-    asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];"
-                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-                 : "l"(p)
-                 : "memory");
-    return v;
-}
 template <int KIND>
 __global__ void __launch_bounds__(kRowThreads)
-row_norm_regs_kernel(const float *in, const float *res, const float *__restrict__ w, const float *__restrict__ b,
-                     int row_size, float eps, float *out) {   // out may be in (in-place plan slot)
+row_norm_regs_kernel(const float *in, const float *res, const float *w, const float *b, int row_size, float eps,
+                     float *out) {   // out may be in (in-place plan slot)
     __shared__ float s_red[kRowThreads / 32];
     pdl_launch_dependents();
     pdl_wait();
@@ -105,7 +96,7 @@ row_norm_regs_kernel(const float *in, const float *res, const float *__restrict_
     for (int i = 0; i < kRowHold; ++i) {
         const int k = (threadIdx.x + i * kRowThreads) * 4;
         float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (k < row_size) t = ld_after_wait4(x + k);
+        if (k < row_size) t = ld_after_wait(reinterpret_cast<const float4 *>(x + k));
         v[i][0] = t.x; v[i][1] = t.y; v[i][2] = t.z; v[i][3] = t.w;
     }
     if (r) {
@@ -113,10 +104,19 @@ row_norm_regs_kernel(const float *in, const float *res, const float *__restrict_
         for (int i = 0; i < kRowHold; ++i) {
             const int k = (threadIdx.x + i * kRowThreads) * 4;
             if (k >= row_size) continue;
-            const float4 t = ld_after_wait4(r + k);
+            const float4 t = ld_after_wait(reinterpret_cast<const float4 *>(r + k));
             v[i][0] = __fadd_rn(v[i][0], t.x); v[i][1] = __fadd_rn(v[i][1], t.y);
             v[i][2] = __fadd_rn(v[i][2], t.z); v[i][3] = __fadd_rn(v[i][3], t.w);
         }
+    }
+    // the weights are requested with the row: they may be inputs of the plan, so not before the wait
+    float4 w4[kRowHold], b4[KIND == 1 ? kRowHold : 1];
+#pragma unroll
+    for (int i = 0; i < kRowHold; ++i) {
+        const int k = (threadIdx.x + i * kRowThreads) * 4;
+        if (k >= row_size) continue;
+        w4[i] = ld_after_wait(reinterpret_cast<const float4 *>(w + k));
+        if constexpr (KIND == 1) b4[i] = ld_after_wait(reinterpret_cast<const float4 *>(b + k));
     }
     float mean = 0.0f;
     if (KIND == 1) {
@@ -138,11 +138,11 @@ row_norm_regs_kernel(const float *in, const float *res, const float *__restrict_
     for (int i = 0; i < kRowHold; ++i) {
         const int k = (threadIdx.x + i * kRowThreads) * 4;
         if (k >= row_size) continue;
-        const float4 w4 = *reinterpret_cast<const float4 *>(w + k);
-        const float wi[4] = {w4.x, w4.y, w4.z, w4.w};
-        float4 b4 = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (KIND == 1) b4 = *reinterpret_cast<const float4 *>(b + k);
-        const float bi[4] = {b4.x, b4.y, b4.z, b4.w};
+        const float wi[4] = {w4[i].x, w4[i].y, w4[i].z, w4[i].w};
+        float bi[4] = {0.f, 0.f, 0.f, 0.f};
+        if constexpr (KIND == 1) {
+            bi[0] = b4[i].x; bi[1] = b4[i].y; bi[2] = b4[i].z; bi[3] = b4[i].w;
+        }
         float o[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j)

@@ -206,14 +206,13 @@ qmm_mma_kernel(MmaParams p) {
 
     unsigned char *my_ring = s_ring + (size_t)warp * S * UNITS * 512 + lane * 16;
 
-    // scale / zero / bias of the group's rows: fetched now, used by the epilogue
+    // scale / zero of the group's rows: fetched now, used by the epilogue (the bias follows griddepcontrol.wait)
     float *my_meta = s_meta + (size_t)group * p.tiles_per_group * 48;
     for (int i = gtid; i < tiles_here * 16; i += kW * 32) {
         const int n = (gg + (i >> 4) * GG) * 16 + (i & 15);
         const bool in = n < p.N;
         my_meta[i * 3 + 0] = in ? __ldg(p.scales + n) : 1.0f;
         my_meta[i * 3 + 1] = (in && has_zero) ? __ldg(p.zeros + n) : 0.0f;
-        my_meta[i * 3 + 2] = (in && p.bias) ? __ldg(p.bias + n) : 0.0f;
     }
     for (int i = tid; i < G * p.tiles_per_group * CG * 128; i += NT) s_out[i] = 0.0f;
     // staged row holding batch column (cg*8 + g), or -1 when that column carries no batch row
@@ -307,8 +306,8 @@ qmm_mma_kernel(MmaParams p) {
                     if (wi < witems && cc[q] < chunks) {
                         const int k = k0 + cc[q] * 8;
                         const float *src = p.act + (size_t)mm[q] * p.K + k;
-                        if (k < p.K) v[q][0] = __ldg(reinterpret_cast<const float4 *>(src));
-                        if (k + 4 < p.K) v[q][1] = __ldg(reinterpret_cast<const float4 *>(src) + 1);
+                        if (k < p.K) v[q][0] = *reinterpret_cast<const float4 *>(src);
+                        if (k + 4 < p.K) v[q][1] = reinterpret_cast<const float4 *>(src)[1];
                     }
                 }
 #pragma unroll
@@ -342,7 +341,7 @@ qmm_mma_kernel(MmaParams p) {
                 const float *src = p.act + (size_t)m * p.K;
                 const float up = s_up[m];
                 for (int k = tid; k < kc_len; k += NT) {
-                    const float a = (k0 + k < p.K) ? __ldg(src + k0 + k) * up : 0.0f;
+                    const float a = (k0 + k < p.K) ? src[k0 + k] * up : 0.0f;
                     const __half h = __float2half_rn(a);
                     const int pos = act_pos<FMT>(k);
                     reinterpret_cast<__half *>(s_act + (size_t)m * RS)[pos] = h;
@@ -353,6 +352,7 @@ qmm_mma_kernel(MmaParams p) {
             }
         }
         __syncthreads();
+        if (k0 == 0 && p.bias) frag::copy_bias(p.bias, p.N, gtid, tiles_here, gg, GG, my_meta);
         // fused gather: the first poll of the previous step's words was issued before the staging
         if (CG == 1 && p.gather_on && k0 == 0 && gc.step > 1u) gather_check_prev(p.g, gc, gridDim.x * NT);
 

@@ -219,7 +219,6 @@ qmm_mma8_kernel(P8 p) {
         const bool in = n < p.N;
         my_meta[i * 3 + 0] = (in && !CB) ? __ldg(p.scales + n) : 1.0f;
         my_meta[i * 3 + 1] = (in && has_zero) ? __ldg(p.zeros + n) : 0.0f;
-        my_meta[i * 3 + 2] = (in && p.bias) ? __ldg(p.bias + n) : 0.0f;
     }
     for (int i = tid; i < kG8 * p.tiles_per_group * CG * 128; i += NT) s_out[i] = 0.0f;
 
@@ -288,7 +287,7 @@ qmm_mma8_kernel(P8 p) {
                 for (int i = tid; i < kc_len / 32 * 8 * CG; i += NT)
                     if ((i & (8 * CG - 1)) >= 2) s_boff[i] = 0;
             // everything above (scales, the first weight copies) is independent of the kernel before
-            // this one on the stream; the activations and the gather counters are not
+            // this one on the stream; the activations, the bias and the gather counters are not
             pdl_wait();
             if (p.gather_on) gc = gather_begin(p.g, blockIdx.x * NT + tid);
             // ---- per-row step and sum: max |a| over the whole row first ---------------------
@@ -309,8 +308,8 @@ qmm_mma8_kernel(P8 p) {
                     const int g8 = tid + j * NT;
                     float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
                     if (g8 * 8 < p.K) {
-                        a = __ldg(reinterpret_cast<const float4 *>(p.act) + 2 * g8);
-                        b = __ldg(reinterpret_cast<const float4 *>(p.act) + 2 * g8 + 1);
+                        a = ld_after_wait(reinterpret_cast<const float4 *>(p.act) + 2 * g8);
+                        b = ld_after_wait(reinterpret_cast<const float4 *>(p.act) + 2 * g8 + 1);
                     }
                     hv[j][0] = a.x; hv[j][1] = a.y; hv[j][2] = a.z; hv[j][3] = a.w;
                     hv[j][4] = b.x; hv[j][5] = b.y; hv[j][6] = b.z; hv[j][7] = b.w;
@@ -379,8 +378,8 @@ qmm_mma8_kernel(P8 p) {
                         if (mb + m < p.M && in) {
                             const float4 *src =
                                 reinterpret_cast<const float4 *>(p.act + (size_t)(mb + m) * p.K + k0 + i8 * 8);
-                            v[m][0] = __ldg(src);
-                            v[m][1] = __ldg(src + 1);
+                            v[m][0] = ld_after_wait(src);
+                            v[m][1] = ld_after_wait(src + 1);
                         }
                     }
 #pragma unroll
@@ -462,7 +461,7 @@ qmm_mma8_kernel(P8 p) {
                         const int i4 = b4 + q * NT + tid;
                         v[q] = make_float4(0.f, 0.f, 0.f, 0.f);
                         if (i4 < n4 && k0 + i4 * 4 < p.K)
-                            v[q] = __ldg(reinterpret_cast<const float4 *>(row + k0 + i4 * 4));
+                            v[q] = ld_after_wait(reinterpret_cast<const float4 *>(row + k0 + i4 * 4));
                     }
 #pragma unroll
                     for (int q = 0; q < 2; ++q) {
@@ -476,7 +475,7 @@ qmm_mma8_kernel(P8 p) {
                     }
                 }
             } else {
-                for (int k = tid; k < kc_len; k += NT) put(k, (k0 + k < p.K) ? __ldg(row + k0 + k) : 0.0f);
+                for (int k = tid; k < kc_len; k += NT) put(k, (k0 + k < p.K) ? ld_after_wait(row + k0 + k) : 0.0f);
             }
         }
         __syncthreads();
@@ -500,6 +499,8 @@ qmm_mma8_kernel(P8 p) {
             }
             __syncthreads();
         }
+
+        if (k0 == 0 && p.bias) frag::copy_bias(p.bias, p.N, gtid, tiles_here, gg, GG, my_meta);
 
         // ---- stream this K range of every tile of the group ----------------------------------
         int c_st = 0;

@@ -60,19 +60,8 @@ __device__ __forceinline__ void split_terms(float x, uint8_t t[3]) {
 }
 
 // The activations are written by the kernel before this one on the stream, so they may only be
-// read after griddepcontrol.wait.  A load through a `const __restrict__` pointer counts as invariant
-// for the compiler, which may then move it above the wait (it did: a chain of layers read the
-// previous run's activations).  The activation pointers of these kernels therefore carry no
-// __restrict__, and the unrolled loads of the register form are volatile asm, which keeps its place
-// after the (volatile asm) wait.
-__device__ __forceinline__ float4 ld_after_wait(const float4 *p) {
-    float4 v;
-    asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];"
-                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-                 : "l"(p)
-                 : "memory");
-    return v;
-}
+// read after griddepcontrol.wait (see ld_after_wait; the compiler did move an invariant load above it once, and a
+// chain of layers read the previous run's activations).  The activation pointers carry no __restrict__.
 
 // ---- activation rewrite ---------------------------------------------------------------------
 // One block per batch row.  Writes T byte planes Bq[t][m][Kp] (rows zero-padded to Kp), the
