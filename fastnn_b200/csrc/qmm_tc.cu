@@ -910,7 +910,11 @@ int launch_tc(fnn_cuda_ctx *ctx, const QmmArgs &a, uint8_t *fixed_scratch = null
     p.stages = stages;
     size_t ring = (size_t)stages * (a_bytes + b_stride + raw_bytes);
     if (parts > 1) ring = std::max(ring, (size_t)T * Mb * kTileN * 4);   // the exchange of a split
-    const size_t smem = 1024 + ring + (3 * stages + 4) * 8 + 8 + kTableBytes;
+    size_t smem = 1024 + ring + (3 * stages + 4) * 8 + 8 + kTableBytes;
+    // A CTA of a split keeps its TMEM until its cluster has met, and the allocation is a wait without a bound: two CTAs
+    // of a split on one SM could wait for each other's columns for good.  More than half of an SM's
+    // shared memory each keeps them apart (I4 up to 16 rows asks for 98 KB and 512 columns).
+    if (parts > 1) smem = std::max(smem, kHalfSmem);
     const int grid = parts > 1 ? tiles * parts : std::min(tiles, ctx->sm_count);
     const int threads = (2 + kEpiWarps + xf_warps(WF)) * 32;
     auto kern = qmm_tc_kernel<KIND, T, WF>;

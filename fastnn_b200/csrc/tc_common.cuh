@@ -297,6 +297,8 @@ __device__ __forceinline__ float *table_after(void *p) {
 // ---- host helpers (qmm_tc.cu) ---------------------------------------------------------------------
 
 constexpr size_t kMaxSmem = 227 * 1024;   // dynamic shared memory a block can have
+constexpr size_t kHalfSmem = 114 * 1024;  // no two blocks of this fit an SM's 228 KB (1 KB of each is the system's)
+static_assert(2 * (kHalfSmem + 1024) > 228 * 1024 && kHalfSmem <= kMaxSmem, "two blocks would share an SM");
 
 int encode_map(CUtensorMap *map, void *base, int rank, const cuuint64_t *dims, const cuuint64_t *strides,
                const cuuint32_t *box, CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_128B,
