@@ -335,7 +335,7 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
         if (WF == WF_CB) prefetch_tensormap(&map_s);
         for (int s = 0; s < p.stages; ++s) {
             // the MMA issuer waits for the activation tile (one arrival with a byte count) and, for the
-            // formats widened in shared memory, for every transform warp
+            // formats that are widened, for every transform warp
             mbar_init(&full[s], 1 + xf_warps(WF));
             mbar_init(&empty[s], 1);
             mbar_init(&rawfull[s], 1);
@@ -491,6 +491,7 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
                     ok = false;
                     break;
                 }
+                tc_fence_after();   // the stage's columns were last read by MMAs another thread issued
                 const unsigned char *raw = s_raw + (size_t)s * raw_bytes + row * 64;
 #pragma unroll
                 for (int i = 0; i < kUnits; ++i) {
