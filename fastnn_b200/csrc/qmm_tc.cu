@@ -909,8 +909,10 @@ int launch_tc(fnn_cuda_ctx *ctx, const QmmArgs &a, uint8_t *fixed_scratch = null
     p.ncols = 32;
     while (p.ncols < p.nbuf * T * Mb + stages * slot_cols) p.ncols <<= 1;
     p.stages = stages;
-    size_t ring = (size_t)stages * (a_bytes + b_stride + raw_bytes);
-    if (parts > 1) ring = std::max(ring, (size_t)T * Mb * kTileN * 4);   // the exchange of a split
+    const size_t ring = (size_t)stages * (a_bytes + b_stride + raw_bytes);
+    // the exchange of a split lies over the drained ring, and the barriers are live right behind the ring
+    FNN_REQUIRE(parts == 1 || (size_t)T * Mb * kTileN * 4 <= ring, FNN_ERR_DISPATCH,
+                "qmatmul: a ring of %d stages does not hold the partial accumulators of %d columns", stages, T * Mb);
     size_t smem = 1024 + ring + (3 * stages + 4) * 8 + 8 + kTableBytes;
     // A CTA of a split keeps its TMEM until its cluster has met, and the allocation is a wait without a bound: two CTAs
     // of a split on one SM could wait for each other's columns for good.  More than half of an SM's
