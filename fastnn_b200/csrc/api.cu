@@ -1,5 +1,6 @@
 // Context, arena, plan-instruction kernels, replay and timing entry points of the C ABI.
 #include "common.cuh"
+#include "page_walk.h"
 
 #include <algorithm>
 #include <stdarg.h>
@@ -326,17 +327,22 @@ int fnn_cuda_arena_free(fnn_cuda_arena *a) {
 static int launch_copy2d(fnn_cuda_ctx *ctx, unsigned char *dst, size_t dpitch, const unsigned char *src, size_t spitch,
                          size_t width, size_t rows);
 
-// Device address of [host, host + bytes) if all of it is pinned host memory, else null.
+// Device address of [host, host + bytes) if all of it is pinned host memory, else null.  Every page is asked: the ends of a
+// buffer can lie in two registered ranges with pageable memory between them, which a kernel must not touch.
 static unsigned char *pinned_device_ptr(void *host, size_t bytes) {
-    cudaPointerAttributes first{}, last{};
-    if (cudaPointerGetAttributes(&first, host) != cudaSuccess ||
-        cudaPointerGetAttributes(&last, (unsigned char *)host + bytes - 1) != cudaSuccess) {
-        (void)cudaGetLastError();
-        return nullptr;
-    }
-    if (first.type != cudaMemoryTypeHost || last.type != cudaMemoryTypeHost || !first.devicePointer) return nullptr;
-    const bool whole = (unsigned char *)last.devicePointer - (unsigned char *)first.devicePointer == (ptrdiff_t)bytes - 1;
-    return whole ? (unsigned char *)first.devicePointer : nullptr;
+    unsigned char *dev = nullptr;
+    const uintptr_t first = reinterpret_cast<uintptr_t>(host);
+    const bool whole = every_page(first, bytes, 4096, [&](uintptr_t p) {
+        cudaPointerAttributes at{};
+        if (cudaPointerGetAttributes(&at, reinterpret_cast<void *>(p)) != cudaSuccess) {
+            (void)cudaGetLastError();
+            return false;
+        }
+        if (at.type != cudaMemoryTypeHost || !at.devicePointer) return false;
+        if (p == first) dev = static_cast<unsigned char *>(at.devicePointer);
+        return static_cast<unsigned char *>(at.devicePointer) == dev + (p - first);
+    });
+    return whole ? dev : nullptr;
 }
 // Recorded transfers up to this size are kernels that read or write the pinned memory themselves: a copy-engine
 // node starts several microseconds after the kernel before it and the kernel after it as late again.  Larger ones
