@@ -20,6 +20,18 @@ int set_error(int code, const char *fmt, ...) {
 }
 void clear_error() { g_err[0] = 0; }
 
+// Whether work queued now is recorded rather than run: between graph_begin and graph_end, or while the caller captures
+// the stream it gave.
+bool stream_capturing(const fnn_cuda_ctx *ctx) {
+    if (ctx->capturing) return true;
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(ctx->stream, &status) != cudaSuccess) {   // the legacy stream while another one is captured
+        (void)cudaGetLastError();
+        return true;
+    }
+    return status != cudaStreamCaptureStatusNone;
+}
+
 int ensure_scratch(fnn_cuda_ctx *ctx, size_t bytes) {
     if (ctx->scratch_bytes >= bytes) return FNN_OK;
     FNN_REQUIRE(!ctx->capturing, FNN_ERR_MEMORY,
@@ -31,7 +43,13 @@ int ensure_scratch(fnn_cuda_ctx *ctx, size_t bytes) {
     // released by fnn_cuda_ctx_destroy.
     size_t want = bytes + (bytes >> 2);
     void *grown = nullptr;
-    FNN_CUDA_CHECK(cudaMalloc(&grown, want), FNN_ERR_MEMORY);
+    // (a caller that captures its own stream may do so in a mode that forbids cudaMalloc to this thread; it records
+    // nothing, and the buffer outlives the graph's use of the context)
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    FNN_CUDA_CHECK(cudaThreadExchangeStreamCaptureMode(&mode), FNN_ERR_MEMORY);
+    const cudaError_t e = cudaMalloc(&grown, want);
+    FNN_CUDA_CHECK(cudaThreadExchangeStreamCaptureMode(&mode), FNN_ERR_MEMORY);
+    FNN_CUDA_CHECK(e, FNN_ERR_MEMORY);
     if (ctx->scratch) ctx->retired_scratch.push_back(ctx->scratch);
     ctx->scratch = grown;
     ctx->scratch_bytes = want;
@@ -449,9 +467,11 @@ static int qmatmul_impl(fnn_cuda_ctx *ctx, fnn_cuda_qweight *w, const float *a, 
             default: frag_max = std::max<size_t>(1, std::min<size_t>(8, ((size_t)48 << 10) / w->K)); break;
             }
             // a capture that finds the scratch buffer too small stays on the kernels that need none, as far as they go
-            const bool no_room = ctx->capturing && ctx->scratch_bytes < qmm_tc_scratch_bytes(w, M);
-            if (!frag_ok) frag_max = 4;
-            else if (no_room && M <= (narrow ? 12u : 8u)) frag_max = narrow ? 12 : 8;
+            if (!frag_ok)
+                frag_max = 4;
+            else if (M > frag_max && M <= (narrow ? 12u : 8u) && ctx->scratch_bytes < qmm_tc_scratch_bytes(w, M) &&
+                     stream_capturing(ctx))
+                frag_max = narrow ? 12 : 8;
             if (qmm_tc_supported(w, M) && M > frag_max) return launch_qmm_tc(ctx, args);
         }
         // tiny layers stay on the row kernel: a 16-row x 128-k fragment tile would be mostly padding

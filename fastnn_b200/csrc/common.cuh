@@ -429,6 +429,7 @@ bool qmm_tc_uses_pair(const fnn_cuda_ctx *ctx, const fnn_cuda_qweight *w, size_t
 int launch_qmm_tc_pair(fnn_cuda_ctx *ctx, const QmmArgs &args);
 void free_qweight_aux(fnn_cuda_qweight *w);
 
+bool stream_capturing(const fnn_cuda_ctx *ctx);
 int ensure_scratch(fnn_cuda_ctx *ctx, size_t bytes);
 
 }  // namespace fnn

@@ -688,7 +688,7 @@ int launch8(fnn_cuda_ctx *ctx, const QmmArgs &a, int blocks_per_sm = 1) {
         const int Kp = (p.K + 15) & ~15;
         // (a capture that finds the scratch buffer too small keeps to the blocks)
         const size_t plane_bytes = ((size_t)2 * p.M * Kp + 255) & ~(size_t)255;
-        if (!ctx->capturing || ctx->scratch_bytes >= plane_bytes + (size_t)p.M * 8) {
+        if (ctx->scratch_bytes >= plane_bytes + (size_t)p.M * 8 || !stream_capturing(ctx)) {
             int rc = ensure_scratch(ctx, plane_bytes + (size_t)p.M * 8);
             if (rc != FNN_OK) return rc;
             uint8_t *planes = (uint8_t *)ctx->scratch;

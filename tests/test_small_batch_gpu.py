@@ -81,3 +81,33 @@ def test_capture_without_scratch(fmt, k, n, m):
         if g:
             lib.fnn_cuda_graph_free(g)
         rig.close()
+
+
+@pytest.mark.parametrize("fmt,k,n,m", [(orc.FMT_I8, 4096, 2304, 8), (orc.FMT_I4, 14336, 256, 4), (orc.FMT_I4, 8192, 256, 4),
+                                       (orc.FMT_F4, 4096, 4352, 5), (orc.FMT_F8, 4096, 512, 40)])
+def test_own_stream_captured_without_scratch(fmt, k, n, m):
+    """The same for a program that captures the stream it gave the context; what needs scratch all the same gets it."""
+    import torch
+    stream = torch.cuda.Stream()
+    fresh = fnn.CudaBackend(0, stream=stream.cuda_stream)
+    lib = fresh.lib
+    q = orc.quantize_kn(fmt, normal(840 + k, (k, n), 0.02))
+    rig = Rig(fresh, q, m)
+    graph = torch.cuda.CUDAGraph()
+    try:
+        assert lib.fnn_cuda_qweight_prepare(fresh.ctx, rig.w.handle, L.PATH_MMA) == 0, L.last_error()
+        x = normal(841, (m, k), 1.0)
+        fresh.write_arena(rig.arena, rig.a_off, x.tobytes())
+        with torch.cuda.graph(graph, stream=stream, capture_error_mode="thread_local"):
+            rc = lib.fnn_cuda_qmatmul(fresh.ctx, rig.w.handle, rig.arena.handle, rig.a_off, rig.out_off, -1, m,
+                                      L.EPI_NONE, L.PATH_AUTO)
+        assert rc == 0, L.last_error()
+        with torch.cuda.stream(stream):
+            graph.replay()
+        fresh.synchronize()
+        got = np.frombuffer(fresh.read_arena(rig.arena, rig.out_off, m * n * 4), np.float32).reshape(m, n)
+        assert max_err_vs_rms(got, orc.qmatmul(q, x)) <= TOL_F32
+    finally:
+        del graph
+        rig.close()
+        fresh.close()
