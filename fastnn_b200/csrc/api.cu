@@ -381,7 +381,10 @@ static int arena_copy(fnn_cuda_arena *a, size_t offset, void *host, size_t bytes
     }
     if (bytes == 0) return rc;
     cudaStream_t s = a->ctx->stream;
-    if (async && a->ctx->capturing && bytes <= kHostCopyKernelMax) {
+    // (the kernels that read a weight in place request it ahead of griddepcontrol.wait: a recorded copy into its rows stays
+    // a copy-engine node, which orders everything after it)
+    if (async && a->ctx->capturing && bytes <= kHostCopyKernelMax &&
+        !(to_device && overlaps_weight_rows(a->base + offset, bytes))) {
         if (unsigned char *pinned = pinned_device_ptr(host, bytes)) {
             unsigned char *dev = a->base + offset;
             const int crc = to_device ? launch_copy2d(a->ctx, dev, bytes, pinned, bytes, bytes, 1)

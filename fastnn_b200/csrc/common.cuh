@@ -428,6 +428,8 @@ double tc_single_cost(const fnn_cuda_ctx *ctx, const fnn_cuda_qweight *w, size_t
 bool qmm_tc_uses_pair(const fnn_cuda_ctx *ctx, const fnn_cuda_qweight *w, size_t M);
 int launch_qmm_tc_pair(fnn_cuda_ctx *ctx, const QmmArgs &args);
 void free_qweight_aux(fnn_cuda_qweight *w);
+// Whether [dev, dev + bytes) holds rows of a weight that is used where the plan wrote it.
+bool overlaps_weight_rows(const void *dev, size_t bytes);
 
 bool stream_capturing(const fnn_cuda_ctx *ctx);
 int ensure_scratch(fnn_cuda_ctx *ctx, size_t bytes);

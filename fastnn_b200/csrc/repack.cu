@@ -2,6 +2,8 @@
 // bit-preserving unrepack, and on-device dequantization.
 #include "common.cuh"
 
+#include <algorithm>
+#include <mutex>
 #include <vector>
 #include <string.h>
 
@@ -12,6 +14,29 @@ void free_qweight_aux(fnn_cuda_qweight *w) {
     if (w->frag_bs) cudaFree(w->frag_bs);
     w->frag = nullptr;
     w->frag_bs = nullptr;
+}
+
+// The weights whose rows are the arena slot itself.  An entry lives as long as its weight object, whatever becomes of the
+// context it was made with.
+static std::mutex g_in_place_lock;
+static std::vector<const fnn_cuda_qweight *> &g_in_place = *new std::vector<const fnn_cuda_qweight *>;   // (never torn down)
+
+static void note_in_place(const fnn_cuda_qweight *w, bool add) {
+    std::lock_guard<std::mutex> hold(g_in_place_lock);
+    if (add)
+        g_in_place.push_back(w);
+    else
+        g_in_place.erase(std::remove(g_in_place.begin(), g_in_place.end(), w), g_in_place.end());
+}
+
+bool overlaps_weight_rows(const void *dev, size_t bytes) {
+    const unsigned char *first = static_cast<const unsigned char *>(dev);
+    std::lock_guard<std::mutex> hold(g_in_place_lock);
+    for (const fnn_cuda_qweight *w : g_in_place) {
+        const unsigned char *rows = reinterpret_cast<const unsigned char *>(w->rows);
+        if (first < rows + w->N * w->ld_u4 * 16 && rows < first + bytes) return true;
+    }
+    return false;
 }
 
 // One thread per element of the [N,K] result: unpack(q)*scale + zero, two roundings.
@@ -180,6 +205,7 @@ static int qweight_build(fnn_cuda_ctx *ctx, int fmt, const void *packed, size_t 
         if ((e = cudaMemcpy(w->codebook, codebook16, 16 * 4, cudaMemcpyHostToDevice)) != cudaSuccess)
             return fail(e, "cudaMemcpy(codebook)");
     }
+    if (!w->rows_owned) note_in_place(w, true);
     *out = w;
     return FNN_OK;
 }
@@ -213,6 +239,7 @@ int fnn_cuda_qweight_free(fnn_cuda_qweight *w) {
     cudaSetDevice(w->ctx->device);
     cudaStreamSynchronize(w->ctx->stream);
     free_qweight_aux(w);
+    if (!w->rows_owned) note_in_place(w, false);
     if (w->rows && w->rows_owned) cudaFree(w->rows);
     if (w->scales) cudaFree(w->scales);
     if (w->zeros) cudaFree(w->zeros);

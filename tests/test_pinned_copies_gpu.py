@@ -2,8 +2,10 @@
 import numpy as np
 import pytest
 
+import oracle as orc
 import fastnn_b200 as fnn
-from helpers import normal
+from fastnn_b200 import _lib as L
+from helpers import max_err_vs_rms, normal
 
 pytestmark = pytest.mark.gpu
 
@@ -57,3 +59,51 @@ def test_runtime_norm_weight_changes_every_step():
             for name, v in step.items():
                 ex.pinned_inputs[name][...] = v
             assert np.array_equal(np.asarray(ex.forward_pinned()["y"]).reshape(w.shape), w)
+
+
+def test_recorded_copy_into_a_weight_used_in_place():
+    """The tcgen05 kernel requests its weights before it waits for the kernel ahead of it: a recorded copy into them has to
+    order what follows all the same."""
+    import ctypes
+    k, n, m = 512, 256, 16
+    be = fnn.CudaBackend(0)
+    lib = be.lib
+    qs = [orc.quantize_kn(orc.FMT_I8, normal(920 + i, (k, n), 0.02)) for i in range(2)]
+    qs[1].scales[:], qs[1].zeros[:] = qs[0].scales, qs[0].zeros   # the weight object keeps the first one's
+    x = normal(922, (m, k), 1.0)
+    want = [orc.qmatmul(q, x) for q in qs]
+    rows = n * k
+    arena = be.allocate_arena(rows + 4096 + (m * k + m * n) * 4)
+    a_off, out_off = rows + 4096, rows + 4096 + m * k * 4
+    be.write_arena(arena, 0, qs[0].payload)
+    be.write_arena(arena, a_off, x.tobytes())
+    meta = fnn.QuantizedWeightMeta(bit_width=8, scales=qs[0].scales, zero_points=qs[0].zeros, shape=[n, k],
+                                   quant_block_size=0, codebooks=[], fmt=orc.FMT_I8)
+    w = be.upload_qweight(b"", meta, arena, 0, len(qs[0].payload))
+    host = ctypes.c_void_p()
+    g = ctypes.c_void_p()
+    assert lib.fnn_cuda_host_alloc(rows, ctypes.byref(host)) == 0
+    try:
+        def call():
+            assert lib.fnn_cuda_arena_write_async(arena.handle, 0, host, rows) == 0, L.last_error()
+            assert lib.fnn_cuda_qmatmul(be.ctx, w.handle, arena.handle, a_off, out_off, -1, m, L.EPI_NONE,
+                                        L.PATH_TC) == 0, L.last_error()
+        ctypes.memmove(host, qs[0].payload, rows)
+        call()
+        be.synchronize()
+        assert lib.fnn_cuda_graph_begin(be.ctx) == 0
+        call()
+        assert lib.fnn_cuda_graph_end(be.ctx, ctypes.byref(g)) == 0
+        for i in range(60):
+            ctypes.memmove(host, qs[i & 1].payload, rows)
+            assert lib.fnn_cuda_graph_launch(be.ctx, g) == 0
+            be.synchronize()
+            got = np.frombuffer(be.read_arena(arena, out_off, m * n * 4), np.float32).reshape(m, n)
+            assert max_err_vs_rms(got, want[i & 1]) <= 1e-3
+    finally:
+        if g:
+            lib.fnn_cuda_graph_free(g)
+        lib.fnn_cuda_host_free(host)
+        w.close()
+        arena.close()
+        be.close()
