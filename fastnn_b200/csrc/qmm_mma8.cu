@@ -685,20 +685,19 @@ int launch8(fnn_cuda_ctx *ctx, const QmmArgs &a, int blocks_per_sm = 1) {
     // I4 K=4096 N=28672 M=4 15.3 / 15.8.  (The codebook format stages groups of eight bytes: slower this way.)
     const size_t elems = a.M * w->K;
     if (MULTI && !TT::codebook && !a.gather && (elems > 16384 || (a.M > 4 && elems >= 8192))) {
-        const int Kp = (p.K + 15) & ~15;
+        const tc::PrepLayout lay = tc::prep_layout(2, 1, a.M, w->K);
         // (a capture that finds the scratch buffer too small keeps to the blocks)
-        const size_t plane_bytes = ((size_t)2 * p.M * Kp + 255) & ~(size_t)255;
-        if (ctx->scratch_bytes >= plane_bytes + (size_t)p.M * 8 || !stream_capturing(ctx)) {
-            int rc = ensure_scratch(ctx, plane_bytes + (size_t)p.M * 8);
+        if (ctx->scratch_bytes >= lay.bytes || !stream_capturing(ctx)) {
+            int rc = ensure_scratch(ctx, lay.bytes);
             if (rc != FNN_OK) return rc;
             uint8_t *planes = (uint8_t *)ctx->scratch;
-            float *dq = (float *)(planes + plane_bytes), *rowsum = dq + p.M;
-            rc = tc::launch_act_prep(ctx, a, tc::KIND_I8, 2, FMT == FNN_FMT_I4, Kp, p.M, planes, dq, rowsum);
+            float *dq = (float *)(planes + lay.dq), *rowsum = (float *)(planes + lay.rowsum);
+            rc = tc::launch_act_prep(ctx, a, tc::KIND_I8, 2, FMT == FNN_FMT_I4, (int)lay.Kp, planes, dq, rowsum);
             if (rc != FNN_OK) return rc;
             p.planes = planes;
             p.dq = dq;
             p.rowsum = rowsum;
-            p.Kp = Kp;
+            p.Kp = (int)lay.Kp;
         }
     }
     const int cols = 2 * p.M;   // int8 pairs

@@ -69,7 +69,7 @@ __device__ __forceinline__ void split_terms(float x, uint8_t t[3]) {
 // in the order 0,2,4,6,1,3,5,7 -- the order in which the I4 transform emits its weights.
 template <int KIND, int T, bool PERM8>
 __global__ void __launch_bounds__(256)
-act_prep_kernel(const float *act, int M, int K, int Kp, int Mpad, uint8_t *bq, float *dq, float *rowsum) {
+act_prep_kernel(const float *act, int M, int K, int Kp, uint8_t *bq, float *dq, float *rowsum) {
     __shared__ float s_max[8], s_sum[8];
     // reads the activations and overwrites planes the previous tensor-core kernel may still read
     pdl_launch_dependents();
@@ -101,7 +101,7 @@ act_prep_kernel(const float *act, int M, int K, int Kp, int Mpad, uint8_t *bq, f
     }
     if (KIND == KIND_F16) {
         // one fp16 term; the row is scaled by a power of two so that its largest element sits just
-        // below 2^15 (exact, any f32 magnitude fits): bq is [Mpad][Kp bytes] of halves
+        // below 2^15 (exact, any f32 magnitude fits): bq is [M][Kp bytes] of halves
         int ex = 15;
         if (mx > 0.0f && isfinite(mx)) (void)frexpf(mx, &ex);
         const int e = max(-120, min(120, 15 - ex));
@@ -127,7 +127,7 @@ act_prep_kernel(const float *act, int M, int K, int Kp, int Mpad, uint8_t *bq, f
         const int i8 = k & 7;
         const int kk = PERM8 ? ((k & ~7) | ((i8 >> 1) + (i8 & 1) * 4)) : k;
 #pragma unroll
-        for (int i = 0; i < T; ++i) bq[((size_t)i * Mpad + m) * Kp + kk] = t[i];
+        for (int i = 0; i < T; ++i) bq[((size_t)i * M + m) * Kp + kk] = t[i];
     }
 }
 
@@ -140,7 +140,7 @@ constexpr int kPrepHold = 8;   // units of eight elements a thread can hold
 // the main kernel before it) and less code to fetch, which a kernel of two microseconds notices.
 template <int KIND, int T, bool PERM8, int HOLD>
 __global__ void __launch_bounds__(256)
-act_prep_regs_kernel(const float *act, int M, int K, int Kp, int Mpad, uint8_t *bq, float *dq, float *rowsum) {
+act_prep_regs_kernel(const float *act, int M, int K, int Kp, uint8_t *bq, float *dq, float *rowsum) {
     __shared__ float s_max[8], s_sum[8];
     pdl_launch_dependents();
     pdl_wait();
@@ -217,7 +217,7 @@ act_prep_regs_kernel(const float *act, int M, int K, int Kp, int Mpad, uint8_t *
         if (Kp > K) {   // K is 8 mod 16: one more unit of zeros pads the row to 16 bytes
 #pragma unroll
             for (int i = 0; i < T; ++i)
-                *reinterpret_cast<uint2 *>(bq + ((size_t)i * Mpad + m) * Kp + K) = make_uint2(0u, 0u);
+                *reinterpret_cast<uint2 *>(bq + ((size_t)i * M + m) * Kp + K) = make_uint2(0u, 0u);
         }
     }
 #pragma unroll
@@ -237,7 +237,7 @@ act_prep_regs_kernel(const float *act, int M, int K, int Kp, int Mpad, uint8_t *
         }
 #pragma unroll
         for (int q = 0; q < T; ++q)
-            *reinterpret_cast<uint2 *>(bq + ((size_t)q * Mpad + m) * Kp + (size_t)u * 8) = make_uint2(w[q][0], w[q][1]);
+            *reinterpret_cast<uint2 *>(bq + ((size_t)q * M + m) * Kp + (size_t)u * 8) = make_uint2(w[q][0], w[q][1]);
     }
 }
 
@@ -749,10 +749,8 @@ int tc::encode_block_scale_map(CUtensorMap *map, const fnn_cuda_qweight *w) {
 namespace {
 
 template <int KIND, int T, bool PERM8>
-int launch_prep(fnn_cuda_ctx *ctx, const QmmArgs &a, int Kp, int Mpad, uint8_t *bq, float *dq, float *rowsum) {
+int launch_prep(fnn_cuda_ctx *ctx, const QmmArgs &a, int Kp, uint8_t *bq, float *dq, float *rowsum) {
     const int M = (int)a.M, K = (int)a.w->K;
-    // Batch rows M .. Mpad of the planes are never written: a batch row is one column of the MMA, so
-    // whatever those rows hold only reaches accumulator columns that the epilogue does not store.
     // same shared-memory carve-out as the main kernel: alternating carve-outs between consecutive
     // kernels makes every SM reconfigure (and drain) twice per call
     const bool regs_ok = K % 8 == 0 && K <= kPrepHold * 256 * 8 && (reinterpret_cast<uintptr_t>(a.a) & 15) == 0;
@@ -763,7 +761,7 @@ int launch_prep(fnn_cuda_ctx *ctx, const QmmArgs &a, int Kp, int Mpad, uint8_t *
     FNN_CUDA_CHECK(cudaFuncSetAttribute(prep, cudaFuncAttributePreferredSharedMemoryCarveout,
                                         cudaSharedmemCarveoutMaxShared),
                    FNN_ERR_DISPATCH);
-    FNN_CUDA_CHECK(launch_pdl(prep, M, 256, 0, ctx, a.a, M, K, Kp, Mpad, bq, dq, rowsum),
+    FNN_CUDA_CHECK(launch_pdl(prep, M, 256, 0, ctx, a.a, M, K, Kp, bq, dq, rowsum),
                    FNN_ERR_DISPATCH);
     ctx->launches++;
     return FNN_OK;
@@ -771,14 +769,32 @@ int launch_prep(fnn_cuda_ctx *ctx, const QmmArgs &a, int Kp, int Mpad, uint8_t *
 
 }  // namespace
 
-int tc::launch_act_prep(fnn_cuda_ctx *ctx, const QmmArgs &a, int kind, int terms, bool perm8, int Kp, int Mpad,
-                        uint8_t *bq, float *dq, float *rowsum) {
+int tc::launch_act_prep(fnn_cuda_ctx *ctx, const QmmArgs &a, int kind, int terms, bool perm8, int Kp, uint8_t *bq,
+                        float *dq, float *rowsum) {
     if (kind == KIND_I8)
-        return perm8 ? launch_prep<KIND_I8, 2, true>(ctx, a, Kp, Mpad, bq, dq, rowsum)
-                     : launch_prep<KIND_I8, 2, false>(ctx, a, Kp, Mpad, bq, dq, rowsum);
-    if (kind == KIND_F16) return launch_prep<KIND_F16, 1, false>(ctx, a, Kp, Mpad, bq, dq, rowsum);
-    return terms == 2 ? launch_prep<KIND_F8, 2, false>(ctx, a, Kp, Mpad, bq, dq, rowsum)
-                      : launch_prep<KIND_F8, 3, false>(ctx, a, Kp, Mpad, bq, dq, rowsum);
+        return perm8 ? launch_prep<KIND_I8, 2, true>(ctx, a, Kp, bq, dq, rowsum)
+                     : launch_prep<KIND_I8, 2, false>(ctx, a, Kp, bq, dq, rowsum);
+    if (kind == KIND_F16) return launch_prep<KIND_F16, 1, false>(ctx, a, Kp, bq, dq, rowsum);
+    return terms == 2 ? launch_prep<KIND_F8, 2, false>(ctx, a, Kp, bq, dq, rowsum)
+                      : launch_prep<KIND_F8, 3, false>(ctx, a, Kp, bq, dq, rowsum);
+}
+
+// Planes of exactly M rows: a tile that reaches past them gets zeros from the copy, so the scratch of a call
+// depends on neither the kernel nor the tile height, and grows with M.
+tc::PrepLayout tc::prep_layout(int terms, int elem_bytes, size_t M, size_t K) {
+    PrepLayout l;
+    l.Kp = (K * elem_bytes + 15) & ~(size_t)15;   // TMA strides are multiples of 16 bytes
+    l.dq = ((size_t)terms * M * l.Kp + 255) & ~(size_t)255;
+    l.rowsum = l.dq + M * 4;
+    l.bytes = l.rowsum + M * 4;
+    return l;
+}
+
+int tc::encode_act_map(CUtensorMap *map, void *planes, const PrepLayout &l, int terms, size_t M, int box_rows, int box_planes) {
+    cuuint64_t dims[3] = {(cuuint64_t)l.Kp, (cuuint64_t)M, (cuuint64_t)terms};
+    cuuint64_t strides[2] = {(cuuint64_t)l.Kp, (cuuint64_t)(l.Kp * M)};
+    cuuint32_t box[3] = {(cuuint32_t)kKBlockBytes, (cuuint32_t)box_rows, (cuuint32_t)box_planes};
+    return encode_map(map, planes, 3, dims, strides, box);
 }
 
 namespace {
@@ -819,7 +835,7 @@ int batch_rows(int terms, int M) {
     return ((M + tiles - 1) / tiles + 15) & ~15;
 }
 
-// Scratch of one call: the rewritten activations Bq[T][Mpad][Kp], then dq[Mpad] and rowsum[Mpad].
+// Scratch of one call: the rewritten activations Bq[T][M][Kp], then dq[M] and rowsum[M] (tc::prep_layout).
 // `fixed_scratch` null: the context's growable buffer; otherwise a caller-supplied region of
 // `fixed_bytes` that must already be large enough (the entry point that may not allocate).
 template <int KIND, int T, int WF>
@@ -829,14 +845,9 @@ int launch_tc(fnn_cuda_ctx *ctx, const QmmArgs &a, uint8_t *fixed_scratch = null
     constexpr int ATOMS = (KIND == KIND_F16) ? 2 : 1;
     const int M = (int)a.M, N = (int)w->N, K = (int)w->K;
     const int Kbytes = K * ES;
-    const int Kp = (Kbytes + 15) & ~15;  // row bytes; TMA strides are multiples of 16 bytes
     const int Mb = batch_rows(T, M);
     const int m_tiles = (M + Mb - 1) / Mb;
-    const int Mpad = m_tiles * Mb;
-
-    const size_t bq_bytes = (size_t)T * Mpad * Kp;
-    const size_t bq_al = (bq_bytes + 255) & ~(size_t)255;
-    const size_t need = bq_al + (size_t)Mpad * 8 + 256;
+    const PrepLayout lay = prep_layout(T, ES, M, K);
     const int n_tiles = (N + kTileN - 1) / kTileN;
     const int kblocks = (Kbytes + kKBlockBytes * ATOMS - 1) / (kKBlockBytes * ATOMS);
     const int tiles = n_tiles * m_tiles;
@@ -844,31 +855,25 @@ int launch_tc(fnn_cuda_ctx *ctx, const QmmArgs &a, uint8_t *fixed_scratch = null
     int rc = FNN_OK;
     uint8_t *bq;
     if (fixed_scratch) {
-        FNN_REQUIRE(need <= fixed_bytes, FNN_ERR_MEMORY,
+        FNN_REQUIRE(lay.bytes <= fixed_bytes, FNN_ERR_MEMORY,
                     "qmatmul_noalloc: M=%d, K=%d needs %zu bytes of activation scratch; the built-in "
                     "scratch holds %zu (use fnn_cuda_qmatmul for larger problems)",
-                    M, K, need, fixed_bytes);
+                    M, K, lay.bytes, fixed_bytes);
         bq = fixed_scratch;
     } else {
-        rc = ensure_scratch(ctx, need);
+        rc = ensure_scratch(ctx, lay.bytes);
         if (rc != FNN_OK) return rc;
         bq = (uint8_t *)ctx->scratch;
     }
-    float *dq = (float *)(bq + bq_al);
-    float *rowsum = dq + Mpad;
-    rc = launch_act_prep(ctx, a, KIND, T, WF == WF_I4, Kp, Mpad, bq, dq, rowsum);
+    float *dq = (float *)(bq + lay.dq), *rowsum = (float *)(bq + lay.rowsum);
+    rc = launch_act_prep(ctx, a, KIND, T, WF == WF_I4, (int)lay.Kp, bq, dq, rowsum);
     if (rc != FNN_OK) return rc;
 
     CUtensorMap map_w, map_a, map_s;
     rc = encode_weight_map(&map_w, w);
     if (rc != FNN_OK) return rc;
-    {
-        cuuint64_t dims[3] = {(cuuint64_t)Kp, (cuuint64_t)Mpad, (cuuint64_t)T};
-        cuuint64_t strides[2] = {(cuuint64_t)Kp, (cuuint64_t)Kp * Mpad};
-        cuuint32_t box[3] = {(cuuint32_t)kKBlockBytes, (cuuint32_t)Mb, (cuuint32_t)T};
-        rc = encode_map(&map_a, bq, 3, dims, strides, box);
-        if (rc != FNN_OK) return rc;
-    }
+    rc = encode_act_map(&map_a, bq, lay, T, M, Mb, T);
+    if (rc != FNN_OK) return rc;
     if (WF == WF_CB) {
         rc = encode_block_scale_map(&map_s, w);
         if (rc != FNN_OK) return rc;
@@ -944,9 +949,7 @@ int terms_of(const fnn_cuda_qweight *w, size_t M) {
 }  // namespace
 
 size_t qmm_tc_scratch_bytes(const fnn_cuda_qweight *w, size_t M) {
-    const int terms = terms_of(w, M), Mb = batch_rows(terms, (int)M);
-    const size_t Mpad = div_ceil(M, (size_t)Mb) * Mb, Kp = (w->K * (w->fmt == FNN_FMT_I4CB ? 2 : 1) + 15) & ~(size_t)15;
-    return (((size_t)terms * Mpad * Kp + 255) & ~(size_t)255) + Mpad * 8 + 256;
+    return prep_layout(terms_of(w, M), w->fmt == FNN_FMT_I4CB ? 2 : 1, M, w->K).bytes;
 }
 
 double tc_single_cost(const fnn_cuda_ctx *ctx, const fnn_cuda_qweight *w, size_t M) {

@@ -413,33 +413,25 @@ int launch_pair(fnn_cuda_ctx *ctx, const QmmArgs &a, const PairTiling &tl) {
     constexpr int TA = SUM ? 1 : T;
     const int M = (int)a.M, N = (int)w->N, K = (int)w->K;
     const int Kbytes = K * ES;
-    const int Kp = (Kbytes + 15) & ~15;
     const int n_tiles = (N + kPairRows - 1) / kPairRows;
     const int pairs = ctx->sm_count / 2;
     const int kblocks = (Kbytes + kKBlockBytes * ATOMS - 1) / (kKBlockBytes * ATOMS);
-    const int Mb = tl.Mb, m_tiles = tl.m_tiles, Mpad = m_tiles * Mb;
+    const int Mb = tl.Mb, m_tiles = tl.m_tiles;
 
-    const size_t bq_bytes = (size_t)T * Mpad * Kp;
-    const size_t bq_al = (bq_bytes + 255) & ~(size_t)255;
-    int rc = ensure_scratch(ctx, bq_al + (size_t)Mpad * 8 + 256);
+    const PrepLayout lay = prep_layout(T, ES, M, K);
+    int rc = ensure_scratch(ctx, lay.bytes);
     if (rc != FNN_OK) return rc;
     uint8_t *bq = (uint8_t *)ctx->scratch;
-    float *dq = (float *)(bq + bq_al);
-    float *rowsum = dq + Mpad;
-    rc = launch_act_prep(ctx, a, KIND, T, WF == WF_I4, Kp, Mpad, bq, dq, rowsum);
+    float *dq = (float *)(bq + lay.dq), *rowsum = (float *)(bq + lay.rowsum);
+    rc = launch_act_prep(ctx, a, KIND, T, WF == WF_I4, (int)lay.Kp, bq, dq, rowsum);
     if (rc != FNN_OK) return rc;
 
     CUtensorMap map_w, map_a, map_s;
     rc = encode_weight_map(&map_w, w);
     if (rc != FNN_OK) return rc;
-    {
-        cuuint64_t dims[3] = {(cuuint64_t)Kp, (cuuint64_t)Mpad, (cuuint64_t)T};
-        cuuint64_t strides[2] = {(cuuint64_t)Kp, (cuuint64_t)Kp * Mpad};
-        // one CTA's half of the activation tile (see load_b)
-        cuuint32_t box[3] = {(cuuint32_t)kKBlockBytes, (cuuint32_t)((SUM || T == 1) ? Mb / 2 : Mb), SUM ? (cuuint32_t)T : 1u};
-        rc = encode_map(&map_a, bq, 3, dims, strides, box);
-        if (rc != FNN_OK) return rc;
-    }
+    // one CTA's half of the activation tile (see load_b)
+    rc = encode_act_map(&map_a, bq, lay, T, M, (SUM || T == 1) ? Mb / 2 : Mb, SUM ? T : 1);
+    if (rc != FNN_OK) return rc;
     if (WF == WF_CB) {
         rc = encode_block_scale_map(&map_s, w);
         if (rc != FNN_OK) return rc;

@@ -306,8 +306,16 @@ int encode_map(CUtensorMap *map, void *base, int rank, const cuuint64_t *dims, c
 int encode_weight_map(CUtensorMap *map, const fnn_cuda_qweight *w);
 int encode_block_scale_map(CUtensorMap *map, const fnn_cuda_qweight *w);
 // Launches the rewrite of the activations as `terms` narrow planes, their row factors and row sums.
-int launch_act_prep(fnn_cuda_ctx *ctx, const QmmArgs &a, int kind, int terms, bool perm8, int Kp, int Mpad, uint8_t *bq,
-                    float *dq, float *rowsum);
+int launch_act_prep(fnn_cuda_ctx *ctx, const QmmArgs &a, int kind, int terms, bool perm8, int Kp, uint8_t *bq, float *dq,
+                    float *rowsum);
+// Where a call's rewritten activations, row factors and row sums lie in its scratch.
+struct PrepLayout {
+    size_t Kp;            // bytes of a row of a plane
+    size_t dq, rowsum;    // byte offsets behind the planes [terms][M][Kp]
+    size_t bytes;
+};
+PrepLayout prep_layout(int terms, int elem_bytes, size_t M, size_t K);
+int encode_act_map(CUtensorMap *map, void *planes, const PrepLayout &l, int terms, size_t M, int box_rows, int box_planes);
 
 }  // namespace tc
 }  // namespace fnn

@@ -134,3 +134,23 @@ def test_noalloc_entry_refuses_what_does_not_fit_or_is_not_served(backend):
     finally:
         wc.close()
         arena.close()
+
+
+# What has to fit the array is the rows of the call, not whole tiles of them: 129 rows of 27008 fp16 are 6.6 MiB (7.0 MB with the
+# row factors), two tiles of 80 rows would be 8.2 MiB.
+def test_noalloc_scratch_holds_exactly_the_rows(backend):
+    k, n, m = 27008, 64, 129
+    q = orc.quantize_kn(orc.FMT_I4CB, normal(940, (k, n), 0.02))
+    x = normal(941, (m, k), 1.0)
+    arena, w, (a_off, out_off, _, _) = _device_rig(backend, q, m)
+    base = arena.device_ptr
+    try:
+        backend.write_arena(arena, a_off, x.tobytes())
+        rc = backend.lib.fnn_cuda_qmatmul_noalloc(backend.ctx, w.handle, base + a_off, base + out_off, None, m, L.EPI_NONE)
+        assert rc == 0, L.last_error()
+        backend.synchronize()
+        got = np.frombuffer(backend.read_arena(arena, out_off, m * n * 4), np.float32).reshape(m, n)
+        assert max_err_vs_rms(got, orc.qmatmul(q, x)) <= 1e-2
+    finally:
+        w.close()
+        arena.close()
