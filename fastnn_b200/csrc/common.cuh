@@ -420,7 +420,6 @@ size_t qmm_tc_scratch_bytes(const fnn_cuda_qweight *w, size_t M);   // of the si
 struct PairTiling {
     int Mb = 0, m_tiles = 0;   // batch rows per tile, tiles over the batch
     int terms = 0;             // narrow terms per activation
-    bool sum = false;          // the terms accumulate into the same columns
     double cost = 0;           // estimated microseconds of the main loops and the last epilogue
 };
 PairTiling pair_tiling(int fmt, int M, int N, int K, int sm_count);

@@ -6,13 +6,12 @@
 // pair computes 256 channels: each SM holds its own 128 weight rows and half of the activation tile,
 // and the tensor cores of both read both halves, so the activation traffic of an SM halves.
 //
-// Two forms, by how the narrow activation terms (see qmm_tc.cu) meet:
-//   SUM   (FP8, FP4: two e4m3 terms of the same scale) both terms accumulate into the same columns, two MMAs
-//         per K step: a tile is 256 channels x up to 256 batch rows and the weight tile is read once
-//         for both terms (48 B per cycle and SM)
-//   !SUM  (I8, I4: hi and lo bytes, whose int32 sums have different weights; codebook: one fp16 term)
-//         one MMA over the (term, batch row) columns; for two terms the first SM holds the hi plane
-//         and the second the lo plane of 128 batch rows (64 B per cycle and SM)
+// Each narrow term of an activation (see qmm_tc.cu) has accumulator columns of its own: one MMA per K step over the
+// (term, batch row) columns, a multiple of 32 and at most 256 of them, each SM holding half.  One term (codebook): half
+// of the batch rows each; two: a plane each; three: a plane and half of the middle one (64 B per cycle and SM
+// at 256 columns).  A form that let the terms of FP8 and FP4 meet in the same columns moved fewer bytes, but its f32
+// accumulators take two or three times the additions: error 1.65e-5 against 1.56e-5 at M=96 K=4096, 1.9e-5 against
+// 1.5e-5 at K=8192.
 //
 // Weight formats, warp roles, TMEM double buffering and the epilogue arithmetic are those of qmm_tc.cu.
 // Differences: the MMA issuer runs in the pair's first CTA only; the operand copies of both CTAs
@@ -105,12 +104,11 @@ struct PairParams {
     int epilogue;
 };
 
-template <int KIND, int T, bool SUM, int WF>
+template <int KIND, int T, int WF>
 __global__ void __launch_bounds__((2 + kEpiWarps + xf_warps(WF)) * 32, 1)
 qmm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a,
                    const __grid_constant__ CUtensorMap map_s, PairParams p) {
     constexpr int ATOMS = (KIND == KIND_F16) ? 2 : 1;
-    constexpr int TA = SUM ? 1 : T;                                    // accumulators per batch row
     constexpr int kRawBytes = (WF == WF_TMA) ? 0 : kTileN * 64;        // packed nibbles: 64 bytes per row
     constexpr int kScBytes = (WF == WF_CB) ? kTileN * 16 : 0;          // four block scales per row
     constexpr int kXf0 = 2 + kEpiWarps;                                // first transform warp
@@ -119,8 +117,7 @@ qmm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     // both CTAs of the pair lay their shared memory out alike: an MMA names one offset for both
     unsigned char *smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-    const int acc_cols = TA * p.Mb;                        // accumulator columns of a tile
-    const int mma_cols = SUM ? p.Mb : T * p.Mb;            // MMA N
+    const int acc_cols = T * p.Mb;                         // accumulator columns of a tile = MMA N
     const int b_rows = T * p.Mb / 2;                       // activation rows this CTA holds per K block
     const int b_atom = b_rows * kKBlockBytes;              // (b_rows is a multiple of 8)
     const int b_bytes = ATOMS * b_atom;
@@ -198,14 +195,17 @@ qmm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             };
             auto load_b = [&](int st, int mt, int kb) {
                 const uint32_t bar = mapa(&full[st], 0);
-                // SUM: rows [rank * Mb / 2, + Mb / 2) of both planes.  Otherwise this CTA's half of the
-                // (term, batch row) columns: plane `rank` for two terms, half of the rows for one.
-                const int row = mt * p.Mb + ((SUM || T == 1) ? (int)rank * (p.Mb / 2) : 0);
-                const int plane = (SUM || T == 1) ? 0 : (int)rank;
+                // This CTA's half of the (term, batch row) columns: plane `rank` for two terms, else T of the 2 T
+                // halves of planes.
 #pragma unroll
                 for (int at = 0; at < ATOMS; ++at)
-                    tma_load_3d_pair(s_b + (size_t)st * b_bytes + at * b_atom, &map_a, bar,
-                                     (kb * ATOMS + at) * kKBlockBytes, row, plane);
+#pragma unroll
+                    for (int i = 0; i < (T == 2 ? 1 : T); ++i) {
+                        const int h = (int)rank * T + i;
+                        const int row = mt * p.Mb + (T == 2 ? 0 : (h & 1) * (p.Mb / 2)), plane = T == 2 ? (int)rank : h >> 1;
+                        tma_load_3d_pair(s_b + (size_t)st * b_bytes + at * b_atom + i * (p.Mb / 2) * kKBlockBytes, &map_a,
+                                         bar, (kb * ATOMS + at) * kKBlockBytes, row, plane);
+                    }
             };
             // the first ring of weight tiles does not depend on the kernel before this one
             int head = 0;
@@ -246,7 +246,7 @@ qmm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     } else if (warp == 1) {
         // ---------------- MMA issuer (first CTA) ----------------
         if (rank == 0) if (elect_one()) {
-            const uint32_t idesc = make_idesc(KIND, mma_cols, p.a_fmt, kPairRows);
+            const uint32_t idesc = make_idesc(KIND, acc_cols, p.a_fmt, kPairRows);
             int s = 0;
             uint32_t phase = 0;
             int as = 0;
@@ -267,14 +267,9 @@ qmm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                         const uint64_t da = make_desc_sw128(smem_u32(s_a + (size_t)s * a_bytes + at * a_atom));
                         const uint64_t db = make_desc_sw128(smem_u32(s_b + (size_t)s * b_bytes + at * b_atom));
 #pragma unroll
-                        for (int t = 0; t < (SUM ? T : 1); ++t) {
-                            // the second term's rows follow the first's
-                            const uint64_t dbt = db + (uint64_t)((t * (p.Mb / 2) * kKBlockBytes) >> 4);
-#pragma unroll
-                            for (int k = 0; k < kKBlockBytes / 32; ++k)
-                                tc_mma_pair<KIND>(d_tmem, da + (uint64_t)(k * 2), dbt + (uint64_t)(k * 2), idesc,
-                                                  (kb > 0 || at > 0 || t > 0 || k > 0) ? 1u : 0u);
-                        }
+                        for (int k = 0; k < kKBlockBytes / 32; ++k)
+                            tc_mma_pair<KIND>(d_tmem, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc,
+                                              (kb > 0 || at > 0 || k > 0) ? 1u : 0u);
                     }
                     tc_commit_pair(&empty[s]);
                     if (++s == p.stages) {
@@ -357,24 +352,24 @@ qmm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             tc_fence_after();
             const uint32_t t_base = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(as * acc_cols);
             for (int c0 = chunk0; c0 < p.Mb; c0 += kStep) {
-                uint32_t r[TA][16];
+                uint32_t r[T][16];
 #pragma unroll
-                for (int t = 0; t < TA; ++t) tmem_ld16(t_base + (uint32_t)(t * p.Mb + c0), r[t]);
+                for (int t = 0; t < T; ++t) tmem_ld16(t_base + (uint32_t)(t * p.Mb + c0), r[t]);
                 const float fac_next = load_rowfac(mt, c0 + kStep);
                 tmem_ld_wait();
                 float v[16];
                 switch (p.epilogue) {
                 case FNN_EPI_RELU:
-                    finish_chunk<KIND, TA, FNN_EPI_RELU>(r, fac, scale, zero, bias, p.bias != nullptr, p.acc_scale, v);
+                    finish_chunk<KIND, T, FNN_EPI_RELU>(r, fac, scale, zero, bias, p.bias != nullptr, p.acc_scale, v);
                     break;
                 case FNN_EPI_GELU:
-                    finish_chunk<KIND, TA, FNN_EPI_GELU>(r, fac, scale, zero, bias, p.bias != nullptr, p.acc_scale, v);
+                    finish_chunk<KIND, T, FNN_EPI_GELU>(r, fac, scale, zero, bias, p.bias != nullptr, p.acc_scale, v);
                     break;
                 case FNN_EPI_SILU:
-                    finish_chunk<KIND, TA, FNN_EPI_SILU>(r, fac, scale, zero, bias, p.bias != nullptr, p.acc_scale, v);
+                    finish_chunk<KIND, T, FNN_EPI_SILU>(r, fac, scale, zero, bias, p.bias != nullptr, p.acc_scale, v);
                     break;
                 default:
-                    finish_chunk<KIND, TA, FNN_EPI_NONE>(r, fac, scale, zero, bias, p.bias != nullptr, p.acc_scale, v);
+                    finish_chunk<KIND, T, FNN_EPI_NONE>(r, fac, scale, zero, bias, p.bias != nullptr, p.acc_scale, v);
                     break;
                 }
                 const int m0 = mt * p.Mb + c0;
@@ -405,12 +400,11 @@ qmm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     }
 }
 
-template <int KIND, int T, bool SUM, int WF>
+template <int KIND, int T, int WF>
 int launch_pair(fnn_cuda_ctx *ctx, const QmmArgs &a, const PairTiling &tl) {
     const fnn_cuda_qweight *w = a.w;
     constexpr int ES = (KIND == KIND_F16) ? 2 : 1;
     constexpr int ATOMS = (KIND == KIND_F16) ? 2 : 1;
-    constexpr int TA = SUM ? 1 : T;
     const int M = (int)a.M, N = (int)w->N, K = (int)w->K;
     const int Kbytes = K * ES;
     const int n_tiles = (N + kPairRows - 1) / kPairRows;
@@ -430,7 +424,7 @@ int launch_pair(fnn_cuda_ctx *ctx, const QmmArgs &a, const PairTiling &tl) {
     rc = encode_weight_map(&map_w, w);
     if (rc != FNN_OK) return rc;
     // one CTA's half of the activation tile (see load_b)
-    rc = encode_act_map(&map_a, bq, lay, T, M, (SUM || T == 1) ? Mb / 2 : Mb, SUM ? T : 1);
+    rc = encode_act_map(&map_a, bq, lay, T, M, T == 2 ? Mb : Mb / 2, 1);
     if (rc != FNN_OK) return rc;
     if (WF == WF_CB) {
         rc = encode_block_scale_map(&map_s, w);
@@ -463,7 +457,7 @@ int launch_pair(fnn_cuda_ctx *ctx, const QmmArgs &a, const PairTiling &tl) {
     const size_t smem = 1024 + (size_t)p.stages * stage_bytes + tail;
     const int grid = 2 * std::min(n_tiles * m_tiles, pairs);
     const int threads = (2 + kEpiWarps + xf_warps(WF)) * 32;
-    auto kern = qmm_tc_pair_kernel<KIND, T, SUM, WF>;
+    auto kern = qmm_tc_pair_kernel<KIND, T, WF>;
     FNN_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
                    FNN_ERR_DISPATCH);
     FNN_CUDA_CHECK(launch_pdl_cluster(kern, grid, 2, threads, smem, ctx, map_w, map_a, map_s, p), FNN_ERR_DISPATCH);
@@ -486,23 +480,20 @@ PairTiling pair_tiling(int fmt, int M, int N, int K, int sm_count) {
     const int terms = cb ? 1 : (f8 && M < 128) ? 3 : 2;
     PairTiling best{};
     double best_cost = 0;
-    for (int sum = 0; sum < 2; ++sum) {
-        if (sum ? !f8 : terms == 3) continue;   // three terms do not split into two halves of planes
-        const int mb_max = (sum || cb) ? 256 : 128, gran = (sum || cb) ? 32 : 16;
-        for (int q = (M + mb_max - 1) / mb_max, i = 0; i < 8; ++i, ++q) {
-            const int rows = (M + q - 1) / q;
-            const int Mb = std::min(mb_max, (rows + gran - 1) / gran * gran);
-            const int m_tiles = (M + Mb - 1) / Mb;
-            const long long waves = ((long long)n_tiles * m_tiles + pairs - 1) / pairs;
-            const int mmas = sum ? 4 * terms : cb ? 8 : 4, cols = sum || cb ? Mb : 2 * Mb;
-            double t_block = mmas * std::max(90, cols / 2) / 1850.0;   // microseconds
-            // widening the weights (codebook: and three stages of 74 KB)
-            t_block = std::max(t_block, cb ? std::max(0.75, Mb / 256.0) : fmt == FNN_FMT_I4 ? 0.25 : 0.0);
-            const double cost = (double)waves * kblocks * t_block + 0.02 * Mb;
-            if (best.Mb == 0 || cost < best_cost) {
-                best_cost = cost;
-                best = {Mb, m_tiles, terms, sum != 0, cost};
-            }
+    // terms x rows columns: at most 256, a multiple of 32
+    const int mb_max = terms == 1 ? 256 : terms == 2 ? 128 : 64, gran = terms == 2 ? 16 : 32;
+    for (int q = (M + mb_max - 1) / mb_max, i = 0; i < 8; ++i, ++q) {
+        const int rows = (M + q - 1) / q;
+        const int Mb = std::min(mb_max, (rows + gran - 1) / gran * gran);
+        const int m_tiles = (M + Mb - 1) / Mb;
+        const long long waves = ((long long)n_tiles * m_tiles + pairs - 1) / pairs;
+        double t_block = (cb ? 8 : 4) * std::max(90, terms * Mb / 2) / 1850.0;   // microseconds
+        // widening the weights (codebook: and three stages of 74 KB)
+        t_block = std::max(t_block, cb ? std::max(0.75, Mb / 256.0) : fmt == FNN_FMT_I4 ? 0.25 : 0.0);
+        const double cost = (double)waves * kblocks * t_block + 0.02 * Mb;
+        if (best.Mb == 0 || cost < best_cost) {
+            best_cost = cost;
+            best = {Mb, m_tiles, terms, cost};
         }
     }
     return best;
@@ -524,15 +515,14 @@ int launch_qmm_tc_pair(fnn_cuda_ctx *ctx, const QmmArgs &a) {
     const PairTiling tl = pair_tiling(a.w->fmt, (int)a.M, (int)a.w->N, (int)a.w->K, ctx->sm_count);
     switch (a.w->fmt) {
     case FNN_FMT_I8:
-        return launch_pair<KIND_I8, 2, false, WF_TMA>(ctx, a, tl);
+        return launch_pair<KIND_I8, 2, WF_TMA>(ctx, a, tl);
     case FNN_FMT_I4:
-        return launch_pair<KIND_I8, 2, false, WF_I4>(ctx, a, tl);
+        return launch_pair<KIND_I8, 2, WF_I4>(ctx, a, tl);
     case FNN_FMT_F8:
     case FNN_FMT_F4:
-        if (tl.terms == 3) return launch_pair<KIND_F8, 3, true, WF_TMA>(ctx, a, tl);
-        return tl.sum ? launch_pair<KIND_F8, 2, true, WF_TMA>(ctx, a, tl) : launch_pair<KIND_F8, 2, false, WF_TMA>(ctx, a, tl);
+        return tl.terms == 3 ? launch_pair<KIND_F8, 3, WF_TMA>(ctx, a, tl) : launch_pair<KIND_F8, 2, WF_TMA>(ctx, a, tl);
     case FNN_FMT_I4CB:
-        return launch_pair<KIND_F16, 1, false, WF_CB>(ctx, a, tl);
+        return launch_pair<KIND_F16, 1, WF_CB>(ctx, a, tl);
     }
     return set_error(FNN_ERR_UNSUPPORTED, "qmatmul: tcgen05 path does not cover format %d", a.w->fmt);
 }

@@ -5,6 +5,7 @@ Bars: 1e-3 of the output's RMS where the activations travel as int8 pairs (15-bi
 triples; 1e-2 for two e4m3 terms (each keeps four significant bits of what is left: 2^-8 of the row maximum) and for
 fp16 operands, as for the other tests of these kernels.
 """
+import numpy as np
 import pytest
 
 import oracle as orc
@@ -51,3 +52,35 @@ def test_k_shares_of_a_cluster(backend, fmt, kn):
 @pytest.mark.parametrize("kn", [(128, 256), (520, 129), (777, 513), (1152, 1100)])
 def test_two_sm_tiles(backend, fmt, kn):
     check(backend, fmt, *kn, [65, 127, 128, 129, 161, 257, 530])
+
+
+def random_codes(fmt, k, n, seed):
+    """A weight of random finite codes (no host quantization: these layers are large)."""
+    rng = np.random.Generator(np.random.Philox(seed))
+    per_word = 4 if fmt in (orc.FMT_I8, orc.FMT_F8) else 8
+    words = rng.integers(0, 1 << 32, (n, -(-k // per_word)), dtype=np.uint32)
+    if fmt == orc.FMT_F8:
+        words &= np.uint32(0xB7B7B7B7)   # no exponent 15 (exponent bit 3 off): |v| < 2
+    tail = np.zeros(16, np.uint32)
+    return orc.QWeight(fmt, n, k, np.concatenate([words.ravel(), tail]), np.full(n, 0.01, np.float32),
+                       np.zeros(n if fmt == orc.FMT_F4 else 0, np.float32))
+
+
+# Three e4m3 terms keep 12 bits of each activation: 1.55e-5 of the output's norm at any K as long as every term has f32
+# accumulators of its own (1.9e-5 at K=8192 when they share one).
+@pytest.mark.parametrize("fmt", [orc.FMT_F8, orc.FMT_F4])
+@pytest.mark.parametrize("k,n,m", [(8192, 18944, 100), (4096, 18944, 65), (2048, 4096, 127)])
+def test_three_terms_keep_their_accuracy(backend, fmt, k, n, m):
+    q = random_codes(fmt, k, n, 730 + k)
+    x = normal(731 + m, (m, k), 1.0)
+    rig = Rig(backend, q, m)
+    try:
+        got = rig.run(x, None, L.EPI_NONE, L.PATH_TC)[:, 256:512]
+        row = (len(q.words) - 16) // n
+        part = orc.QWeight(fmt, 256, k, np.concatenate([q.words[256 * row:512 * row], q.words[-16:]]), q.scales[256:512],
+                           q.zeros[256:512])
+        want = x.astype(np.float64) @ orc.dequant(part).astype(np.float64).T
+        err = np.linalg.norm(got - want) / np.linalg.norm(want)
+        assert err <= 1.7e-5, (orc.FMT_NAMES[fmt], k, n, m, err)
+    finally:
+        rig.close()
