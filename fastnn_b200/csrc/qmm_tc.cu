@@ -270,7 +270,12 @@ struct TcParams {
 
 // ATOMS: 128-byte swizzle atoms of K per pipeline stage (2 for fp16 operands: a stage is 128 k for
 // every format).  Shared memory per stage: operand tile, raw tile (transformed formats), activations.
-template <int KIND, int T, int WF>
+// W: batch rows per epilogue chunk.  Each chunk is a chain of TMEM loads, shuffles and stores, so 16 at a time where
+// whole tiles are finished (us of a wave of 148 tiles of 128 rows, K=512, SiLU, 8 / 16: I8 5.6 / 4.65, codebook 6.1 / 5.4,
+// FP8 5.4 / 4.4).  Eight where the CTAs of a cluster deal the chunks out, for tiles of a single chunk of 16, which
+// would leave half of the warps idle, and for three terms, whose 48 accumulators a thread cost the registers that the
+// next kernel's early blocks need (FP4 64 rows K=2048: 11.0 / 12.3).
+template <int KIND, int T, int WF, int W>
 __global__ void __launch_bounds__((2 + kEpiWarps + xf_warps(WF)) * 32, 1)
 qmm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a,
               const __grid_constant__ CUtensorMap map_s, TcParams p) {
@@ -522,7 +527,7 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
         // taking alternate 8-column chunks) ----------------
         pdl_wait();   // dq, rowsum and the output buffer belong to kernels before this one
         const int quad = warp & 3, grp = (warp - 2) >> 2;
-        constexpr int W = 8, kStep = W * (kEpiWarps / 4);   // columns per chunk; per round of a quadrant's warps
+        constexpr int kStep = W * (kEpiWarps / 4);   // columns per round of a quadrant's warps
         int as = 0;
         uint32_t aphase = 0;
         const bool has_zero = p.zeros != nullptr;
@@ -555,7 +560,7 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
 #pragma unroll
                     for (int t = 0; t < T; ++t) {
                         uint32_t x[W];
-                        tmem_ld8(t_base + (uint32_t)(t * p.Mb + c0), x);
+                        tmem_ld_cols(t_base + (uint32_t)(t * p.Mb + c0), x);
                         tmem_ld_wait();
 #pragma unroll
                         for (int j = 0; j < W; ++j) s_dump[(t * p.Mb + c0 + j) * kTileN + row] = __uint_as_float(x[j]);
@@ -568,7 +573,7 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
             for (int c0 = chunk0; c0 < p.Mb; c0 += parts * kStep) {
                 uint32_t r[T][W];
 #pragma unroll
-                for (int t = 0; t < T; ++t) tmem_ld8(t_base + (uint32_t)(t * p.Mb + c0), r[t]);
+                for (int t = 0; t < T; ++t) tmem_ld_cols(t_base + (uint32_t)(t * p.Mb + c0), r[t]);
                 const float fac_next = load_rowfac(mt, c0 + parts * kStep);   // next chunk's
                 tmem_ld_wait();
                 for (int q = 0; q < parts; ++q) {   // the other shares, in a fixed order
@@ -925,7 +930,9 @@ int launch_tc(fnn_cuda_ctx *ctx, const QmmArgs &a, uint8_t *fixed_scratch = null
     if (parts > 1) smem = std::max(smem, kHalfSmem);
     const int grid = parts > 1 ? tiles * parts : std::min(tiles, ctx->sm_count);
     const int threads = (2 + kEpiWarps + xf_warps(WF)) * 32;
-    auto kern = qmm_tc_kernel<KIND, T, WF>;
+    auto kern = qmm_tc_kernel<KIND, T, WF, 8>;
+    if constexpr (T < 3)
+        if (parts == 1 && Mb > 16) kern = qmm_tc_kernel<KIND, T, WF, 16>;
     FNN_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
                    FNN_ERR_DISPATCH);
     if (parts > 1) {
