@@ -131,33 +131,38 @@ act_prep_kernel(const float *act, int M, int K, int Kp, uint8_t *bq, float *dq, 
     }
 }
 
-// The same rewrite for rows of a multiple of 8 and at most 16384 elements that start on 16 bytes
-// (every layer of a real model): the row is read once, eight consecutive elements per thread and
+// The same rewrite for rows of at most 32768 elements: the row is read once, eight consecutive elements per thread and
 // step with all loads in flight together, stays in registers between the scan and the rewrite, and
-// every plane is written eight bytes at a time.
-constexpr int kPrepHold = 8;   // units of eight elements a thread can hold
-// HOLD: 2, 4 or 8 units, the smallest that covers the row: fewer registers (more rows at once on an SM, and room beside
-// the main kernel before it) and less code to fetch, which a kernel of two microseconds notices.
-template <int KIND, int T, bool PERM8, int HOLD>
+// every plane is written eight bytes at a time.  (The loop above is a chain of two passes of 4-byte loads, about 8 us
+// for K=11308.)
+constexpr int kPrepHold = 16;   // units of eight elements a thread can hold
+// HOLD: 2, 4, 8 or 16 units, the smallest that covers the row: fewer registers (more rows at once on an SM, and room
+// beside the main kernel before it) and less code to fetch, which a kernel of two microseconds notices.
+// VEC: rows of a multiple of four elements that start on 16 bytes (every layer of a real model); else 4-byte loads.
+template <int KIND, int T, bool PERM8, int HOLD, bool VEC>
 __global__ void __launch_bounds__(256)
 act_prep_regs_kernel(const float *act, int M, int K, int Kp, uint8_t *bq, float *dq, float *rowsum) {
     __shared__ float s_max[8], s_sum[8];
     pdl_launch_dependents();
     pdl_wait();
     const int m = blockIdx.x, tid = threadIdx.x;
-    const float4 *row4 = reinterpret_cast<const float4 *>(act + (size_t)m * K);
-    const int units = K >> 3;
+    const float *row = act + (size_t)m * K;
+    const float4 *row4 = reinterpret_cast<const float4 *>(row);
+    const int units = (K + 7) >> 3;   // the last one may be partly past the row: zeros there
     float v[HOLD][8];
 #pragma unroll
     for (int i = 0; i < HOLD; ++i) {
         const int u = tid + i * 256;
-        float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
-        if (u < units) {
-            a = ld_after_wait(row4 + 2 * u);
-            b = ld_after_wait(row4 + 2 * u + 1);
+        if (VEC) {
+            float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
+            if (8 * u < K) a = ld_after_wait(row4 + 2 * u);
+            if (8 * u + 4 < K) b = ld_after_wait(row4 + 2 * u + 1);
+            v[i][0] = a.x; v[i][1] = a.y; v[i][2] = a.z; v[i][3] = a.w;
+            v[i][4] = b.x; v[i][5] = b.y; v[i][6] = b.z; v[i][7] = b.w;
+        } else {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) v[i][j] = 8 * u + j < K ? ld_after_wait(row + 8 * u + j) : 0.0f;
         }
-        v[i][0] = a.x; v[i][1] = a.y; v[i][2] = a.z; v[i][3] = a.w;
-        v[i][4] = b.x; v[i][5] = b.y; v[i][6] = b.z; v[i][7] = b.w;
     }
     float mx = 0.0f, sum = 0.0f;
 #pragma unroll
@@ -193,7 +198,7 @@ act_prep_regs_kernel(const float *act, int M, int K, int Kp, uint8_t *bq, float 
             dq[m] = ldexpf(1.0f, -e);
             rowsum[m] = sum;
         }
-        uint4 *dst = reinterpret_cast<uint4 *>(bq + (size_t)m * Kp);   // Kp = 2 K bytes here
+        uint4 *dst = reinterpret_cast<uint4 *>(bq + (size_t)m * Kp);   // Kp = 16 bytes per unit here
 #pragma unroll
         for (int i = 0; i < HOLD; ++i) {
             const int u = tid + i * 256;
@@ -214,10 +219,10 @@ act_prep_regs_kernel(const float *act, int M, int K, int Kp, uint8_t *bq, float 
     if (tid == 0) {
         dq[m] = step;
         rowsum[m] = sum;
-        if (Kp > K) {   // K is 8 mod 16: one more unit of zeros pads the row to 16 bytes
+        if (Kp > 8 * units) {   // one more unit of zeros pads the row to 16 bytes
 #pragma unroll
             for (int i = 0; i < T; ++i)
-                *reinterpret_cast<uint2 *>(bq + ((size_t)i * M + m) * Kp + K) = make_uint2(0u, 0u);
+                *reinterpret_cast<uint2 *>(bq + ((size_t)i * M + m) * Kp + 8 * units) = make_uint2(0u, 0u);
         }
     }
 #pragma unroll
@@ -753,16 +758,23 @@ int tc::encode_block_scale_map(CUtensorMap *map, const fnn_cuda_qweight *w) {
 
 namespace {
 
+template <int KIND, int T, bool PERM8, bool VEC>
+auto prep_kernel(int K) {
+    return K <= 2 * 256 * 8   ? act_prep_regs_kernel<KIND, T, PERM8, 2, VEC>
+           : K <= 4 * 256 * 8 ? act_prep_regs_kernel<KIND, T, PERM8, 4, VEC>
+           : K <= 8 * 256 * 8 ? act_prep_regs_kernel<KIND, T, PERM8, 8, VEC>
+                              : act_prep_regs_kernel<KIND, T, PERM8, kPrepHold, VEC>;
+}
+
 template <int KIND, int T, bool PERM8>
 int launch_prep(fnn_cuda_ctx *ctx, const QmmArgs &a, int Kp, uint8_t *bq, float *dq, float *rowsum) {
     const int M = (int)a.M, K = (int)a.w->K;
     // same shared-memory carve-out as the main kernel: alternating carve-outs between consecutive
     // kernels makes every SM reconfigure (and drain) twice per call
-    const bool regs_ok = K % 8 == 0 && K <= kPrepHold * 256 * 8 && (reinterpret_cast<uintptr_t>(a.a) & 15) == 0;
-    auto prep = !regs_ok             ? act_prep_kernel<KIND, T, PERM8>
-                : K <= 2 * 256 * 8 ? act_prep_regs_kernel<KIND, T, PERM8, 2>
-                : K <= 4 * 256 * 8 ? act_prep_regs_kernel<KIND, T, PERM8, 4>
-                                   : act_prep_regs_kernel<KIND, T, PERM8, kPrepHold>;
+    const bool vec = K % 4 == 0 && (reinterpret_cast<uintptr_t>(a.a) & 15) == 0;
+    auto prep = K > kPrepHold * 256 * 8 ? act_prep_kernel<KIND, T, PERM8>
+                : vec                   ? prep_kernel<KIND, T, PERM8, true>(K)
+                                        : prep_kernel<KIND, T, PERM8, false>(K);
     FNN_CUDA_CHECK(cudaFuncSetAttribute(prep, cudaFuncAttributePreferredSharedMemoryCarveout,
                                         cudaSharedmemCarveoutMaxShared),
                    FNN_ERR_DISPATCH);

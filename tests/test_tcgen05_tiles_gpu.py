@@ -54,6 +54,14 @@ def test_two_sm_tiles(backend, fmt, kn):
     check(backend, fmt, *kn, [65, 127, 128, 129, 161, 257, 530])
 
 
+# the rewrite of the rows: both sides of the lengths a thread's registers take, rows that start on 16 bytes and rows that do
+# not, the last unit of eight whole, short, and followed by one of padding; the longest ones in two passes
+@pytest.mark.parametrize("fmt", [orc.FMT_I8, orc.FMT_I4, orc.FMT_F8])
+@pytest.mark.parametrize("k", [1028, 4096, 4099, 8196, 8209, 16388, 20002, 32768, 32777])
+def test_rewritten_rows_of_any_length(backend, fmt, k):
+    check(backend, fmt, k, 40, [3, 9])
+
+
 def random_codes(fmt, k, n, seed):
     """A weight of random finite codes (no host quantization: these layers are large)."""
     rng = np.random.Generator(np.random.Philox(seed))
