@@ -420,10 +420,10 @@ size_t qmm_tc_scratch_bytes(const fnn_cuda_qweight *w, size_t M);   // of the si
 struct PairTiling {
     int Mb = 0, m_tiles = 0;   // batch rows per tile, tiles over the batch
     int terms = 0;             // narrow terms per activation
-    double cost = 0;           // estimated microseconds of the main loops and the last epilogue
+    double cost = 0;           // estimated microseconds
 };
 PairTiling pair_tiling(int fmt, int M, int N, int K, int sm_count);
-double tc_single_cost(const fnn_cuda_ctx *ctx, const fnn_cuda_qweight *w, size_t M);   // of the single-SM kernel
+double tc_single_cost(const fnn_cuda_ctx *ctx, const fnn_cuda_qweight *w, size_t M);   // estimate of the single-SM kernel
 bool qmm_tc_uses_pair(const fnn_cuda_ctx *ctx, const fnn_cuda_qweight *w, size_t M);
 int launch_qmm_tc_pair(fnn_cuda_ctx *ctx, const QmmArgs &args);
 void free_qweight_aux(fnn_cuda_qweight *w);

@@ -825,24 +825,29 @@ namespace {
 // A cluster lives inside one GPC, so fewer of the larger ones run at once (74, 45, 33, 26, 22 of 2 .. 6 on a
 // B200, and only 15 of 8); a cluster that has to wait for a second round costs more than the split gains
 // (48 tiles in 3 parts: 19.9 us against 11.8 in 2).
-struct Split {
-    int parts;
-    double cost;   // estimated microseconds of the main loops
-};
-Split split_parts(const fnn_cuda_ctx *ctx, int tiles, int kblocks, int cols, int wf) {
+int split_parts(const fnn_cuda_ctx *ctx, int tiles, int kblocks, int cols, int wf) {
     static const int kActive[] = {0, 148, 74, 45, 33, 26, 22};   // of 148 SMs
     const double t_step = (wf == WF_CB) ? 0.8 : 0.15 + 0.25 * cols / 256.0;
     const double t_part = 0.8 + 0.4 * cols / 128.0;
     const int waves = (tiles + ctx->sm_count - 1) / ctx->sm_count;
-    Split best{1, waves * kblocks * t_step};
+    int best = 1;
+    double best_cost = waves * kblocks * t_step;
     for (int q = 2; q <= 6 && q <= kblocks; ++q) {
         if (tiles > kActive[q] * ctx->sm_count / 148) break;
         const bool crowded = 4 * tiles * q > 3 * ctx->sm_count;
         const double cost = (kblocks + q - 1) / q * t_step + t_part * (q - 1) + (crowded ? 1.5 : 0.0);
-        if (cost < best.cost) best = {q, cost};
+        if (cost < best_cost) {
+            best = q;
+            best_cost = cost;
+        }
     }
     return best;
 }
+
+// TMEM columns of a widened operand tile, and accumulator buffers: two (the next tile's MMAs run under a tile's epilogue)
+// where the widened operands of at least four stages fit beside them in the 512 columns, else one.
+constexpr int operand_cols(int wf) { return wf == WF_TMA ? 0 : wf == WF_I4 ? 32 : 64; }
+int acc_buffers(int cols, int slot_cols) { return 2 * cols + 4 * slot_cols <= 512 ? 2 : 1; }
 
 // Batch rows per tile: T * Mb is the MMA N (multiple of 16, at most 256), tiles of equal height.  The codebook format stops at
 // 128: two accumulator buffers then fit beside the widened operands, and the epilogue of a tile runs under the
@@ -868,7 +873,7 @@ int launch_tc(fnn_cuda_ctx *ctx, const QmmArgs &a, uint8_t *fixed_scratch = null
     const int n_tiles = (N + kTileN - 1) / kTileN;
     const int kblocks = (Kbytes + kKBlockBytes * ATOMS - 1) / (kKBlockBytes * ATOMS);
     const int tiles = n_tiles * m_tiles;
-    const int parts = split_parts(ctx, tiles, kblocks, T * Mb, WF).parts;
+    const int parts = split_parts(ctx, tiles, kblocks, T * Mb, WF);
     int rc = FNN_OK;
     uint8_t *bq;
     if (fixed_scratch) {
@@ -923,10 +928,8 @@ int launch_tc(fnn_cuda_ctx *ctx, const QmmArgs &a, uint8_t *fixed_scratch = null
     const int raw_bytes = (WF == WF_TMA) ? 0 : kTileN * 64 + (WF == WF_CB ? kTileN * 16 : 0);
     int stages = (int)((200 * 1024) / (size_t)(a_bytes + b_stride + raw_bytes));
     stages = std::max(2, std::min(stages, 8));
-    // Accumulators: two buffers (the next tile's MMAs run under a tile's epilogue) where the widened
-    // operands of at least four stages fit beside them in the 512 TMEM columns, else one.
-    const int slot_cols = (WF == WF_TMA) ? 0 : 32 * ATOMS;
-    p.nbuf = (2 * T * Mb + 4 * slot_cols <= 512) ? 2 : 1;
+    const int slot_cols = operand_cols(WF);
+    p.nbuf = acc_buffers(T * Mb, slot_cols);
     if (slot_cols) stages = std::min(stages, (512 - p.nbuf * T * Mb) / slot_cols);
     p.ncols = 32;
     while (p.ncols < p.nbuf * T * Mb + stages * slot_cols) p.ncols <<= 1;
@@ -961,21 +964,41 @@ int launch_tc(fnn_cuda_ctx *ctx, const QmmArgs &a, uint8_t *fixed_scratch = null
 
 int dispatch_tc(fnn_cuda_ctx *ctx, const QmmArgs &a, uint8_t *fixed, size_t fixed_bytes);
 
-namespace {
-int terms_of(const fnn_cuda_qweight *w, size_t M) {
-    return w->fmt == FNN_FMT_I4CB ? 1 : (w->fmt == FNN_FMT_F8 || w->fmt == FNN_FMT_F4) && M < 128 ? 3 : 2;
+int tc::tc_terms(int fmt, size_t M) {
+    return fmt == FNN_FMT_I4CB ? 1 : (fmt == FNN_FMT_F8 || fmt == FNN_FMT_F4) && M < 128 ? 3 : 2;
 }
-}  // namespace
+
+// Fitted (least squares of the logarithms, 6 to 7 % rms) to chains of one layer with a SiLU: 786 shapes from M=65 on, both
+// kernels and up to three tile heights each.
+const tc::TileCosts &tc::tile_costs(int fmt, int terms) {
+    static const TileCosts i8 = {3.28, 0.283, 0.091, 0.028, 0.53, 1.49, 3.40, 0.110, 0.207, 0.037};
+    static const TileCosts i4 = {2.89, 0.135, 0.200, 0.039, 0.0, 1.56, 3.26, 0.194, 0.125, 0.039};
+    static const TileCosts f8x3 = {2.53, 0.064, 0.290, 0.043, 2.81, 0.0, 2.78, 0.116, 0.138, 0.042};
+    static const TileCosts f8x2 = {3.43, 0.111, 0.267, 0.028, 0.0, 1.70, 3.59, 0.050, 0.293, 0.036};
+    static const TileCosts cb = {2.91, 0.450, 0.297, 0.033, 0.0, 2.45, 2.45, 0.699, 0.281, 0.037};
+    switch (fmt) {
+    case FNN_FMT_I8: return i8;
+    case FNN_FMT_I4: return i4;
+    case FNN_FMT_I4CB: return cb;
+    default: return terms == 3 ? f8x3 : f8x2;
+    }
+}
 
 size_t qmm_tc_scratch_bytes(const fnn_cuda_qweight *w, size_t M) {
-    return prep_layout(terms_of(w, M), w->fmt == FNN_FMT_I4CB ? 2 : 1, M, w->K).bytes;
+    return prep_layout(tc_terms(w->fmt, M), w->fmt == FNN_FMT_I4CB ? 2 : 1, M, w->K).bytes;
 }
 
 double tc_single_cost(const fnn_cuda_ctx *ctx, const fnn_cuda_qweight *w, size_t M) {
-    const bool cb = w->fmt == FNN_FMT_I4CB;
-    const int terms = terms_of(w, M), Mb = batch_rows(terms, (int)M);
+    const int terms = tc_terms(w->fmt, M), Mb = batch_rows(terms, (int)M), cols = terms * Mb;
+    const int wf = w->fmt == FNN_FMT_I4CB ? WF_CB : w->fmt == FNN_FMT_I4 ? WF_I4 : WF_TMA;
     const int tiles = (int)(div_ceil(w->N, (size_t)kTileN) * div_ceil(M, (size_t)Mb));
-    return split_parts(ctx, tiles, (int)div_ceil(w->K, (size_t)kKBlockBytes), terms * Mb, cb ? WF_CB : WF_TMA).cost;
+    const int kblocks = (int)div_ceil(w->K, (size_t)kKBlockBytes), parts = split_parts(ctx, tiles, kblocks, cols, wf);
+    const TileCosts &c = tile_costs(w->fmt, terms);
+    const double step = c.step + c.step_256 * cols / 256.0, epilogue = c.row * Mb;
+    if (parts > 1)
+        return c.fixed + (kblocks + parts - 1) / parts * step + (c.part + c.part_128 * cols / 128.0) * (parts - 1) +
+               epilogue / parts;
+    return c.fixed + tile_time(tiles, ctx->sm_count, kblocks * step, epilogue, acc_buffers(cols, operand_cols(wf)) == 2);
 }
 
 bool qmm_tc_supported(const fnn_cuda_qweight *w, size_t M) {

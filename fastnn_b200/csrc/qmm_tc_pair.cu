@@ -468,47 +468,40 @@ int launch_pair(fnn_cuda_ctx *ctx, const QmmArgs &a, const PairTiling &tl) {
 
 }  // namespace
 
-// Batch rows per pair tile and how the terms meet.  All pairs run whole tiles, so the time is waves x K blocks x the
-// MMAs of a K block, plus the epilogue of the last tile, which nothing hides (about 0.02 us per batch row).
-// An MMA takes max(90, columns / 2) cycles.  The accumulators of two tiles share the 512 TMEM columns.
-// Among the first tile heights that cover M the cheapest is taken: I8, M = 512, N = 11008 is 172
-// tiles of 128 rows (three waves of 128 on 74 pairs) or 215 tiles of 112 (three waves of 112).
+// Batch rows per pair tile.  All pairs run whole tiles and the accumulators of two tiles share the 512 TMEM columns
+// (tile_time).  Among the first tile heights that cover M the cheapest is taken, a lower one only if it is 3 % cheaper: more
+// tiles also move more bytes.  I8, M = 512, N = 11008 is 172 tiles of 128 rows (three waves of 128 on 74 pairs) or
+// 215 tiles of 112 (three waves of 112).
 PairTiling pair_tiling(int fmt, int M, int N, int K, int sm_count) {
-    const bool f8 = fmt == FNN_FMT_F8 || fmt == FNN_FMT_F4, cb = fmt == FNN_FMT_I4CB;
     const int n_tiles = (N + kPairRows - 1) / kPairRows, pairs = std::max(1, sm_count / 2);
     const int kblocks = (K + kKBlockBytes - 1) / kKBlockBytes;
-    const int terms = cb ? 1 : (f8 && M < 128) ? 3 : 2;
+    const int terms = tc_terms(fmt, M);
+    const TileCosts &c = tile_costs(fmt, terms);
     PairTiling best{};
-    double best_cost = 0;
     // terms x rows columns: at most 256, a multiple of 32
     const int mb_max = terms == 1 ? 256 : terms == 2 ? 128 : 64, gran = terms == 2 ? 16 : 32;
     for (int q = (M + mb_max - 1) / mb_max, i = 0; i < 8; ++i, ++q) {
         const int rows = (M + q - 1) / q;
         const int Mb = std::min(mb_max, (rows + gran - 1) / gran * gran);
         const int m_tiles = (M + Mb - 1) / Mb;
-        const long long waves = ((long long)n_tiles * m_tiles + pairs - 1) / pairs;
-        double t_block = (cb ? 8 : 4) * std::max(90, terms * Mb / 2) / 1850.0;   // microseconds
-        // widening the weights (codebook: and three stages of 74 KB)
-        t_block = std::max(t_block, cb ? std::max(0.75, Mb / 256.0) : fmt == FNN_FMT_I4 ? 0.25 : 0.0);
-        const double cost = (double)waves * kblocks * t_block + 0.02 * Mb;
-        if (best.Mb == 0 || cost < best_cost) {
-            best_cost = cost;
-            best = {Mb, m_tiles, terms, cost};
-        }
+        const double step = c.pair_step + c.pair_step_256 * terms * Mb / 256.0;
+        const double cost = c.pair_fixed + tile_time((long long)n_tiles * m_tiles, pairs, kblocks * step, c.pair_row * Mb, true);
+        if (best.Mb == 0 || cost < 0.97 * best.cost) best = {Mb, m_tiles, terms, cost};
     }
     return best;
 }
 
-// From 65 batch rows on (codebook: 129, its lookups bound both kernels alike below), unless the single-SM kernel gets
-// further by splitting K: the estimates of both, with 1.5 us for the single-SM kernel's longer last epilogue.
-// Measured, us single / pair: I8 K=4096 N=4096 M=64 13.5 (11 split) / 12.5, M=96 13.7 split / 11.9; I8 N=11008 M=96
-// 18.3 / 16.7, M=256 32.7 / 24.9; I4 N=11008 M=96 20.7 / 17.3; I4 M=128 K=14336 N=4096 25.5 split / 36.6.
-// Codebook: M=512 K=4096 N=14336 89.3 / 78.3, M=4096 569 / 476, K=2048 N=8192 188 / 156; short K is the epilogue's (M=674 K=512
-// N=8320 30.3 / 35.8: below 2048 never).
+// From 65 batch rows on, where the estimate is 4 % below the single-SM kernel's (which may split K); the codebook format
+// from K=2560 on a tie, where the fit understates the single-SM kernel.  Over 760 shapes of all formats (M 65 to
+// 4096, K 128 to 8192, N 512 to 28672) the kernel and tile height so chosen are 0.6 % from the fastest on average.
+// us single / pair: I8 N=4096 M=100 K=4096 14.9 / 11.5; I8 N=11008 M=256 K=4096 32.4 / 25.2; I4 N=28672 M=1024 K=4096 203 /
+// 173; I4 N=4096 M=128 K=14336 25.5 split / 36.6.  Codebook: N=16384 M=2048 K=512 87.0 / 89.6, K=1024 108 / 118, K=2048 177 /
+// 173; N=16384 M=1024 K=4096 166 / 147; N=4096 M=333 K=4096 26.8 split / 36.6.
 bool qmm_tc_uses_pair(const fnn_cuda_ctx *ctx, const fnn_cuda_qweight *w, size_t M) {
-    if (M <= (w->fmt == FNN_FMT_I4CB ? 128u : 64u) || (w->fmt == FNN_FMT_I4CB && w->K < 2048)) return false;
+    if (M <= 64) return false;
     const PairTiling tl = pair_tiling(w->fmt, (int)M, (int)w->N, (int)w->K, ctx->sm_count);
-    return tl.cost < tc_single_cost(ctx, w, M) + 1.5;
+    const double margin = w->fmt == FNN_FMT_I4CB && w->K >= 2560 ? 1.0 : 1.04;
+    return tl.cost * margin < tc_single_cost(ctx, w, M);
 }
 
 int launch_qmm_tc_pair(fnn_cuda_ctx *ctx, const QmmArgs &a) {

@@ -307,6 +307,26 @@ int encode_map(CUtensorMap *map, void *base, int rank, const cuuint64_t *dims, c
                CUtensorMapDataType dtype = CU_TENSOR_MAP_DATA_TYPE_UINT8);
 int encode_weight_map(CUtensorMap *map, const fnn_cuda_qweight *w);
 int encode_block_scale_map(CUtensorMap *map, const fnn_cuda_qweight *w);
+// Narrow terms per activation.
+int tc_terms(int fmt, size_t M);
+// Microseconds of the parts of a call, for the choice between the kernels and of the tile height.
+struct TileCosts {
+    // single-SM kernel: a call; a K block of 128 (and what 256 columns add); the epilogue of a batch row of a tile; an
+    // extra CTA of a K split (and what 128 columns add)
+    double fixed, step, step_256, row, part, part_128;
+    // two-SM kernel: a call; a K block (and what 256 columns add); a row's epilogue
+    double pair_fixed, pair_step, pair_step_256, pair_row;
+};
+const TileCosts &tile_costs(int fmt, int terms);
+// Whole tiles in waves over `units` SMs or pairs: the first K loop and the last epilogue are exposed; in between, where the
+// accumulators are double-buffered, the longer of both per wave and half of the shorter, which competes for the
+// same issue slots and shared memory (half: fitted, 0.43 to 0.62 by format); else both.
+inline double tile_time(long long tiles, int units, double main_loop, double epilogue, bool two_buffers) {
+    const double waves = (double)((tiles + units - 1) / units);
+    const double longer = main_loop > epilogue ? main_loop : epilogue, both = main_loop + epilogue;
+    const double wave = two_buffers ? 0.5 * (longer + both) : both;
+    return both + (waves - 1) * wave;
+}
 // Launches the rewrite of the activations as `terms` narrow planes, their row factors and row sums.
 int launch_act_prep(fnn_cuda_ctx *ctx, const QmmArgs &a, int kind, int terms, bool perm8, int Kp, uint8_t *bq, float *dq,
                     float *rowsum);
