@@ -58,6 +58,7 @@ SIGNATURES = {
     "fnn_cuda_qmatmul_ptr": (_int, [_vp, _vp, _vp, _vp, _vp, _sz, _int, _int]),
     "fnn_cuda_qmatmul_noalloc": (_int, [_vp, _vp, _vp, _vp, _vp, _sz, _int]),
     "fnn_cuda_last_path": (_c.c_char_p, [_vp]),
+    "fnn_cuda_last_kernel": (_c.c_char_p, [_vp]),
     "fnn_cuda_ipc_export": (_int, [_vp, _vp]),
     "fnn_cuda_ipc_open": (_int, [_vp, _vp, _c.POINTER(_vp)]),
     "fnn_cuda_ipc_close": (_int, [_vp, _vp]),

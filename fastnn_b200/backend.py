@@ -312,6 +312,9 @@ class CudaBackend:
     def last_path(self) -> str:
         return self.lib.fnn_cuda_last_path(self.ctx).decode()
 
+    def last_kernel(self) -> str:
+        return self.lib.fnn_cuda_last_kernel(self.ctx).decode()
+
     def device_info(self) -> dict:
         sm, ma, mi, mem = ctypes.c_int(), ctypes.c_int(), ctypes.c_int(), ctypes.c_size_t()
         _check(self.lib.fnn_cuda_device_info(self.ctx, ctypes.byref(sm), ctypes.byref(ma),

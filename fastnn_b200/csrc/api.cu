@@ -532,6 +532,7 @@ int fnn_cuda_qmatmul_ptr(fnn_cuda_ctx *ctx, fnn_cuda_qweight *w, const float *a_
 }
 
 const char *fnn_cuda_last_path(fnn_cuda_ctx *ctx) { return ctx ? ctx->last_path : ""; }
+const char *fnn_cuda_last_kernel(fnn_cuda_ctx *ctx) { return ctx ? ctx->last_kernel : ""; }
 
 // ---- column-sharded layers: peer memory and the fused GEMV + all-gather ----------------------
 

@@ -54,6 +54,7 @@ struct fnn_cuda_ctx {
     size_t total_mem = 0;
     uint64_t launches = 0;
     const char *last_path = "";
+    const char *last_kernel = "";
     bool capturing = false;
     uint64_t launches_at_capture = 0;
     cudaEvent_t ev_start[64] = {};

@@ -628,7 +628,7 @@ int launch_mma_fmt(fnn_cuda_ctx *ctx, const QmmArgs &a) {
             rc = launch_mma<FMT, 8>(ctx, a, act, out, M, 0);
         if (rc != FNN_OK) return rc;
     }
-    ctx->last_path = "mma";
+    ctx->last_path = ctx->last_kernel = "mma";
     return FNN_OK;
 }
 

@@ -726,6 +726,7 @@ int launch8(fnn_cuda_ctx *ctx, const QmmArgs &a, int blocks_per_sm = 1) {
     FNN_CUDA_CHECK(launch_pdl(kern, sz.grid, kG8 * kW8 * 32, sz.smem, ctx, p), FNN_ERR_DISPATCH);
     ctx->launches++;
     ctx->last_path = "mma8";
+    ctx->last_kernel = p.planes ? "mma8-rewritten" : "mma8";
     return FNN_OK;
 }
 

@@ -288,7 +288,7 @@ int launch_one(fnn_cuda_ctx *ctx, const QmmArgs &a) {
                                                 (int)w->N, (int)w->K, KT, a.epilogue);
     FNN_CUDA_CHECK(cudaGetLastError(), FNN_ERR_DISPATCH);
     ctx->launches++;
-    ctx->last_path = "rows";
+    ctx->last_path = ctx->last_kernel = "rows";
     return FNN_OK;
 }
 

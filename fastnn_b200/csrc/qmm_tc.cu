@@ -957,6 +957,7 @@ int launch_tc(fnn_cuda_ctx *ctx, const QmmArgs &a, uint8_t *fixed_scratch = null
     }
     ctx->launches++;
     ctx->last_path = fixed_scratch ? "tc-noalloc" : "tc";
+    ctx->last_kernel = parts > 1 ? "tc-split" : "tc";
     return FNN_OK;
 }
 

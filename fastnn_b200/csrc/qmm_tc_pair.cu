@@ -463,6 +463,7 @@ int launch_pair(fnn_cuda_ctx *ctx, const QmmArgs &a, const PairTiling &tl) {
     FNN_CUDA_CHECK(launch_pdl_cluster(kern, grid, 2, threads, smem, ctx, map_w, map_a, map_s, p), FNN_ERR_DISPATCH);
     ctx->launches++;
     ctx->last_path = "tc";
+    ctx->last_kernel = "tc-pair";
     return FNN_OK;
 }
 

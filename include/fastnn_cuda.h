@@ -201,6 +201,9 @@ int fnn_cuda_qmatmul_noalloc(fnn_cuda_ctx *ctx, fnn_cuda_qweight *w, const float
                              float *out_dev, const float *bias_dev, size_t M, int epilogue);
 /* Name of the kernel family the last fnn_cuda_qmatmul on `ctx` launched. */
 const char *fnn_cuda_last_path(fnn_cuda_ctx *ctx);
+/* Which kernel of that family it was: "rows", "mma", "mma8" or "mma8-rewritten" (several rows, rewritten once
+ * for all blocks), "tc" (one SM per tile), "tc-split" (a cluster shares a tile's K) or "tc-pair" (two SMs per tile). */
+const char *fnn_cuda_last_kernel(fnn_cuda_ctx *ctx);
 
 /* ---- column-sharded layers on the GPUs of one node --------------------------------------------
  * No counterpart in the reference (it has no collective of any kind).  A layer is sharded by
