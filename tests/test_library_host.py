@@ -76,3 +76,11 @@ def test_quant_size_helpers():
     assert lib.fnn_quant_packed_bytes(L.FMT_F8, 3, 20) == (3 * 5 + 16) * 4
     assert lib.fnn_quant_num_scales(L.FMT_I4CB, 3, 70) == 9
     assert lib.fnn_quant_packed_bytes(99, 3, 20) == 0
+
+
+def test_documented_build_lists_every_source():
+    """The build script that INTEGRATION.md gives compiles the same CUDA sources as this repository's build."""
+    from fastnn_b200 import build
+    text = open(os.path.join(ROOT, "INTEGRATION.md")).read()
+    listed = re.search(r"let src = \[(.*?)\];", text, flags=re.S).group(1)
+    assert re.findall(r'"(\w+\.cu)"', listed) == build.CUDA_SOURCES
