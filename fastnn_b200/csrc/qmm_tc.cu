@@ -995,7 +995,7 @@ double tc_single_cost(const fnn_cuda_ctx *ctx, const fnn_cuda_qweight *w, size_t
     const int tiles = (int)(div_ceil(w->N, (size_t)kTileN) * div_ceil(M, (size_t)Mb));
     const int kblocks = (int)div_ceil(w->K, (size_t)kKBlockBytes), parts = split_parts(ctx, tiles, kblocks, cols, wf);
     const TileCosts &c = tile_costs(w->fmt, terms);
-    const double step = c.step + c.step_256 * cols / 256.0, epilogue = c.row * Mb;
+    const double step = c.step + c.step_256 * cols / 256.0, epilogue = c.row * Mb * (splits_sectors(M, w->N) ? 1.8 : 1.0);
     if (parts > 1)
         return c.fixed + (kblocks + parts - 1) / parts * step + (c.part + c.part_128 * cols / 128.0) * (parts - 1) +
                epilogue / parts;

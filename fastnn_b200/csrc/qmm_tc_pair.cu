@@ -486,7 +486,8 @@ PairTiling pair_tiling(int fmt, int M, int N, int K, int sm_count) {
         const int Mb = std::min(mb_max, (rows + gran - 1) / gran * gran);
         const int m_tiles = (M + Mb - 1) / Mb;
         const double step = c.pair_step + c.pair_step_256 * terms * Mb / 256.0;
-        const double cost = c.pair_fixed + tile_time((long long)n_tiles * m_tiles, pairs, kblocks * step, c.pair_row * Mb, true);
+        const double epilogue = c.pair_row * Mb * (splits_sectors(M, N) ? 1.3 : 1.0);
+        const double cost = c.pair_fixed + tile_time((long long)n_tiles * m_tiles, pairs, kblocks * step, epilogue, true);
         if (best.Mb == 0 || cost < 0.97 * best.cost) best = {Mb, m_tiles, terms, cost};
     }
     return best;

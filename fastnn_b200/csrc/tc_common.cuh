@@ -318,6 +318,11 @@ struct TileCosts {
     double pair_fixed, pair_step, pair_step_256, pair_row;
 };
 const TileCosts &tile_costs(int fmt, int terms);
+// Output rows that start off a 32-byte sector, in a result that L2 does not keep until both halves of a sector are written,
+// stretch the epilogues, the single-SM kernel's more (the two SMs of a pair write neighbouring channels at the same
+// time).  us single / pair, rows on sectors -> off: FP8 M=1601 K=1920 N=8704 -> 8718 53.4 / 61.4 -> 84.2 / 71.6, M=3165 K=2560
+// N=3456 -> 3465 59.1 / 61.2 -> 73.7 / 65.1; of 22 MB (M=900 N=6016 -> 6001) 22.5 / 23.1 -> 24.0 / 23.6.
+inline bool splits_sectors(size_t M, size_t N) { return N % 8 != 0 && M * N * 4 > (size_t)32 << 20; }
 // Whole tiles in waves over `units` SMs or pairs: the first K loop and the last epilogue are exposed; in between, where the
 // accumulators are double-buffered, the longer of both per wave and half of the shorter, which competes for the
 // same issue slots and shared memory (half: fitted, 0.43 to 0.62 by format); else both.
