@@ -13,6 +13,8 @@ namespace frag {
 constexpr int kWarpsPerGroup = 8;   // warps that split K of one 16-row tile
 constexpr int kChunkBlocks = 2;     // k-blocks per ring chunk
 
+constexpr int kCbHalf = 8192;   // 8-bit kernel, codebook format: centroid c is carried as v = round(c / cmax * 8191) + 8192
+
 // 16-byte global -> shared copy that bypasses registers; src_bytes == 0 writes zeros.
 __device__ __forceinline__ void cp_async16(void *dst, const void *src, int src_bytes) {
     unsigned d = (unsigned)__cvta_generic_to_shared(dst);

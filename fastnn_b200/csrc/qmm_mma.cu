@@ -513,6 +513,24 @@ __global__ void to_frag_scales_kernel(const float *scales, size_t bpr, size_t N,
     }
 }
 
+// Codebook format: the 16 centroids as the 8-bit kernel's 14-bit fixed point, laid out as its two byte tables
+// (hi = v >> 7: 16 bytes, lo = v & 127: 16 bytes), then the value of one step.  Built once: in the prologue of every block
+// this was 150 instructions behind a trip to memory.
+__global__ void cb_tables_kernel(const float *codebook, uint8_t *tables) {
+    const int j = threadIdx.x & 15;
+    const float c = codebook[j];
+    float cmax = fabsf(c);
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) cmax = fmaxf(cmax, __shfl_xor_sync(0xFFFFFFFFu, cmax, o));
+    const float to_fix = cmax > 0.0f ? (float)(frag::kCbHalf - 1) / cmax : 0.0f;
+    const int v = __float2int_rn(c * to_fix) + frag::kCbHalf;   // 1 .. 16383
+    if (threadIdx.x < 16) {
+        tables[j] = (uint8_t)(v >> 7);
+        tables[16 + j] = (uint8_t)(v & 127);
+    }
+    if (threadIdx.x == 0) *reinterpret_cast<float *>(tables + 32) = cmax / (float)(frag::kCbHalf - 1);
+}
+
 int kblk_for(int fmt) {
     return (fmt == FNN_FMT_I8 || fmt == FNN_FMT_F8) ? 64 : 128;
 }
@@ -525,6 +543,10 @@ int ensure_frag(fnn_cuda_ctx *ctx, fnn_cuda_qweight *w) {
     const size_t KB = div_ceil(w->K, (size_t)kblk_for(w->fmt));
     const size_t ntiles = div_ceil(w->N, 16);
     const size_t units = ntiles * KB * 64;
+    if (w->fmt == FNN_FMT_I4CB) {   // before `frag`, whose presence says that all of them are there
+        if (!w->frag_bs) FNN_CUDA_CHECK(cudaMalloc((void **)&w->frag_bs, units * sizeof(float)), FNN_ERR_MEMORY);
+        if (!w->cb_tables) FNN_CUDA_CHECK(cudaMalloc((void **)&w->cb_tables, 3 * sizeof(uint4)), FNN_ERR_MEMORY);
+    }
     FNN_CUDA_CHECK(cudaMalloc((void **)&w->frag, units * sizeof(uint4)), FNN_ERR_MEMORY);
     w->frag_bytes = units * sizeof(uint4);
     int blocks = (int)std::min<size_t>(div_ceil(units, 256), (size_t)ctx->sm_count * 16);
@@ -536,7 +558,9 @@ int ensure_frag(fnn_cuda_ctx *ctx, fnn_cuda_qweight *w) {
     FNN_CUDA_CHECK(cudaGetLastError(), FNN_ERR_DISPATCH);
     ctx->launches++;
     if (w->fmt == FNN_FMT_I4CB) {
-        FNN_CUDA_CHECK(cudaMalloc((void **)&w->frag_bs, units * sizeof(float)), FNN_ERR_MEMORY);
+        cb_tables_kernel<<<1, 32, 0, ctx->stream>>>(w->codebook, reinterpret_cast<uint8_t *>(w->cb_tables));
+        FNN_CUDA_CHECK(cudaGetLastError(), FNN_ERR_DISPATCH);
+        ctx->launches++;
         to_frag_scales_kernel<<<blocks, 256, 0, ctx->stream>>>(w->scales, w->blocks_per_row, w->N, KB,
                                                              ntiles, w->frag_bs);
         FNN_CUDA_CHECK(cudaGetLastError(), FNN_ERR_DISPATCH);

@@ -27,6 +27,7 @@ namespace {
 using frag::cp_async_commit;
 using frag::cp_async_wait;
 using frag::group_barrier;
+using frag::kCbHalf;
 
 constexpr int kW8 = frag::kWarpsPerGroup;   // warps per group
 constexpr int kU8 = frag::kChunkBlocks;     // k-blocks per ring chunk
@@ -104,7 +105,6 @@ __device__ __forceinline__ void decode_cb(const CbTables &t, uint32_t w, CbOpera
     o.lo_b[0] = prmt(t.lo[2], t.lo[3], f);
     o.lo_b[1] = prmt(t.lo[2], t.lo[3], f16);
 }
-constexpr int kCbHalf = 8192;   // centroid c is carried as v = round(c / cmax * 8191) + 8192
 
 // Staged byte position of activation k inside its row: where its group of eight goes, plus its place
 // inside the group.  I4 reorders inside the group (0,2,4,6,1,3,5,7: even codes of a word, then odd);
@@ -131,7 +131,7 @@ __device__ __forceinline__ int act_pos8(int k) {
 struct P8 {
     const uint4 *frag;
     const float *frag_bs;   // I4CB: block scales in fragment order
-    const float *codebook;  // I4CB: 16 centroids
+    const uint4 *cb_tables; // I4CB: the centroids as fixed point (cb_tables_kernel)
     const float *scales;
     const float *zeros;
     const float *act;
@@ -153,8 +153,13 @@ struct P8 {
 // keeps the shortest prologue.  CG 8-column groups hold the (term, batch row) columns: up to 4 * CG rows.
 // PLANES: the rows arrive rewritten (p.planes); its own instantiation, since the branch and the longer code cost the
 // smallest calls 2 %.
-template <int FMT, int CG, int kG8, bool MULTI, bool PLANES>
-__global__ void __launch_bounds__(kG8 * kW8 * 32, (kG8 == 1 && CG == 1 && !MULTI && !T8<FMT>::codebook) ? 3 : 1)
+// HELD: groups of eight activations a thread keeps of a single row between the scan and the rewrite, so that the row is read
+// once (0: never).  A row that is scanned and then read again behind two more block barriers costs 0.8 us (I8 K=11008 N=4096
+// 11.5 -> 10.7 us) to 2 us (I4 K=8192 N=2048 7.8 -> 5.6, one warp of byte stores per plane before).  As few groups as cover
+// the row: the prologue is straight-line code that every block runs once, and the instructions of groups
+// that are not there cost time too (I8 K=1024 N=2048 2.70 with 2, 3.46 with 8).
+template <int FMT, int CG, int kG8, bool MULTI, bool PLANES, int BPS, int HELD>
+__global__ void __launch_bounds__(kG8 * kW8 * 32, BPS)
 qmm_mma8_kernel(P8 p) {
     using TT = T8<FMT>;
     constexpr int KBLK = TT::KBLK, MMAS = TT::MMAS;
@@ -194,25 +199,7 @@ qmm_mma8_kernel(P8 p) {
     unsigned char *my_ring = s_ring + (size_t)warp * kS8 * UNITS * 512 + lane * 16;
     float *my_ring_bs = s_ring_bs + (size_t)warp * kS8 * UNITS * 32;
 
-    // I4CB: the centroids as 14-bit fixed point (every thread builds its own copy of the two tables)
     CbTables cbt{};
-    float cb_unit = 0.0f;   // value of one fixed-point step
-    if (CB) {
-        float cv[16], cmax = 0.0f;
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
-            cv[j] = __ldg(p.codebook + j);
-            cmax = fmaxf(cmax, fabsf(cv[j]));
-        }
-        const float to_fix = cmax > 0.0f ? (float)(kCbHalf - 1) / cmax : 0.0f;
-        cb_unit = cmax / (float)(kCbHalf - 1);
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
-            const int v = __float2int_rn(cv[j] * to_fix) + kCbHalf;   // 1 .. 16383
-            cbt.hi[j >> 2] |= (uint32_t)(v >> 7) << ((j & 3) * 8);
-            cbt.lo[j >> 2] |= (uint32_t)(v & 127) << ((j & 3) * 8);
-        }
-    }
 
     for (int i = gtid; i < tiles_here * 16; i += kW8 * 32) {
         const int n = (gg + (i >> 4) * GG) * 16 + (i & 15);
@@ -241,10 +228,8 @@ qmm_mma8_kernel(P8 p) {
 
     const bool vec_ok = (p.K % 4 == 0) && ((reinterpret_cast<uintptr_t>(p.act) & 15u) == 0);
     const int Kpad = p.KB * KBLK;
-    // groups of eight activations a thread keeps (single row, K <= 4096 per group of warps in the
-    // block); three-group blocks have no registers to spare for it
-    constexpr bool kCanHold = !MULTI && kG8 <= 2;
-    constexpr int kHeld = 2;
+    constexpr int kHeld = HELD;
+    constexpr bool kCanHold = kHeld > 0;
     float hv[kCanHold ? kHeld : 1][8];
     bool held = false;
     for (int k0 = 0; k0 < Kpad; k0 += p.Kc) {
@@ -283,6 +268,11 @@ qmm_mma8_kernel(P8 p) {
         for (int i = 0; i < kS8 - 1; ++i) issue_next();
 
         if (k0 == 0) {   // under the first weight loads: the per-row scan of the activations
+            if (CB) {
+                const uint4 hi = __ldg(p.cb_tables), lo = __ldg(p.cb_tables + 1);
+                cbt.hi[0] = hi.x; cbt.hi[1] = hi.y; cbt.hi[2] = hi.z; cbt.hi[3] = hi.w;
+                cbt.lo[0] = lo.x; cbt.lo[1] = lo.y; cbt.lo[2] = lo.z; cbt.lo[3] = lo.w;
+            }
             if (CB && kCanHold)   // columns of a single row that hold nothing (its own two are written as it is staged)
                 for (int i = tid; i < kc_len / 32 * 8 * CG; i += NT)
                     if ((i & (8 * CG - 1)) >= 2) s_boff[i] = 0;
@@ -297,7 +287,7 @@ qmm_mma8_kernel(P8 p) {
                     s_dq[tid] = __ldcg(p.dq + tid);
                     s_rs[tid] = __ldcg(p.rowsum + tid);
                 }
-            } else if (kCanHold && vec_ok && p.K % 8 == 0 && p.K <= NT * 8 * kHeld && kc_len >= Kpad) {
+            } else if (kCanHold && p.K <= NT * 8 * kHeld && kc_len >= Kpad) {
                 // A single batch row that is staged in one pass: every thread keeps its groups of eight
                 // consecutive activations in registers between the scan and the rewrite, so the row is
                 // read once.
@@ -306,19 +296,24 @@ qmm_mma8_kernel(P8 p) {
 #pragma unroll
                 for (int j = 0; j < kHeld; ++j) {
                     const int g8 = tid + j * NT;
-                    float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
-                    if (g8 * 8 < p.K) {
-                        a = ld_after_wait(reinterpret_cast<const float4 *>(p.act) + 2 * g8);
-                        b = ld_after_wait(reinterpret_cast<const float4 *>(p.act) + 2 * g8 + 1);
+                    if (vec_ok) {
+                        float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
+                        if (g8 * 8 < p.K) a = ld_after_wait(reinterpret_cast<const float4 *>(p.act) + 2 * g8);
+                        if (g8 * 8 + 4 < p.K) b = ld_after_wait(reinterpret_cast<const float4 *>(p.act) + 2 * g8 + 1);
+                        hv[j][0] = a.x; hv[j][1] = a.y; hv[j][2] = a.z; hv[j][3] = a.w;
+                        hv[j][4] = b.x; hv[j][5] = b.y; hv[j][6] = b.z; hv[j][7] = b.w;
+                    } else {
+#pragma unroll
+                        for (int q = 0; q < 8; ++q) hv[j][q] = g8 * 8 + q < p.K ? ld_after_wait(p.act + g8 * 8 + q) : 0.0f;
                     }
-                    hv[j][0] = a.x; hv[j][1] = a.y; hv[j][2] = a.z; hv[j][3] = a.w;
-                    hv[j][4] = b.x; hv[j][5] = b.y; hv[j][6] = b.z; hv[j][7] = b.w;
+                }
+#pragma unroll
+                for (int j = 0; j < kHeld; ++j)
 #pragma unroll
                     for (int q = 0; q < 8; ++q) {
                         mx = fmaxf(mx, fabsf(hv[j][q]));
                         sum += hv[j][q];
                     }
-                }
 #pragma unroll
                 for (int o = 16; o > 0; o >>= 1) {
                     mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, o));
@@ -328,22 +323,10 @@ qmm_mma8_kernel(P8 p) {
                     s_part[warp * 2] = mx;
                     s_part[warp * 2 + 1] = sum;
                 }
-                __syncthreads();
-                if (tid == 0) {   // fixed order: the sums do not depend on scheduling
-                    float bm = 0.0f, bs = 0.0f;
-#pragma unroll
-                    for (int w = 0; w < NW; ++w) {
-                        bm = fmaxf(bm, s_part[w * 2]);
-                        bs += s_part[w * 2 + 1];
-                    }
-                    s_mx[0] = bm;
-                    s_rs[0] = bs;
-                }
-                __syncthreads();
             } else {
                 frag::scan_rows<NT, MULTI ? 4 : 1>(p.act, p.M, p.K, vec_ok, s_part, s_mx, s_rs);
             }
-            if (!PLANES && tid < p.M) {
+            if (!PLANES && !(kCanHold && held) && tid < p.M) {
                 const float bm = s_mx[tid];
                 s_dq[tid] = (bm > 0.0f && isfinite(bm)) ? bm / 16256.0f : 1.0f;
             }   // (published by the barrier below)
@@ -407,7 +390,21 @@ qmm_mma8_kernel(P8 p) {
                 }
             }
         } else if (kCanHold && held) {
-            const float inv = 1.0f / s_dq[0];
+            // every thread folds the warps' partials itself, in the same fixed order: one barrier and a broadcast
+            // less than handing the result round
+            float bm = 0.0f, bs = 0.0f;
+#pragma unroll
+            for (int w = 0; w < NW; ++w) {
+                const float2 part = *reinterpret_cast<const float2 *>(s_part + w * 2);
+                bm = fmaxf(bm, part.x);
+                bs += part.y;
+            }
+            const float dq0 = (bm > 0.0f && isfinite(bm)) ? bm / 16256.0f : 1.0f;
+            if (tid == 0) {   // (published by the barrier below, for the epilogue)
+                s_dq[0] = dq0;
+                s_rs[0] = bs;
+            }
+            const float inv = 1.0f / dq0;
 #pragma unroll
             for (int j = 0; j < kHeld; ++j) {
                 const int g8 = tid + j * NT;
@@ -643,7 +640,7 @@ qmm_mma8_kernel(P8 p) {
         const float *meta = my_meta + (tl * 16 + r16) * 3;
         float v;
         if (CB) {   // no per-row scale or zero point: the block scales are inside acc
-            const float dot = acc * s_dq[m] * cb_unit;
+            const float dot = acc * s_dq[m] * __ldg(reinterpret_cast<const float *>(p.cb_tables + 2));
             v = apply_act(p.bias ? __fadd_rn(dot, meta[2]) : dot, p.epilogue);
         } else {
             v = finish_output(acc * s_dq[m], meta[0], meta[1], has_zero ? s_rs[m] : 0.0f, p.bias != nullptr,
@@ -658,14 +655,14 @@ qmm_mma8_kernel(P8 p) {
     if (p.gather_on) gather_finish(p.g, step, p.M, p.N);
 }
 
-template <int FMT, int CG, int kG8, bool MULTI>
-int launch8(fnn_cuda_ctx *ctx, const QmmArgs &a, int blocks_per_sm = 1) {
+template <int FMT, int CG, int kG8, bool MULTI, int BPS = 1, int HELD = 0>
+int launch8(fnn_cuda_ctx *ctx, const QmmArgs &a) {
     using TT = T8<FMT>;
     const fnn_cuda_qweight *w = a.w;
     P8 p{};
     p.frag = w->frag;
     p.frag_bs = w->frag_bs;
-    p.codebook = w->codebook;
+    p.cb_tables = w->cb_tables;
     p.scales = w->scales;
     p.zeros = w->zeros;
     p.act = a.a;
@@ -712,15 +709,16 @@ int launch8(fnn_cuda_ctx *ctx, const QmmArgs &a, int blocks_per_sm = 1) {
             return ((((size_t)cols * (kc + TT::PAD)) + 15) & ~(size_t)15) +
                    (TT::codebook ? (size_t)(kc / 32) * 8 * CG * 4 : 0);
         },
-        &sz, blocks_per_sm);
-    if (!fits && blocks_per_sm > 1) return launch8<FMT, CG, kG8, MULTI>(ctx, a, 1);
+        &sz, BPS);
+    if constexpr (BPS > 1)
+        if (!fits) return launch8<FMT, CG, kG8, MULTI, 1, HELD>(ctx, a);
     FNN_REQUIRE(fits, FNN_ERR_UNSUPPORTED,
                 "qmatmul: shared memory budget exceeded for M=%d on the 8-bit fragment kernel", p.M);
     p.tiles_per_group = sz.tiles_per_group;
     p.Kc = sz.Kc;
-    auto kern = qmm_mma8_kernel<FMT, CG, kG8, MULTI, false>;
+    auto kern = qmm_mma8_kernel<FMT, CG, kG8, MULTI, false, BPS, HELD>;
     if constexpr (MULTI && !TT::codebook)
-        if (p.planes) kern = qmm_mma8_kernel<FMT, CG, kG8, MULTI, true>;
+        if (p.planes) kern = qmm_mma8_kernel<FMT, CG, kG8, MULTI, true, BPS, HELD>;
     FNN_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sz.smem),
                    FNN_ERR_DISPATCH);
     FNN_CUDA_CHECK(launch_pdl(kern, sz.grid, kG8 * kW8 * 32, sz.smem, ctx, p), FNN_ERR_DISPATCH);
@@ -730,31 +728,42 @@ int launch8(fnn_cuda_ctx *ctx, const QmmArgs &a, int blocks_per_sm = 1) {
     return FNN_OK;
 }
 
-// Groups per block: three while that still gives (nearly) every SM a block; layers with fewer row
-// tiles run two or one group per block so that the tiles spread over more SMs.  Two and four column
-// groups (5..8 and 9..16 batch rows) keep more accumulators per thread and run at most two groups.
+// A single batch row: groups per block and blocks per SM (the registers of a thread are bounded for that many).  The SMs are
+// shared with the blocks of the next kernel on the stream, which prefetch their weights as soon as one fits, so smaller
+// blocks win where there are enough of them; every block stages the row, so a long one wants few of them; and up to one
+// tile per SM two blocks on an SM would leave another idle.  us, one group x 1 / x 2 / x 3 blocks per SM, two
+// groups x 1 (three groups x 1 are never the fastest):
+//   up to a tile per SM        I8 K=8192 N=2048 6.18 / 6.72 / 8.35 / 6.57;  FP4 K=8192 N=2048 5.64 / 7.05 / 8.45 / 6.79;
+//                              codebook K=8192 N=2048 7.47 / 11.2 / - / 10.4
+//   K up to 4096               I4 K=4096 N=4096 - / 4.61 / 5.13 / 4.98;  FP4 K=4096 N=11008 - / 7.80 / 9.84 / 8.41;
+//                              I8 K=2048 N=8192 - / 5.05 / 5.65 / 5.70;  codebook K=2048 N=8192 7.77 / 6.60 / - / 7.56
+//   and I8 of four tiles a SM  K=4096 N=11008 11.1 / 10.0 / 9.84 / 9.88, N=14336 13.4 / 11.9 / 11.6 / 12.3
+//   longer                     I8 K=11008 N=4096 - / 11.1 / 15.8 / 10.7, K=8192 N=28672 - / 37.7 / 41.1 / 37.5; I4 K=14336 N=4096
+//                              - / 9.20 / 16.0 / 8.62; codebook, whose tables cost a second group its registers,
+//                              K=11008 N=4096 15.2 / 17.4 / - / 15.8
+template <int FMT>
+int launch8_single(fnn_cuda_ctx *ctx, const QmmArgs &a, int ntiles) {
+    const int units = (int)div_ceil(a.w->K, 8);
+    if (ntiles > ctx->sm_count) {
+        if constexpr (FMT == FNN_FMT_I8)
+            if (units <= 512 && ntiles >= 4 * ctx->sm_count) return launch8<FMT, 1, 1, false, 3, 2>(ctx, a);
+        if (units <= 512) return launch8<FMT, 1, 1, false, 2, 2>(ctx, a);
+        if constexpr (!T8<FMT>::codebook)
+            return units <= 1024 ? launch8<FMT, 1, 2, false, 1, 2>(ctx, a) : launch8<FMT, 1, 2, false, 1, 4>(ctx, a);
+    }
+    return units <= 512    ? launch8<FMT, 1, 1, false, 1, 2>(ctx, a)
+           : units <= 1024 ? launch8<FMT, 1, 1, false, 1, 4>(ctx, a)
+                           : launch8<FMT, 1, 1, false, 1, 8>(ctx, a);
+}
+
+// Several batch rows: two groups per block while that still gives (nearly) every SM a block, else one, so that the tiles
+// spread over more SMs.  (us with three / two groups: I8 M=4 K=4096 N=11008 12.5 / 12.0, K=2048 N=8192 8.05 / 7.17.)
 template <int FMT, int CG>
 int launch8_cg(fnn_cuda_ctx *ctx, const QmmArgs &a) {
-    const int ntiles = (int)div_ceil(a.w->N, 16), want = ctx->sm_count * 4 / 5;
-    if (CG == 1) {
-        const bool multi = a.M > 1;
-        // (the codebook format keeps its two lookup tables in registers: two groups at most)
-        if constexpr (!T8<FMT>::codebook) {
-            // A single batch row on a layer with one to three tiles per group runs as three independent
-            // one-group blocks per SM instead of one three-group block: blocks of the next kernel on the
-            // stream then take the place of single finished blocks and prefetch their weights under
-            // this kernel's tail (config 2: 9.8 -> 9.0 us per step).  Smaller layers lose more to the
-            // smaller blocks' repeated prologue than they gain, larger ones have no tail to speak of.
-            if (!multi && ntiles >= 3 * ctx->sm_count && ntiles < 9 * ctx->sm_count)
-                return launch8<FMT, 1, 1, false>(ctx, a, 3);
-            if ((ntiles + 2) / 3 >= want)
-                return multi ? launch8<FMT, 1, 3, true>(ctx, a) : launch8<FMT, 1, 3, false>(ctx, a);
-        }
-        if ((ntiles + 1) / 2 >= want)
-            return multi ? launch8<FMT, 1, 2, true>(ctx, a) : launch8<FMT, 1, 2, false>(ctx, a);
-        return multi ? launch8<FMT, 1, 1, true>(ctx, a) : launch8<FMT, 1, 1, false>(ctx, a);
-    }
-    if ((ntiles + 1) / 2 >= want) return launch8<FMT, CG, 2, true>(ctx, a);
+    const int ntiles = (int)div_ceil(a.w->N, 16);
+    if constexpr (CG == 1)
+        if (a.M == 1) return launch8_single<FMT>(ctx, a, ntiles);
+    if ((ntiles + 1) / 2 >= ctx->sm_count * 4 / 5) return launch8<FMT, CG, 2, true>(ctx, a);
     return launch8<FMT, CG, 1, true>(ctx, a);
 }
 

@@ -12,8 +12,10 @@ namespace fnn {
 void free_qweight_aux(fnn_cuda_qweight *w) {
     if (w->frag) cudaFree(w->frag);
     if (w->frag_bs) cudaFree(w->frag_bs);
+    if (w->cb_tables) cudaFree(w->cb_tables);
     w->frag = nullptr;
     w->frag_bs = nullptr;
+    w->cb_tables = nullptr;
 }
 
 // The weights whose rows are the arena slot itself.  An entry lives as long as its weight object, whatever becomes of the

@@ -37,6 +37,25 @@ def test_fragment_kernel_rows(backend, fmt, kn):
         rig.close()
 
 
+# one row: lengths on both sides of what a thread keeps of it (4096, 8192 and 16384 elements), ragged ones among them, by up to
+# a tile of 16 channels per SM, more, and (I8) four: every launch shape of the 8-bit fragment kernel for a single row
+@pytest.mark.parametrize("fmt,k,n", [
+    (fmt, k, n) for fmt in (orc.FMT_I8, orc.FMT_I4, orc.FMT_F4, orc.FMT_I4CB)
+    for k, n in [(4096, 200), (4097, 200), (8199, 72), (8192, 2400), (4094, 2400), (10001, 2385), (16388, 40)]
+] + [(orc.FMT_I8, 520, 9488), (orc.FMT_I4, 520, 9488)])
+def test_single_row_launches(backend, fmt, k, n):
+    q = orc.quantize_kn(fmt, normal(850 + k, (k, n), 0.02))
+    bias = normal(851, (n,), 0.01)
+    rig = Rig(backend, q, 1)
+    try:
+        x = normal(852 + n, (1, k), 1.0)
+        got = rig.run(x, bias, L.EPI_NONE, L.PATH_MMA)
+        err = max_err_vs_rms(got, orc.qmatmul(q, x, bias, L.EPI_NONE))
+        assert err <= TOL_F32, (orc.FMT_NAMES[fmt], k, n, err)
+    finally:
+        rig.close()
+
+
 # both sides of the lines that automatic dispatch draws by format, rows, K and size of the weights
 @pytest.mark.parametrize("fmt,k,n,m,tc", [
     (orc.FMT_I8, 4096, 2304, 4, False), (orc.FMT_I8, 4096, 2304, 5, True), (orc.FMT_I8, 1024, 512, 8, False),
