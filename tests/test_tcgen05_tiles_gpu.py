@@ -62,6 +62,15 @@ def test_rewritten_rows_of_any_length(backend, fmt, k):
     check(backend, fmt, k, 40, [3, 9])
 
 
+# I4 rows of more than 4096 elements are shared by the blocks of a cluster up to a row per SM: both sides of that line, whole and
+# short last units, parts of unequal length
+@pytest.mark.parametrize("k", [4104, 8209])
+def test_rewritten_rows_by_cluster_or_by_block(backend, k):
+    import torch
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    check(backend, orc.FMT_I4, k, 40, [sms, sms + 1])
+
+
 def random_codes(fmt, k, n, seed):
     """A weight of random finite codes (no host quantization: these layers are large)."""
     rng = np.random.Generator(np.random.Philox(seed))
