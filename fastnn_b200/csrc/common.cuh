@@ -65,9 +65,10 @@ struct fnn_cuda_ctx {
     void *scratch = nullptr;
     size_t scratch_bytes = 0;
     std::vector<void *> retired_scratch;   // outgrown scratch buffers (captured graphs may still name them)
-    int *err_flag = nullptr;  // device flag written by bounded waits that gave up; err_flag[1]: CTA ticket of
-                              // the fused GEMM + all-gather
-    int *err_host = nullptr;  // pinned host copy of err_flag[0], refreshed by fnn_cuda_sync
+    // Device words: [0] flag of the bounded waits that gave up, [1] CTA ticket of the fused GEMM + all-gather,
+    // [2..3] device address of err_host (raise_error)
+    int *err_flag = nullptr;
+    int *err_host = nullptr;  // pinned host word that a kernel sets when it raises err_flag[0]
     bool overlap_launches = true;   // programmatic dependent launch (fnn_cuda_ctx_set_overlap)
 };
 
@@ -198,6 +199,17 @@ __device__ __forceinline__ float finish_output_fast(float dot, float scale, floa
     if (has_bias) x = __fadd_rn(x, bias);
     return apply_act_fast(x, epi);
 }
+
+// A bounded wait gave up: the code goes into the context's device flag, and a word of pinned host memory says that there is
+// one, so that fnn_cuda_sync has nothing to copy back (see there).
+#ifdef __CUDACC__
+__device__ __forceinline__ void raise_error(int *err_flag, int code) {
+    atomicOr(err_flag, code);
+    volatile int *host = *reinterpret_cast<int *volatile *>(err_flag + 2);
+    *host = 1;
+    __threadfence_system();
+}
+#endif
 
 // ---- programmatic dependent launch ------------------------------------------------------------
 // A kernel launched through launch_pdl may start while the kernel before it on the stream is still
@@ -341,7 +353,7 @@ __device__ __forceinline__ void gather_check_prev(const GatherArgs &g, const Gat
         if (!(first && (int)((unsigned)(w >> 32) - (c.step - 1u)) >= 0) &&
             !wait_word(c.prev_words + (size_t)r * kGatherRows * g.n_stride + (i - r * c.prev_per_rank),
                        c.step - 1u, w)) {
-            atomicOr(g.err_flag, 0x100);
+            raise_error(g.err_flag, 0x100);
             break;
         }
         first = false;

@@ -804,7 +804,7 @@ __global__ void gather_wait_kernel(const unsigned long long *words, const unsign
         const int r = i / per_rank;
         unsigned long long w;
         if (!wait_word(slot + (size_t)r * kGatherRows * n_stride + (i - r * per_rank), step, w)) {
-            atomicOr(err_flag, 0x100);
+            raise_error(err_flag, 0x100);
             return;
         }
         if (out) out[i] = __uint_as_float((unsigned)w);

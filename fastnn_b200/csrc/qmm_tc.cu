@@ -703,7 +703,7 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
                     break;
                 }
                 if (clock64() - t0 > kWaitCycles) {   // gives up without consuming
-                    atomicOr(p.err_flag, 0x400);
+                    raise_error(p.err_flag, 0x400);
                     break;
                 }
             }

@@ -75,7 +75,7 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, volati
         if (*abort_flag) return false;
         if (clock64() - t0 > kWaitCycles) {
             *abort_flag = 1;
-            atomicOr(err_flag, code);
+            raise_error(err_flag, code);
             return false;
         }
     }
