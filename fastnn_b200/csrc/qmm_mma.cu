@@ -157,15 +157,16 @@ struct MmaParams {
 };
 
 // Warp groups per block for a given number of 8-column groups (register budget).
-__host__ __device__ constexpr int groups_for(int cg) { return cg == 1 ? 3 : (cg <= 4 ? 2 : 1); }
+__host__ __device__ constexpr int groups_for(int cg) { return cg <= 4 ? 2 : 1; }   // (several column groups)
 
 // Stages of each lane's private cp.async ring (weights in flight = STAGES - 1 chunks per lane).
 __host__ __device__ constexpr int stages_for(int cg) { return cg == 4 ? 2 : 3; }
 
-// One block per SM.  Its G groups of 8 warps share the staged activations; each group streams
-// its own row tiles, splitting K across its warps.
-template <int FMT, int CG, int G>
-__global__ void __launch_bounds__(G * kW * 32, 1)
+// BPS blocks per SM.  The G groups of 8 warps of a block share the staged activations; each group streams
+// its own row tiles, splitting K across its warps.  HELD: groups of eight activations a thread keeps of a single batch
+// row between the scan and the rewrite, so that the row is read once (0: never).
+template <int FMT, int CG, int G, int BPS, int HELD>
+__global__ void __launch_bounds__(G * kW * 32, BPS)
 qmm_mma_kernel(MmaParams p) {
     using T = FragTraits<FMT>;
     constexpr int KBLK = T::KBLK, VEC = T::VEC;
@@ -235,6 +236,8 @@ qmm_mma_kernel(MmaParams p) {
     const bool vec_ok = (p.K % 4 == 0) && ((reinterpret_cast<uintptr_t>(p.act) & 15u) == 0);
 
     const int Kpad = p.KB * KBLK;
+    float hv[HELD > 0 ? HELD : 1][8];
+    bool held = false;
     for (int k0 = 0; k0 < Kpad; k0 += p.Kc) {
         const int kc_len = min(p.Kc, Kpad - k0);
         const int KBc = kc_len / KBLK;
@@ -277,8 +280,43 @@ qmm_mma_kernel(MmaParams p) {
             if (CG == 1 && p.gather_on) gc = gather_begin(p.g, blockIdx.x * NT + tid);
             // per-row maximum and sum; the row is staged as a * 2^e with the largest element in
             // [2^14, 2^15): exact, inside the fp16 range whatever the magnitude of the activations
-            frag::scan_rows<NT, 4>(p.act, p.M, p.K, vec_ok, s_part, s_mx, s_rs);
-            if (tid < p.M) {
+            if (HELD > 0 && p.K <= NT * 8 * HELD && kc_len >= Kpad) {
+                held = true;
+                float mx = 0.0f, sum = 0.0f;
+#pragma unroll
+                for (int j = 0; j < HELD; ++j) {
+                    const int g8 = tid + j * NT;
+                    if (vec_ok) {
+                        float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
+                        if (g8 * 8 < p.K) a = ld_after_wait(reinterpret_cast<const float4 *>(p.act) + 2 * g8);
+                        if (g8 * 8 + 4 < p.K) b = ld_after_wait(reinterpret_cast<const float4 *>(p.act) + 2 * g8 + 1);
+                        hv[j][0] = a.x; hv[j][1] = a.y; hv[j][2] = a.z; hv[j][3] = a.w;
+                        hv[j][4] = b.x; hv[j][5] = b.y; hv[j][6] = b.z; hv[j][7] = b.w;
+                    } else {
+#pragma unroll
+                        for (int q = 0; q < 8; ++q) hv[j][q] = g8 * 8 + q < p.K ? ld_after_wait(p.act + g8 * 8 + q) : 0.0f;
+                    }
+                }
+#pragma unroll
+                for (int j = 0; j < HELD; ++j)
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) {
+                        mx = fmaxf(mx, fabsf(hv[j][q]));
+                        sum += hv[j][q];
+                    }
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) {
+                    mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, o));
+                    sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
+                }
+                if (lane == 0) {
+                    s_part[warp * 2] = mx;
+                    s_part[warp * 2 + 1] = sum;
+                }
+            } else {
+                frag::scan_rows<NT, (HELD > 0 ? 1 : 4)>(p.act, p.M, p.K, vec_ok, s_part, s_mx, s_rs);
+            }
+            if (!held && tid < p.M) {
                 const float bm = s_mx[tid];
                 int ex = 15;
                 if (bm > 0.0f && isfinite(bm)) (void)frexpf(bm, &ex);   // bm = f * 2^ex, f in [0.5, 1)
@@ -292,7 +330,40 @@ qmm_mma_kernel(MmaParams p) {
         // Work item of a warp = 32 groups of eight consecutive k of one batch row: two 16-byte loads
         // per lane, one 16-byte store per plane (an 8-group is contiguous in the staged order of every
         // format).  Two items are in flight per warp.
-        if (vec_ok) {
+        if (HELD > 0 && held) {
+            // every thread folds the warps' partials itself, in the same fixed order
+            float bm = 0.0f, bs = 0.0f;
+#pragma unroll
+            for (int w = 0; w < NW; ++w) {
+                bm = fmaxf(bm, s_part[w * 2]);
+                bs += s_part[w * 2 + 1];
+            }
+            int ex = 15;
+            if (bm > 0.0f && isfinite(bm)) (void)frexpf(bm, &ex);
+            const int e = max(-120, min(120, 15 - ex));
+            const float up = ldexpf(1.0f, e);
+            if (tid == 0) {   // (published by the barrier below, for the epilogue)
+                s_dq[0] = ldexpf(1.0f, -e);
+                s_rs[0] = bs;
+            }
+#pragma unroll
+            for (int j = 0; j < HELD; ++j) {
+                const int g8 = tid + j * NT;
+                if (g8 * 8 >= kc_len) continue;   // (beyond K the held values are zero: the padding of the last block)
+                __align__(16) __half hi[8];
+                __align__(16) __half lo[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const float a = hv[j][i] * up;
+                    const int pos = FragTraits<FMT>::four_bit ? pos8<FMT>(i) : i;
+                    hi[pos] = __float2half_rn(a);
+                    lo[pos] = __float2half_rn(a - __half2float(hi[pos]));
+                }
+                const int base = act_pos<FMT>(g8 * 8) * 2;
+                *reinterpret_cast<uint4 *>(s_act + base) = *reinterpret_cast<const uint4 *>(hi);
+                *reinterpret_cast<uint4 *>(s_act + (size_t)RS + base) = *reinterpret_cast<const uint4 *>(lo);
+            }
+        } else if (vec_ok) {
             const int chunks = kc_len / 8, cg32 = (chunks + 31) / 32, witems = p.M * cg32;
             for (int w0 = warp; w0 < witems; w0 += 2 * NW) {
                 float4 v[2][2];
@@ -569,7 +640,7 @@ int ensure_frag(fnn_cuda_ctx *ctx, fnn_cuda_qweight *w) {
     return FNN_OK;
 }
 
-template <int FMT, int CG, int G>
+template <int FMT, int CG, int G, int BPS = 1, int HELD = 0>
 int launch_mma_g(fnn_cuda_ctx *ctx, const QmmArgs &a, const float *act, float *out, int M, int split) {
     using T = FragTraits<FMT>;
     const fnn_cuda_qweight *w = a.w;
@@ -599,14 +670,16 @@ int launch_mma_g(fnn_cuda_ctx *ctx, const QmmArgs &a, const float *act, float *o
     frag::FragSizing sz;
     const bool fits = frag::size_frag_launch(
         ctx->sm_count, p.ntiles, G, p.KB * T::KBLK, T::KBLK, fixed, per_tile,
-        [&](int kc) { return (size_t)act_rows * (2 * kc + T::PAD_BYTES); }, &sz);
+        [&](int kc) { return (size_t)act_rows * (2 * kc + T::PAD_BYTES); }, &sz, BPS);
+    if constexpr (BPS > 1)
+        if (!fits) return launch_mma_g<FMT, CG, G, 1, HELD>(ctx, a, act, out, M, split);
     FNN_REQUIRE(fits, FNN_ERR_UNSUPPORTED,
                 "qmatmul: shared memory budget exceeded for M=%d on the skinny tensor-core path", M);
     p.tiles_per_group = sz.tiles_per_group;
     p.Kc = sz.Kc;
     const size_t smem = sz.smem;
     const int grid = sz.grid;
-    auto kern = qmm_mma_kernel<FMT, CG, G>;
+    auto kern = qmm_mma_kernel<FMT, CG, G, BPS, HELD>;
     FNN_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
                    FNN_ERR_DISPATCH);
     FNN_CUDA_CHECK(launch_pdl(kern, grid, G * kW * 32, smem, ctx, p), FNN_ERR_DISPATCH);
@@ -614,19 +687,42 @@ int launch_mma_g(fnn_cuda_ctx *ctx, const QmmArgs &a, const float *act, float *o
     return FNN_OK;
 }
 
-// Groups per block: the most the register and shared-memory budget allows (groups_for) while that
-// still gives (nearly) every SM a block; for the single-column-group kernels, layers with fewer row
-// tiles run fewer groups per block so that the tiles spread over more SMs.
+// A single batch row of FP8: groups per block and blocks per SM, by the same considerations as on the 8-bit kernel (launch8_single
+// there).  us, three groups x 1 that scanned and re-read the row / one group x 1 / x 2 / two groups x 1:
+//   up to a tile per SM             K=8192 N=2048 9.77 / 6.19 / 7.57 / 7.41
+//   K up to 4096, or eight tiles    K=4096 N=4096 6.94 / 6.03 / 5.54 / 6.18, N=28672 22.6 / 23.9 / 20.9 / 21.4;
+//   per SM                          K=8192 N=28672 40.4 / 42.9 / 37.7 / 38.3
+//   longer                          K=8192 N=8192 16.1 / 15.8 / 14.3 / 13.9, K=11008 N=4096 12.6 / 12.3 / 11.9 / 10.8
+template <int FMT>
+int launch_mma_single(fnn_cuda_ctx *ctx, const QmmArgs &a, const float *act, float *out) {
+    const int ntiles = (int)div_ceil(a.w->N, 16), units = (int)div_ceil(a.w->K, 8);
+    if (ntiles > ctx->sm_count) {
+        if (units <= 512) return launch_mma_g<FMT, 1, 1, 2, 2>(ctx, a, act, out, 1, 1);
+        if (units <= 1024)
+            return ntiles >= 8 * ctx->sm_count ? launch_mma_g<FMT, 1, 1, 2, 4>(ctx, a, act, out, 1, 1)
+                                               : launch_mma_g<FMT, 1, 2, 1, 2>(ctx, a, act, out, 1, 1);
+        return launch_mma_g<FMT, 1, 2, 1, 4>(ctx, a, act, out, 1, 1);
+    }
+    return units <= 512    ? launch_mma_g<FMT, 1, 1, 1, 2>(ctx, a, act, out, 1, 1)
+           : units <= 1024 ? launch_mma_g<FMT, 1, 1, 1, 4>(ctx, a, act, out, 1, 1)
+                           : launch_mma_g<FMT, 1, 1, 1, 8>(ctx, a, act, out, 1, 1);
+}
+
+// Groups per block.  Single-column-group kernels: three where every SM has many tiles, two while that still gives (nearly) every
+// SM a block, else one, so that the tiles spread over more SMs (us with three / two groups: FP8 M=4 K=8192 N=28672
+// 46.2 / 46.8, K=4096 N=11008 15.2 / 12.7, M=3 K=2048 N=8192 8.3 / 7.4).  More columns: what the registers allow.
 template <int FMT, int CG>
 int launch_mma(fnn_cuda_ctx *ctx, const QmmArgs &a, const float *act, float *out, int M, int split) {
-    constexpr int GMAX = groups_for(CG);
-    if (CG == 1) {
-        const int ntiles = (int)div_ceil(a.w->N, 16), want = ctx->sm_count * 4 / 5;
-        if (GMAX >= 3 && (ntiles + 2) / 3 >= want) return launch_mma_g<FMT, CG, GMAX>(ctx, a, act, out, M, split);
-        if ((ntiles + 1) / 2 >= want) return launch_mma_g<FMT, CG, (GMAX < 2 ? GMAX : 2)>(ctx, a, act, out, M, split);
+    if constexpr (CG == 1) {
+        const int ntiles = (int)div_ceil(a.w->N, 16);
+        if constexpr (FMT == FNN_FMT_F8)   // (the other formats' few rows are on the 8-bit kernel)
+            if (M == 1) return launch_mma_single<FMT>(ctx, a, act, out);
+        if (ntiles >= 8 * ctx->sm_count) return launch_mma_g<FMT, CG, 3>(ctx, a, act, out, M, split);
+        if ((ntiles + 1) / 2 >= ctx->sm_count * 4 / 5) return launch_mma_g<FMT, CG, 2>(ctx, a, act, out, M, split);
         return launch_mma_g<FMT, CG, 1>(ctx, a, act, out, M, split);
+    } else {
+        return launch_mma_g<FMT, CG, groups_for(CG)>(ctx, a, act, out, M, split);
     }
-    return launch_mma_g<FMT, CG, GMAX>(ctx, a, act, out, M, split);
 }
 
 template <int FMT>

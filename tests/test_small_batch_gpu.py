@@ -38,9 +38,9 @@ def test_fragment_kernel_rows(backend, fmt, kn):
 
 
 # one row: lengths on both sides of what a thread keeps of it (4096, 8192 and 16384 elements), ragged ones among them, by up to
-# a tile of 16 channels per SM, more, and (I8) four: every launch shape of the 8-bit fragment kernel for a single row
+# a tile of 16 channels per SM, more, and (I8) four: the launch shapes of the fragment kernels for a single row
 @pytest.mark.parametrize("fmt,k,n", [
-    (fmt, k, n) for fmt in (orc.FMT_I8, orc.FMT_I4, orc.FMT_F4, orc.FMT_I4CB)
+    (fmt, k, n) for fmt in (orc.FMT_I8, orc.FMT_I4, orc.FMT_F4, orc.FMT_I4CB, orc.FMT_F8)
     for k, n in [(4096, 200), (4097, 200), (8199, 72), (8192, 2400), (4094, 2400), (10001, 2385), (16388, 40)]
 ] + [(orc.FMT_I8, 520, 9488), (orc.FMT_I4, 520, 9488)])
 def test_single_row_launches(backend, fmt, k, n):
