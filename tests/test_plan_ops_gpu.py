@@ -7,7 +7,7 @@ import pytest
 
 import oracle as orc
 import fastnn_b200 as fnn
-from fastnn_b200 import GraphBuilder, TensorType
+from fastnn_b200 import GraphBuilder, TensorType, _lib as L
 from fastnn_b200.backend import _check
 from helpers import max_err_vs_rms, normal
 
@@ -156,3 +156,29 @@ def test_residual_block_through_the_graph_builder(backend):
     ln = orc.layer_norm(x, g, beta, 1e-5, o)
     want = orc.qmatmul(orc.quantize_kn(orc.FMT_I8, wu), ln, None, orc.EPI_GELU)
     assert max_err_vs_rms(got, want) <= 2e-3
+
+
+# every instantiation of the vector kernel; the last one to three elements of a length that is no multiple of four
+@pytest.mark.parametrize("op", [b | (a << 8) for b in (L.EW_ADD, L.EW_MUL, L.EW_SUB)
+                                for a in (L.EPI_NONE, L.EPI_RELU, L.EPI_GELU, L.EPI_SILU)] +
+                         [L.EW_RELU, L.EW_GELU, L.EW_SILU])
+def test_elementwise_lengths(backend, op):
+    """The first n results of a longer call, and nothing behind them; sums and products to the bit."""
+    x, y = normal(70, (4104,), 1.0), normal(71, (4104,), 1.0)
+    arena = backend.allocate_arena(3 * 4104 * 4)
+
+    def run(n):
+        backend.write_arena(arena, 0, np.concatenate([x, y, np.full(4104, 7, np.float32)]).tobytes())
+        assert backend.lib.fnn_cuda_elementwise(backend.ctx, op, arena.handle, 0, n, 4 * 4104, n, 8 * 4104, n) == 0
+        return np.frombuffer(backend.read_arena(arena, 8 * 4104, 4 * 4104), np.float32)
+
+    try:
+        whole = run(4104)
+        exact = {L.EW_ADD: x + y, L.EW_MUL: x * y, L.EW_SUB: x - y, L.EW_RELU: np.maximum(x, 0)}
+        if op in exact:
+            assert (whole == exact[op]).all()
+        for n in (1, 2, 3, 5, 1023, 4098, 4099, 4101):
+            got = run(n)
+            assert (got[:n] == whole[:n]).all() and (got[n:] == 7).all(), n
+    finally:
+        arena.close()
