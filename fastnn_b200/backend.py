@@ -263,8 +263,40 @@ class CudaBackend:
         if arena.latched_error is not None:
             err, arena.latched_error = arena.latched_error, None
             raise err
-        for instr in plan.instructions:
+        todo = iter(plan.instructions)
+        instr = next(todo, None)
+        while instr is not None:
+            following = next(todo, None)
+            if (isinstance(instr, CallKernel) and instr.kernel_name in _QMATMUL_KERNELS
+                    and isinstance(following, CallKernel) and following.kernel_name == "add_f32"):
+                residual = self._residual_of(instr, following, shape_env)
+                if residual is not None:
+                    self._dispatch_qmatmul(instr, arena, shape_env, residual, following.output_slice)
+                    instr = next(todo, None)
+                    continue
             self._dispatch_one(instr, arena, shape_env)
+            instr = following
+
+    @staticmethod
+    def _residual_of(matmul: CallKernel, add: CallKernel, env: ShapeEnv) -> Optional[BufferSlice]:
+        """The other operand of an addition to the whole result of the MatMul before it, or None if it is anything
+        else (a broadcast, another slice, a symbolic size that differs): the two then run as they stand."""
+        if len(add.input_slices) != 2 or len(matmul.input_slices) < 2:
+            return None
+        m, _, n = resolve_params(matmul.params, matmul.param_dims, env, 3)
+        size = 4 * m * n
+        out_size = add.output_slice.size // 4 * 4
+        if add.param_dims:
+            out_size = 4
+            for d in add.param_dims:
+                out_size *= env.resolve(d)
+        x, y = add.input_slices
+        if y.offset == matmul.output_slice.offset:
+            x, y = y, x
+        if (x.offset != matmul.output_slice.offset or out_size != size
+                or min(x.size, y.size, add.output_slice.size) < size):
+            return None
+        return y
 
     def dispatch_profile(self, plan: ExecutablePlan, arena: CudaBuffer,
                          shape_env: ShapeEnv) -> List[ProfileEntry]:
@@ -425,7 +457,9 @@ class CudaBackend:
         # no CPU fallback: anything else is not this backend's job
         raise BackendError("UnsupportedOp", f"kernel '{name}' is not implemented by the CUDA backend")
 
-    def _dispatch_qmatmul(self, instr: CallKernel, arena: CudaBuffer, env: ShapeEnv) -> None:
+    def _dispatch_qmatmul(self, instr: CallKernel, arena: CudaBuffer, env: ShapeEnv,
+                          residual: Optional[BufferSlice] = None, total: Optional[BufferSlice] = None) -> None:
+        """With ``residual`` and ``total``: the addition that follows as well, in the same launch."""
         name = instr.kernel_name
         if len(instr.input_slices) < 2:
             raise BackendError("Dispatch", f"{name}: expected activation and weight slices")
@@ -450,6 +484,11 @@ class CudaBackend:
             arena.qweights[key] = qw
         epilogue = instr.params[3] if len(instr.params) > 3 else L.EPI_NONE
         bias_off = instr.input_slices[2].offset if len(instr.input_slices) > 2 else -1
+        if residual is not None:
+            _check(self.lib.fnn_cuda_qmatmul_add(self.ctx, qw.handle, arena.handle, a_slice.offset,
+                                                 instr.output_slice.offset, bias_off, m, epilogue, self.path,
+                                                 residual.offset, total.offset))
+            return
         _check(self.lib.fnn_cuda_qmatmul(self.ctx, qw.handle, arena.handle, a_slice.offset,
                                          instr.output_slice.offset, bias_off, m, epilogue,
                                          self.path))

@@ -414,6 +414,8 @@ struct QmmArgs {
     int epilogue;
     const GatherArgs *gather = nullptr;
     const AllGatherArgs *allgather = nullptr;
+    const float *add = nullptr;   // [M,N]: sum = out + add beside out (fnn_cuda_qmatmul_add), or nullptr
+    float *sum = nullptr;
 };
 
 int launch_qmm_rows(fnn_cuda_ctx *ctx, const QmmArgs &args);

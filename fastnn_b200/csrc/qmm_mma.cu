@@ -145,6 +145,8 @@ struct MmaParams {
     const float *act;
     float *out;
     const float *bias;
+    const float *add;   // sum = out + add, where sum is given
+    float *sum;
     int M, N, K;
     int KB;          // k-blocks per row (padded)
     int ntiles;      // row tiles of 16
@@ -526,8 +528,10 @@ qmm_mma_kernel(MmaParams p) {
                                       bias, p.epilogue);
         if (CG == 1 && p.gather_on)
             gather_store(p.g, gc.step, m, n, r);
-        else
+        else {
             p.out[(size_t)m * p.N + n] = r;
+            if (p.sum) p.sum[(size_t)m * p.N + n] = __fadd_rn(r, ld_after_wait(p.add + (size_t)m * p.N + n));
+        }
     }
     if (CG == 1 && p.gather_on) gather_finish(p.g, gc.step, p.M, p.N);
 }
@@ -651,6 +655,8 @@ int launch_mma_g(fnn_cuda_ctx *ctx, const QmmArgs &a, const float *act, float *o
     p.act = act;
     p.out = out;
     p.bias = a.bias;
+    p.add = a.add ? a.add + (out - a.out) : nullptr;   // (`out` may start at a later batch row)
+    p.sum = a.sum ? a.sum + (out - a.out) : nullptr;
     p.M = M;
     p.N = (int)w->N;
     p.K = (int)w->K;
@@ -784,6 +790,10 @@ int launch_qmm_mma(fnn_cuda_ctx *ctx, const QmmArgs &a) {
             QmmArgs part = a;
             part.a = a.a + m0 * a.w->K;
             part.out = a.out + m0 * a.w->N;
+            if (a.sum) {
+                part.add = a.add + m0 * a.w->N;
+                part.sum = a.sum + m0 * a.w->N;
+            }
             part.M = std::min<size_t>(16, a.M - m0);
             rc = launch_qmm_mma8(ctx, part);
             if (rc != FNN_OK) return rc;

@@ -137,6 +137,8 @@ struct P8 {
     const float *act;
     float *out;
     const float *bias;
+    const float *add;   // sum = out + add, where sum is given
+    float *sum;
     int M, N, K;
     int KB, ntiles, tiles_per_group;
     int Kc;      // activations staged per pass (multiple of KBLK)
@@ -619,11 +621,17 @@ qmm_mma8_kernel(P8 p) {
         }
         cp_async_wait<0>();
     }
+    // the residual of this thread's first output is requested ahead of the barrier
+    const int total = tiles_here * 16 * p.M;
+    auto add_at = [&](int i) -> float {
+        const int tl = i / (16 * p.M), rem = i - tl * 16 * p.M, n = (gg + tl * GG) * 16 + (rem & 15);
+        return p.sum && i < total && n < p.N ? ld_after_wait(p.add + (size_t)(rem >> 4) * p.N + n) : 0.0f;
+    };
+    const float first_add = add_at(gtid);
     __syncthreads();
     const unsigned step = gc.step;
 
     // ---- epilogue ----------------------------------------------------------------------------
-    const int total = tiles_here * 16 * p.M;
     for (int i = gtid; i < total; i += kW8 * 32) {
         const int tl = i / (16 * p.M);
         const int rem = i - tl * 16 * p.M;
@@ -648,6 +656,7 @@ qmm_mma8_kernel(P8 p) {
         }
         if (!p.gather_on) {
             p.out[(size_t)m * p.N + n] = v;
+            if (p.sum) p.sum[(size_t)m * p.N + n] = __fadd_rn(v, i == gtid ? first_add : add_at(i));
         } else {
             gather_store(p.g, step, m, n, v);
         }
@@ -668,6 +677,8 @@ int launch8(fnn_cuda_ctx *ctx, const QmmArgs &a) {
     p.act = a.a;
     p.out = a.out;
     p.bias = a.bias;
+    p.add = a.add;
+    p.sum = a.sum;
     p.M = (int)a.M;
     p.N = (int)w->N;
     p.K = (int)w->K;

@@ -276,6 +276,8 @@ struct TcParams {
     const float *rowsum;
     const float *codebook;   // WF_CB: 16 centroids
     float *out;
+    const float *add;   // sum = out + add, where sum is given
+    float *sum;
     int *err_flag;
     int M, N, K;
     int Mb;        // batch rows per tile
@@ -642,6 +644,19 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
 #pragma unroll
                     for (int j = 0; j < W; ++j)
                         if (j < jmax) dst[(size_t)j * p.N] = v[j];
+                    if (p.sum) {   // the sums beside them, eight loads in flight together
+                        const float *ad = p.add + (size_t)m0 * p.N + n;
+                        float *sm = p.sum + (size_t)m0 * p.N + n;
+#pragma unroll
+                        for (int h = 0; h < W; h += 8) {
+                            float x[8];
+#pragma unroll
+                            for (int j = 0; j < 8; ++j) x[j] = h + j < jmax ? ld_after_wait(ad + (size_t)(h + j) * p.N) : 0.0f;
+#pragma unroll
+                            for (int j = 0; j < 8; ++j)
+                                if (h + j < jmax) sm[(size_t)(h + j) * p.N] = __fadd_rn(v[h + j], x[j]);
+                        }
+                    }
                 } else {   // plain peer stores over NVLink (and one local store)
                     const size_t at = (size_t)m0 * p.ag.n_total + p.ag.col0 + n;
                     for (int rk = 0; rk < p.ag.world; ++rk) {
@@ -947,6 +962,8 @@ int launch_tc(fnn_cuda_ctx *ctx, const QmmArgs &a, uint8_t *fixed_scratch = null
     p.rowsum = rowsum;
     p.codebook = w->codebook;
     p.out = a.out;
+    p.add = a.add;
+    p.sum = a.sum;
     p.err_flag = ctx->err_flag;
     p.M = M;
     p.N = N;

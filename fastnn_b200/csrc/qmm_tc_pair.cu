@@ -93,6 +93,8 @@ struct PairParams {
     const float *rowsum;
     const float *codebook;   // WF_CB: 16 centroids
     float *out;
+    const float *add;   // sum = out + add, where sum is given
+    float *sum;
     int *err_flag;
     int M, N;
     int Mb;        // batch rows per tile
@@ -378,6 +380,19 @@ qmm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
 #pragma unroll
                 for (int j = 0; j < 16; ++j)
                     if (j < jmax) dst[(size_t)j * p.N] = v[j];
+                if (p.sum) {   // the sums beside them, eight loads in flight together
+                    const float *ad = p.add + (size_t)m0 * p.N + n;
+                    float *sm = p.sum + (size_t)m0 * p.N + n;
+#pragma unroll
+                    for (int h = 0; h < 16; h += 8) {
+                        float x[8];
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) x[j] = h + j < jmax ? ld_after_wait(ad + (size_t)(h + j) * p.N) : 0.0f;
+#pragma unroll
+                        for (int j = 0; j < 8; ++j)
+                            if (h + j < jmax) sm[(size_t)(h + j) * p.N] = __fadd_rn(v[h + j], x[j]);
+                    }
+                }
                 fac = fac_next;
             }
             tc_fence_before();
@@ -440,6 +455,8 @@ int launch_pair(fnn_cuda_ctx *ctx, const QmmArgs &a, const PairTiling &tl) {
     p.rowsum = rowsum;
     p.codebook = w->codebook;
     p.out = a.out;
+    p.add = a.add;
+    p.sum = a.sum;
     p.err_flag = ctx->err_flag;
     p.M = M;
     p.N = N;

@@ -173,7 +173,15 @@ int fnn_cuda_qweight_dequant(fnn_cuda_qweight *w, fnn_cuda_arena *arena, size_t 
 int fnn_cuda_qmatmul(fnn_cuda_ctx *ctx, fnn_cuda_qweight *w, fnn_cuda_arena *arena,
                      size_t a_offset, size_t out_offset, int64_t bias_offset, size_t M,
                      int epilogue, int path);
-/* Same with explicit device pointers (activations/outputs outside any arena). */
+/* fnn_cuda_qmatmul followed by the plan's element-wise addition of another [M,N] slice to its result (a residual):
+ *   out[m,n] as above;  sum[m,n] = out[m,n] + add[m,n]
+ * Both slices are written, as by the two instructions.  The kernels store both from the same epilogue where the
+ * slices allow it, that is where neither `sum` nor `out` covers anything the other instruction reads (`sum` may be
+ * `add` itself); otherwise the two run one after the other. */
+int fnn_cuda_qmatmul_add(fnn_cuda_ctx *ctx, fnn_cuda_qweight *w, fnn_cuda_arena *arena,
+                         size_t a_offset, size_t out_offset, int64_t bias_offset, size_t M,
+                         int epilogue, int path, size_t add_offset, size_t sum_offset);
+/* Same as fnn_cuda_qmatmul with explicit device pointers (activations/outputs outside any arena). */
 int fnn_cuda_qmatmul_ptr(fnn_cuda_ctx *ctx, fnn_cuda_qweight *w, const float *a_dev,
                          float *out_dev, const float *bias_dev, size_t M, int epilogue,
                          int path);

@@ -1,0 +1,94 @@
+"""A MatMul and the addition of a residual to its result as one call against the two instructions, on every kernel that may
+serve it: the same bits in both slices, whatever the slices share."""
+import numpy as np
+import pytest
+
+import oracle as orc
+import fastnn_b200 as fnn
+from fastnn_b200 import _lib as L
+from helpers import normal
+from test_qmatmul_gpu import Rig, meta_of
+
+pytestmark = pytest.mark.gpu
+
+KERNELS = {orc.FMT_I8: "matmul_i8", orc.FMT_I4: "matmul_i4", orc.FMT_F8: "matmul_f8", orc.FMT_F4: "matmul_f4",
+           orc.FMT_I4CB: "matmul_i4"}
+
+
+def slots(m, k, n):
+    """a | out | add | sum | weight, in floats from the start of the arena"""
+    al = lambda x: -(-x // 64) * 64
+    a, out = 0, al(m * k)
+    add = out + al(m * n)
+    return a, out, add, add + al(m * n), add + 2 * al(m * n)
+
+
+# rows (K < 128), fragment kernels of one and of several rows, whole and shared tcgen05 tiles, two-SM tiles; ragged N
+@pytest.mark.parametrize("fmt", list(orc.FMT_NAMES))
+@pytest.mark.parametrize("m,k,n", [(3, 100, 37), (1, 1024, 600), (1, 4100, 2500), (4, 1024, 333), (7, 640, 1000),
+                                   (20, 1280, 130), (64, 256, 19100), (130, 384, 1001)])
+def test_sum_and_result_are_those_of_two_calls(backend, fmt, m, k, n):
+    q = orc.quantize_kn(fmt, normal(900 + k, (k, n), 0.02))
+    a, out, add, total, end = slots(m, k, n)
+    arena = backend.allocate_arena(4 * end)
+    w = backend.upload_qweight(q.payload, meta_of(q))
+    try:
+        def run(fused, sum_at):
+            backend.write_arena(arena, 0, np.zeros(end, np.float32).tobytes())
+            backend.write_arena(arena, 0, normal(901 + m, (m, k), 1.0).tobytes())
+            backend.write_arena(arena, 4 * add, normal(902 + n, (m, n), 1.0).tobytes())
+            args = (backend.ctx, w.handle, arena.handle, 4 * a, 4 * out, -1, m, L.EPI_SILU, L.PATH_AUTO)
+            if fused:
+                assert backend.lib.fnn_cuda_qmatmul_add(*args, 4 * add, 4 * sum_at) == 0, L.last_error()
+            else:
+                assert backend.lib.fnn_cuda_qmatmul(*args) == 0, L.last_error()
+                assert backend.lib.fnn_cuda_elementwise(backend.ctx, L.EW_ADD, arena.handle, 4 * out, m * n, 4 * add, m * n,
+                                                        4 * sum_at, m * n) == 0
+            return np.frombuffer(backend.read_arena(arena, 0, 4 * end), np.uint32).copy()
+
+        # a slice of its own; in place of the residual, of the result, of the activations (where they are large enough),
+        # and half over the residual
+        for sum_at in (total, add, out) + ((a,) if k >= n else ()):
+            assert (run(True, sum_at) == run(False, sum_at)).all(), sum_at
+    finally:
+        w.close()
+        arena.close()
+
+
+def test_plans_fuse_whole_residuals_only(backend):
+    """One launch less where the addition takes the MatMul's whole result and an equal slice; a broadcast, another
+    operand and a chain run as they stand."""
+    m, k, n = 2, 512, 256
+    q = orc.quantize_kn(orc.FMT_I8, normal(910, (k, n), 0.02))
+    a, out, add, total, end = slots(m, k, n)
+    payload = q.payload
+    arena = backend.allocate_arena(4 * end + len(payload) + 256)
+    f = lambda at, count: fnn.BufferSlice(4 * at, 4 * count)
+    weight = fnn.BufferSlice(4 * end, len(payload))
+    matmul = fnn.CallKernel("matmul_i8", [f(a, m * k), weight], f(out, m * n), [m, k, n, L.EPI_NONE], weight_meta=meta_of(q))
+    try:
+        backend.write_arena(arena, 4 * end, payload)
+        x, r = normal(911, (m, k), 1.0), normal(912, (m, n), 1.0)
+
+        def launches(second):
+            backend.write_arena(arena, 0, x.tobytes())
+            backend.write_arena(arena, 4 * add, r.tobytes())
+            plan = fnn.ExecutablePlan([matmul, second], arena.total_bytes)
+            backend.dispatch(plan, arena, fnn.ShapeEnv())       # (first use builds the layouts)
+            before = backend.launch_count()
+            backend.dispatch(plan, arena, fnn.ShapeEnv())
+            got = np.frombuffer(backend.read_arena(arena, 4 * total, 4 * m * n), np.float32).reshape(m, n)
+            y = np.frombuffer(backend.read_arena(arena, 4 * out, 4 * m * n), np.float32).reshape(m, n)
+            return backend.launch_count() - before, y, got
+
+        for ins in ([f(out, m * n), f(add, m * n)], [f(add, m * n), f(out, m * n)]):
+            count, y, got = launches(fnn.CallKernel("add_f32", ins, f(total, m * n), []))
+            assert count == 1 and (got == y + r).all()
+        count, y, got = launches(fnn.CallKernel("add_f32", [f(out, m * n), f(add, n)], f(total, m * n), []))
+        assert count == 2 and (got == y + r[0]).all()
+        count, y, got = launches(fnn.CallKernel("add_f32", [f(add, m * n), f(add, m * n)], f(total, m * n), []))
+        assert count == 2 and (got == r + r).all()
+        count, y, got = launches(fnn.CallKernel("mul_f32", [f(out, m * n), f(add, m * n)], f(total, m * n), []))
+        assert count == 2 and (got == y * r).all()
+    finally:
+        arena.close()
