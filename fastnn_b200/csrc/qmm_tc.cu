@@ -302,7 +302,12 @@ struct TcParams {
 // FP8 5.4 / 4.4).  Eight where the CTAs of a cluster deal the chunks out, for tiles of a single chunk of 16, which
 // would leave half of the warps idle, and for three terms, whose 48 accumulators a thread cost the registers that the
 // next kernel's early blocks need (FP4 64 rows K=2048: 11.0 / 12.3).
-template <int KIND, int T, int WF, int W>
+// SPLIT: the K blocks of a tile may be shared by a cluster (p.parts).  I8, FP8 and FP4 take whole tiles of up to 16 rows (FP8
+// and FP4 below 128 rows: all) through the same function, so that a program whose layers alternate between the two
+// keeps its instructions in the SMs' caches: with a function each every switch cost 0.7 us (six I8 pairs at 16
+// rows 161 / 154.5 us, four FP8 ones 119 / 110).  The widened formats, whose function is longer, are better off with
+// the two apart (four I4 pairs at 16 rows 75.3 / 72.2, six codebook ones at 64 155.3 / 152.8).
+template <int KIND, int T, int WF, int W, bool SPLIT>
 __global__ void __launch_bounds__((2 + kEpiWarps + xf_warps(WF)) * 32, 1)
 qmm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a,
               const __grid_constant__ CUtensorMap map_s, TcParams p) {
@@ -328,7 +333,8 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
     uint64_t *bars = reinterpret_cast<uint64_t *>(s_sc + (size_t)p.stages * sc_bytes);
     uint64_t *full = bars, *empty = bars + p.stages, *rawfull = bars + 2 * p.stages;
     uint64_t *tfull = bars + 3 * p.stages, *tempty = tfull + 2;
-    uint32_t *s_tmem = reinterpret_cast<uint32_t *>(tempty + 2);
+    uint64_t *tlast = tempty + 2;   // the accumulators of this CTA's last tile are complete
+    uint32_t *s_tmem = reinterpret_cast<uint32_t *>(tlast + 1);
     float *s_dump = reinterpret_cast<float *>(smem);   // parts > 1: raw accumulators [T * Mb][128], over the drained ring
     volatile int *s_abort = reinterpret_cast<volatile int *>(s_tmem + 1);
     float *s_cb = table_after(s_tmem + 2);                                // [16]
@@ -339,7 +345,8 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
 
     const int total_tiles = p.n_tiles * p.m_tiles;
     // whole tiles blockIdx.x, + gridDim.x, ...; a cluster of `parts` CTAs works on one tile
-    const int parts = p.parts, part = (int)(blockIdx.x % (unsigned)parts);
+    const int parts = SPLIT ? p.parts : 1, part = SPLIT ? (int)(blockIdx.x % (unsigned)parts) : 0;
+    const bool split = SPLIT && (WF != WF_TMA || parts > 1);
     const int first_tile = (int)(blockIdx.x / (unsigned)parts), tile_step = (int)(gridDim.x / (unsigned)parts);
     const int kb0 = p.kblocks * part / parts, kb1 = p.kblocks * (part + 1) / parts;
     // weights of stage `st`: the operand tile itself, or the packed nibbles (+ block scales) for the
@@ -376,6 +383,7 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
             mbar_init(&tfull[i], 1);
             mbar_init(&tempty[i], kEpiWarps);
         }
+        mbar_init(tlast, 1);
         *s_abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         // This thread is the TMA producer.  The weights do not depend on the kernel before this one on
@@ -493,7 +501,7 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
                     }
                 }
                 if (!ok) break;
-                tc_commit(&tfull[as]);  // accumulator complete
+                tc_commit(tile + tile_step < total_tiles ? &tfull[as] : tlast);  // accumulator complete
                 if (++as == p.nbuf) {
                     as = 0;
                     aphase ^= 1;
@@ -549,12 +557,17 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
                 }
             }
         }
-    } else if (warp < kXf0) {
-        // ---------------- epilogue (8 warps: a TMEM lane quadrant each, two warps per quadrant
-        // taking alternate 8-column chunks) ----------------
+    }
+    if (warp >= 2) {
+        // ---------------- epilogue (8 warps: a TMEM lane quadrant each, the two warps of a quadrant taking
+        // alternate chunks of the columns).  The transform warps have nothing left to do when the last tile's
+        // accumulators are complete and take their share of its chunks: every chunk is a chain of TMEM loads, exchange,
+        // shuffles and stores of about a microsecond, and at the end of a call all of it is exposed
+        // (us before / now: I4 M=64 K=4096 N=28672 24.1 / 23.7; together with the exchange below, N=4096 in three parts
+        // 10.5 / 10.0, codebook M=64 K=2048 N=8192 in two 11.1 / 10.6). ----------------
         pdl_wait();   // dq, rowsum and the output buffer belong to kernels before this one
         const int quad = warp & 3, grp = (warp - 2) >> 2;
-        constexpr int kStep = W * (kEpiWarps / 4);   // columns per round of a quadrant's warps
+        constexpr int kGroups = kEpiWarps / 4, kLastGroups = (kEpiWarps + xf_warps(WF)) / 4;   // warps per quadrant
         int as = 0;
         uint32_t aphase = 0;
         const bool has_zero = p.zeros != nullptr;
@@ -567,6 +580,12 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
             return want ? (lane < 16 ? p.dq : p.rowsum)[m] : 0.0f;
         };
         for (int tile = first_tile; tile < total_tiles; tile += tile_step) {
+            const bool last = tile + tile_step >= total_tiles;
+            if (WF != WF_TMA && !last && warp >= kXf0) {
+                if (++as == p.nbuf) as = 0;
+                continue;
+            }
+            const int step = W * (last ? kLastGroups : kGroups);   // columns per round of a quadrant's warps
             const int nt = tile / p.m_tiles, mt = tile - nt * p.m_tiles;
             // Everything the epilogue needs besides the accumulator is requested before the wait for
             // it, so these loads (a trip to L2 or HBM each) run under the tile's main loop.
@@ -576,13 +595,14 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
             const float zero = (n_ok && has_zero) ? __ldg(p.zeros + n) : 0.0f;
             const float bias = (n_ok && p.bias) ? p.bias[n] : 0.0f;
             float fac = load_rowfac(mt, chunk0);
-            const bool ok = mbar_wait(&tfull[as], aphase, s_abort, p.err_flag, 0x80);
+            const bool ok = last ? mbar_wait(tlast, 0, s_abort, p.err_flag, 0x80)
+                                 : mbar_wait(&tfull[as], aphase, s_abort, p.err_flag, 0x80);
             tc_fence_after();
             const uint32_t t_base = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(as * BNt);
-            if (parts > 1) {
+            if (split) {
                 // Every MMA of this CTA has read its operands, so the ring is free: the chunks that other
                 // CTAs finish go there ([column][row]: a warp stores 32 consecutive rows).
-                for (int c0 = grp * W; c0 < p.Mb && ok; c0 += kStep) {
+                for (int c0 = grp * W; c0 < p.Mb && ok; c0 += step) {
                     if ((c0 / W) % parts == part) continue;
 #pragma unroll
                     for (int t = 0; t < T; ++t) {
@@ -596,27 +616,61 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
                 __syncwarp();
                 cluster_sync();
             }
-            if (!ok) break;
-            for (int c0 = chunk0; c0 < p.Mb; c0 += parts * kStep) {
+            if (!ok) {
+                if (split) cluster_arrive();
+                break;
+            }
+            bool arrived = !split;
+            for (int c0 = chunk0; c0 < p.Mb; c0 += parts * step) {
                 uint32_t r[T][W];
 #pragma unroll
                 for (int t = 0; t < T; ++t) tmem_ld_cols(t_base + (uint32_t)(t * p.Mb + c0), r[t]);
-                const float fac_next = load_rowfac(mt, c0 + parts * kStep);   // next chunk's
+                const float fac_next = load_rowfac(mt, c0 + parts * step);   // next chunk's
                 tmem_ld_wait();
-                for (int q = 0; q < parts; ++q) {   // the other shares, in a fixed order
-                    if (q == part) continue;
-                    const uint32_t src = mapa(s_dump + (size_t)c0 * kTileN + row, (uint32_t)q);
-                    uint32_t x[T][W];
+                if (split) {
+                    // The other shares in a fixed order, two of them in flight at once where the registers allow it (I8 M=16
+                    // K=11008 N=4096 in three parts 14.4 -> 13.5 us; FP8 in flight behind the arrival below 10.1 -> 9.4).
+                    auto fetch = [&](int q, uint32_t (&x)[T][W]) {
+                        const uint32_t src = mapa(s_dump + (size_t)c0 * kTileN + row, (uint32_t)q);
 #pragma unroll
-                    for (int t = 0; t < T; ++t)
+                        for (int t = 0; t < T; ++t)
 #pragma unroll
-                        for (int j = 0; j < W; ++j) x[t][j] = ld_cluster(src + (uint32_t)((t * p.Mb + j) * kTileN * 4));
+                            for (int j = 0; j < W; ++j) x[t][j] = ld_cluster(src + (uint32_t)((t * p.Mb + j) * kTileN * 4));
+                    };
+                    auto add = [&](const uint32_t (&x)[T][W]) {
 #pragma unroll
-                    for (int t = 0; t < T; ++t)
+                        for (int t = 0; t < T; ++t)
 #pragma unroll
-                        for (int j = 0; j < W; ++j)
-                            r[t][j] = (KIND == KIND_I8) ? (uint32_t)((int)r[t][j] + (int)x[t][j])
-                                                        : __float_as_uint(__uint_as_float(r[t][j]) + __uint_as_float(x[t][j]));
+                            for (int j = 0; j < W; ++j)
+                                r[t][j] = (KIND == KIND_I8) ? (uint32_t)((int)r[t][j] + (int)x[t][j])
+                                                            : __float_as_uint(__uint_as_float(r[t][j]) + __uint_as_float(x[t][j]));
+                    };
+                    if constexpr (T == 3) {   // (the registers of a second one cost more)
+#pragma unroll 1
+                        for (int q = part + 1 < parts ? part + 1 : 0; q != part; q = q + 1 < parts ? q + 1 : 0) {
+                            uint32_t x[T][W];
+                            fetch(q, x);
+                            add(x);
+                        }
+                    } else
+                    for (int i = 1; i < parts; i += 2) {
+                        uint32_t x[T][W], y[T][W];
+                        const int q0 = part + i < parts ? part + i : part + i - parts;
+                        const int q1 = q0 + 1 < parts ? q0 + 1 : 0;
+                        fetch(q0, x);
+                        if (i + 1 < parts) {
+                            fetch(q1, y);
+                            add(x);
+                            add(y);
+                        } else {
+                            add(x);
+                        }
+                    }
+                    if (c0 + parts * step >= p.Mb) {   // this warp reads nothing more of the other CTAs
+                        __syncwarp();
+                        cluster_arrive();
+                        arrived = true;
+                    }
                 }
                 // The outputs of a chunk are computed in straight-line code (one specialisation per
                 // activation, no branch per output: with a branch per output the two warps a
@@ -668,9 +722,11 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
                 }
                 fac = fac_next;
             }
+            __syncwarp();
+            if (!arrived) cluster_arrive();
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&tempty[as]);
+            if (!last && lane == 0) mbar_arrive(&tempty[as]);
             if (++as == p.nbuf) {
                 as = 0;
                 aphase ^= 1;
@@ -679,11 +735,15 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
     }
 
     __syncwarp();
-    if (parts > 1) {
-        // The roles without an epilogue meet the exchange here; then nobody leaves while its shares are read.
-        if (warp < 2 || warp >= kXf0) cluster_sync();
+    if (split) {
+        // The roles without an epilogue meet the exchange here; then nobody leaves while its shares are read.  (The epilogue
+        // warps have arrived for that behind their last read.)
+        if (warp < 2) {
+            cluster_sync();
+            cluster_arrive();
+        }
         __syncwarp();
-        cluster_sync();
+        cluster_wait();
     }
     tc_fence_before();
     __syncthreads();
@@ -992,16 +1052,18 @@ int launch_tc(fnn_cuda_ctx *ctx, const QmmArgs &a, uint8_t *fixed_scratch = null
     // the exchange of a split lies over the drained ring, and the barriers are live right behind the ring
     FNN_REQUIRE(parts == 1 || (size_t)T * Mb * kTileN * 4 <= ring, FNN_ERR_DISPATCH,
                 "qmatmul: a ring of %d stages does not hold the partial accumulators of %d columns", stages, T * Mb);
-    size_t smem = 1024 + ring + (3 * stages + 4) * 8 + 8 + kTableBytes;
+    size_t smem = 1024 + ring + (3 * stages + 5) * 8 + 8 + kTableBytes;
     // A CTA of a split keeps its TMEM until its cluster has met, and the allocation is a wait without a bound: two CTAs
     // of a split on one SM could wait for each other's columns for good.  More than half of an SM's
     // shared memory each keeps them apart (I4 up to 16 rows asks for 98 KB and 512 columns).
     if (parts > 1) smem = std::max(smem, kHalfSmem);
     const int grid = parts > 1 ? tiles * parts : std::min(tiles, ctx->sm_count);
     const int threads = (2 + kEpiWarps + xf_warps(WF)) * 32;
-    auto kern = qmm_tc_kernel<KIND, T, WF, 8>;
+    auto kern = qmm_tc_kernel<KIND, T, WF, 8, true>;
+    if constexpr (WF != WF_TMA)
+        if (parts == 1) kern = qmm_tc_kernel<KIND, T, WF, 8, false>;
     if constexpr (T < 3)
-        if (parts == 1 && Mb > 16) kern = qmm_tc_kernel<KIND, T, WF, 16>;
+        if (parts == 1 && Mb > 16) kern = qmm_tc_kernel<KIND, T, WF, 16, false>;
     FNN_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
                    FNN_ERR_DISPATCH);
     if (parts > 1) {
