@@ -672,25 +672,9 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
                         arrived = true;
                     }
                 }
-                // The outputs of a chunk are computed in straight-line code (one specialisation per
-                // activation, no branch per output: with a branch per output the two warps a
-                // scheduler has here ran them one after another at full instruction latency), then
-                // stored under a predicate.
+                // (straight-line code, stored under a predicate)
                 float v[W];
-                switch (p.epilogue) {
-                case FNN_EPI_RELU:
-                    finish_chunk<KIND, T, FNN_EPI_RELU>(r, fac, scale, zero, bias, p.bias != nullptr, p.acc_scale, v);
-                    break;
-                case FNN_EPI_GELU:
-                    finish_chunk<KIND, T, FNN_EPI_GELU>(r, fac, scale, zero, bias, p.bias != nullptr, p.acc_scale, v);
-                    break;
-                case FNN_EPI_SILU:
-                    finish_chunk<KIND, T, FNN_EPI_SILU>(r, fac, scale, zero, bias, p.bias != nullptr, p.acc_scale, v);
-                    break;
-                default:
-                    finish_chunk<KIND, T, FNN_EPI_NONE>(r, fac, scale, zero, bias, p.bias != nullptr, p.acc_scale, v);
-                    break;
-                }
+                finish_chunk<KIND, T>(r, fac, scale, zero, bias, p.bias != nullptr, p.acc_scale, p.epilogue, v);
                 const int m0 = mt * p.Mb + c0;
                 const int jmax = n_ok ? min(W, min(p.Mb - c0, p.M - m0)) : 0;   // rows of this chunk that exist
                 if (p.ag.world == 0) {   // a warp writes 32 consecutive n

@@ -360,20 +360,7 @@ qmm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                 const float fac_next = load_rowfac(mt, c0 + kStep);
                 tmem_ld_wait();
                 float v[16];
-                switch (p.epilogue) {
-                case FNN_EPI_RELU:
-                    finish_chunk<KIND, T, FNN_EPI_RELU>(r, fac, scale, zero, bias, p.bias != nullptr, p.acc_scale, v);
-                    break;
-                case FNN_EPI_GELU:
-                    finish_chunk<KIND, T, FNN_EPI_GELU>(r, fac, scale, zero, bias, p.bias != nullptr, p.acc_scale, v);
-                    break;
-                case FNN_EPI_SILU:
-                    finish_chunk<KIND, T, FNN_EPI_SILU>(r, fac, scale, zero, bias, p.bias != nullptr, p.acc_scale, v);
-                    break;
-                default:
-                    finish_chunk<KIND, T, FNN_EPI_NONE>(r, fac, scale, zero, bias, p.bias != nullptr, p.acc_scale, v);
-                    break;
-                }
+                finish_chunk<KIND, T>(r, fac, scale, zero, bias, p.bias != nullptr, p.acc_scale, p.epilogue, v);
                 const int m0 = mt * p.Mb + c0;
                 const int jmax = n_ok ? min(16, min(p.Mb - c0, p.M - m0)) : 0;   // rows of this chunk that exist
                 float *dst = p.out + (size_t)m0 * p.N + n;   // a warp writes 32 consecutive n
