@@ -148,6 +148,32 @@ __device__ __forceinline__ float i8_to_f32(uint32_t word, int i) {
     return (float)(int8_t)((word >> (8 * i)) & 0xFFu);
 }
 
+// Four integers as the bytes of a word, the first one lowest.
+__device__ __forceinline__ uint32_t pack_s8(int a, int b, int c, int d) {
+    uint32_t high, w;
+    asm("cvt.pack.sat.s8.s32.b32 %0, %1, %2, 0;" : "=r"(high) : "r"(d), "r"(c));
+    asm("cvt.pack.sat.s8.s32.b32 %0, %1, %2, %3;" : "=r"(w) : "r"(b), "r"(a), "r"(high));
+    return w;
+}
+// Eight activations, already divided by the row's step, as int8 pairs hi * 128 + lo (15 bits): the two words of each.
+// PERM: in the order 0,2,4,6,1,3,5,7.
+template <bool PERM>
+__device__ __forceinline__ void int8_pairs(const float (&x)[8], uint32_t (&high)[2], uint32_t (&low)[2]) {
+    int hi[8], lo[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        const int q = max(-16256, min(16256, __float2int_rn(x[j])));
+        hi[j] = (q + 64) >> 7;
+        lo[j] = q - hi[j] * 128;
+    }
+    constexpr int S = PERM ? 2 : 1, H = PERM ? 1 : 4;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        high[h] = pack_s8(hi[h * H], hi[h * H + S], hi[h * H + 2 * S], hi[h * H + 3 * S]);
+        low[h] = pack_s8(lo[h * H], lo[h * H + S], lo[h * H + 2 * S], lo[h * H + 3 * S]);
+    }
+}
+
 // act(x) of the fused epilogue (src/backend/cpu/mod.rs:3140-3171).
 __device__ __forceinline__ float apply_act(float x, int epi) {
     switch (epi) {

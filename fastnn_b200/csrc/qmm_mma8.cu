@@ -371,18 +371,10 @@ qmm_mma8_kernel(P8 p) {
                     for (int m = 0; m < 4; ++m) {
                         if (mb + m < p.M) {
                             const float inv = 1.0f / s_dq[mb + m];
-                            const float e[8] = {v[m][0].x, v[m][0].y, v[m][0].z, v[m][0].w,
-                                                v[m][1].x, v[m][1].y, v[m][1].z, v[m][1].w};
-                            uint32_t hi[2] = {0u, 0u}, lo[2] = {0u, 0u};
-#pragma unroll
-                            for (int j = 0; j < 8; ++j) {
-                                int q = __float2int_rn(e[j] * inv);
-                                q = max(-16256, min(16256, q));
-                                const int h = (q + 64) >> 7;
-                                const int pos = inner_pos8<FMT>(j);   // position inside the 8-group
-                                hi[pos >> 2] |= (uint32_t)(h & 0xFF) << ((pos & 3) * 8);
-                                lo[pos >> 2] |= (uint32_t)((q - h * 128) & 0xFF) << ((pos & 3) * 8);
-                            }
+                            const float e[8] = {v[m][0].x * inv, v[m][0].y * inv, v[m][0].z * inv, v[m][0].w * inv,
+                                                v[m][1].x * inv, v[m][1].y * inv, v[m][1].z * inv, v[m][1].w * inv};
+                            uint32_t hi[2], lo[2];
+                            int8_pairs<FMT == FNN_FMT_I4>(e, hi, lo);   // (inner_pos8)
                             const int gp = group_pos8<FMT>(i8 * 8);
                             *reinterpret_cast<uint2 *>(s_act + (size_t)(mb + m) * RS + gp) = make_uint2(hi[0], hi[1]);
                             *reinterpret_cast<uint2 *>(s_act + (size_t)(p.M + mb + m) * RS + gp) =
@@ -411,16 +403,11 @@ qmm_mma8_kernel(P8 p) {
             for (int j = 0; j < kHeld; ++j) {
                 const int g8 = tid + j * NT;
                 if (g8 * 8 >= kc_len) continue;   // (beyond K the held values are zero: the padding of the last block)
-                uint32_t hi[2] = {0u, 0u}, lo[2] = {0u, 0u};
+                float e[8];
 #pragma unroll
-                for (int q8 = 0; q8 < 8; ++q8) {
-                    int q = __float2int_rn(hv[j][q8] * inv);
-                    q = max(-16256, min(16256, q));
-                    const int h = (q + 64) >> 7;
-                    const int pos = inner_pos8<FMT>(q8);
-                    hi[pos >> 2] |= (uint32_t)(h & 0xFF) << ((pos & 3) * 8);
-                    lo[pos >> 2] |= (uint32_t)((q - h * 128) & 0xFF) << ((pos & 3) * 8);
-                }
+                for (int q8 = 0; q8 < 8; ++q8) e[q8] = hv[j][q8] * inv;
+                uint32_t hi[2], lo[2];
+                int8_pairs<FMT == FNN_FMT_I4>(e, hi, lo);   // (inner_pos8)
                 const int gp = group_pos8<FMT>(g8 * 8);
                 *reinterpret_cast<uint2 *>(s_act + gp) = make_uint2(hi[0], hi[1]);
                 *reinterpret_cast<uint2 *>(s_act + (size_t)RS + gp) = make_uint2(lo[0], lo[1]);
@@ -625,9 +612,10 @@ qmm_mma8_kernel(P8 p) {
     const int total = tiles_here * 16 * p.M;
     auto add_at = [&](int i) -> float {
         const int tl = i / (16 * p.M), rem = i - tl * 16 * p.M, n = (gg + tl * GG) * 16 + (rem & 15);
-        return p.sum && i < total && n < p.N ? ld_after_wait(p.add + (size_t)(rem >> 4) * p.N + n) : 0.0f;
+        return i < total && n < p.N ? ld_after_wait(p.add + (size_t)(rem >> 4) * p.N + n) : 0.0f;
     };
-    const float first_add = add_at(gtid);
+    float first_add = 0.0f;
+    if (p.sum) first_add = add_at(gtid);
     __syncthreads();
     const unsigned step = gc.step;
 

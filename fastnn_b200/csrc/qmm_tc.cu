@@ -59,33 +59,14 @@ __device__ __forceinline__ void split_terms(float x, uint8_t t[3]) {
     }
 }
 
-// Four integers as the bytes of a word, the first one lowest.
-__device__ __forceinline__ uint32_t pack_s8(int a, int b, int c, int d) {
-    uint32_t high, w;
-    asm("cvt.pack.sat.s8.s32.b32 %0, %1, %2, 0;" : "=r"(high) : "r"(d), "r"(c));
-    asm("cvt.pack.sat.s8.s32.b32 %0, %1, %2, %3;" : "=r"(w) : "r"(b), "r"(a), "r"(high));
-    return w;
-}
-// The same for a unit of eight, as the two words of each term (the bytes split_terms gives).  Two elements per conversion and
+// split_terms for a unit of eight, as the two words of each term (the bytes split_terms gives).  Two elements per conversion and
 // four per pack: a block runs this code once per unit it holds, straight through, and fetching it is what it waits for (us
 // element by element / so: four FP8 pairs at 16 rows 108.3 / 106.0, at 24 rows of K=3072 94.0 / 90.4; FP4 M=4 K=8192 N=28672
 // 29.6 / 29.1; four I4 decoder layers at 64 rows 299.4 / 298.7).
 template <int KIND, int T, bool PERM8>
 __device__ __forceinline__ void split_unit(float (&x)[8], uint32_t (&w)[T][2]) {
     if constexpr (KIND == KIND_I8) {
-        int hi[8], lo[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int q = max(-16256, min(16256, __float2int_rn(x[j])));
-            hi[j] = (q + 64) >> 7;
-            lo[j] = q - hi[j] * 128;
-        }
-        constexpr int S = PERM8 ? 2 : 1, H = PERM8 ? 1 : 4;   // k 0,2,4,6 | 1,3,5,7 or 0..3 | 4..7
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            w[0][h] = pack_s8(hi[h * H], hi[h * H + S], hi[h * H + 2 * S], hi[h * H + 3 * S]);
-            w[T - 1][h] = pack_s8(lo[h * H], lo[h * H + S], lo[h * H + 2 * S], lo[h * H + 3 * S]);
-        }
+        int8_pairs<PERM8>(x, w[0], w[T - 1]);
     } else {
 #pragma unroll
         for (int t = 0; t < T; ++t) {
