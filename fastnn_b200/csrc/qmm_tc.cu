@@ -163,19 +163,23 @@ act_prep_kernel(const float *act, int M, int K, int Kp, uint8_t *bq, float *dq, 
 // The same rewrite for rows of at most 32768 elements, read once: a thread holds HOLD units of eight consecutive elements
 // between the scan and the rewrite, with all loads in flight together, and every plane is written eight bytes at a
 // time.  (The loop above is a chain of two passes of 4-byte loads, about 8 us for K=11308.)
-// CLUSTER (I4 only): no more rows than SMs, more than 4096 elements each.  The rewrite is then bound by latency, and a block
+// CLUSTER (I4 only): 32 rows to a row per SM, more than 4096 elements each.  The rewrite is then bound by latency, and a block
 // that holds up to 16 units a thread needs registers that the main kernel's 576 threads leave on no SM, so that the CTAs
 // which share an SM with one start when the rewrite is done.  The blocks of a cluster take an even part of a row
 // each and hand their maxima and sums round through distributed shared memory: two units a thread and 40 registers
 // whatever the length, which fit.  M=64 K=14336 N=4096 19.7 -> 18.4 us.  The main kernels of the other formats leave
 // room for the single block (I8, FP8, FP4: 320 threads) or for neither (codebook: 832); they lose the half microsecond that
 // the cluster's barriers take (FP8 M=32 K=11008 N=4096 16.6 / 17.5, FP4 M=4 K=8192 N=28672 29.4 / 30.1), and so do
-// more rows than SMs (M=4096 K=8192 N=1024 93.8 / 106).
+// more rows than SMs (M=4096 K=8192 N=1024 93.8 / 106) and few, whose blocks are on few SMs (I4 M=4 K=6000 N=4096 6.9 / 7.8,
+// three decoder layers at 16 rows 135.8 / 138.5).
 constexpr int kPrepCluster = 8;    // blocks of the longest rows
 constexpr int kPrepHold = 16;      // units a thread holds of the longest rows in one block
 // VEC: rows of a multiple of four elements that start on 16 bytes (every layer of a real model); else 4-byte loads.
-template <int KIND, int T, bool PERM8, int HOLD, bool VEC, bool CLUSTER>
-__global__ void __launch_bounds__(256)
+// LEAN: 32 registers a thread instead of 40.  With a few rows the blocks then fit beside the fragment kernels' 512 threads of 112,
+// which leave 8192, and start before those end (I4 M=8 K=4096 N=6144 9.7 -> 8.2 us, N=22528 18.1 -> 15.4); from 33 rows on the
+// wider form is a little faster (four I4 decoder layers at 64 rows 302.0 lean, 299.1).
+template <int KIND, int T, bool PERM8, int HOLD, bool VEC, bool CLUSTER, bool LEAN>
+__global__ void __launch_bounds__(256, LEAN ? 8 : 1)
 act_prep_regs_kernel(const float *act, int M, int K, int Kp, int blocks, uint8_t *bq, float *dq, float *rowsum) {
     __shared__ float2 s_part[8];                       // of this block's warps
     __shared__ float2 s_all[kPrepCluster];             // of the row's blocks
@@ -861,11 +865,12 @@ int tc::encode_block_scale_map(CUtensorMap *map, const fnn_cuda_qweight *w) {
 namespace {
 
 template <int KIND, int T, bool PERM8, bool VEC>
-auto prep_kernel(int K) {
-    return K <= 2 * 256 * 8   ? act_prep_regs_kernel<KIND, T, PERM8, 2, VEC, false>
-           : K <= 4 * 256 * 8 ? act_prep_regs_kernel<KIND, T, PERM8, 4, VEC, false>
-           : K <= 8 * 256 * 8 ? act_prep_regs_kernel<KIND, T, PERM8, 8, VEC, false>
-                              : act_prep_regs_kernel<KIND, T, PERM8, kPrepHold, VEC, false>;
+auto prep_kernel(int M, int K) {
+    return K <= 2 * 256 * 8   ? (M <= 32 ? act_prep_regs_kernel<KIND, T, PERM8, 2, VEC, false, true>
+                                         : act_prep_regs_kernel<KIND, T, PERM8, 2, VEC, false, false>)
+           : K <= 4 * 256 * 8 ? act_prep_regs_kernel<KIND, T, PERM8, 4, VEC, false, false>
+           : K <= 8 * 256 * 8 ? act_prep_regs_kernel<KIND, T, PERM8, 8, VEC, false, false>
+                              : act_prep_regs_kernel<KIND, T, PERM8, kPrepHold, VEC, false, false>;
 }
 
 template <int KIND, int T, bool PERM8>
@@ -885,10 +890,11 @@ int launch_prep(fnn_cuda_ctx *ctx, const QmmArgs &a, int Kp, uint8_t *bq, float 
         return FNN_OK;
     }
     if constexpr (PERM8) {   // (I4)
-        if (K > 2 * 256 * 8 && M <= ctx->sm_count) {
+        if (K > 2 * 256 * 8 && M >= 32 && M <= ctx->sm_count) {
             const int blocks = (K + 2 * 256 * 8 - 1) / (2 * 256 * 8);
             static_assert(kPrepCluster * 2 >= kPrepHold, "a cluster covers the longest row");
-            auto prep = vec ? act_prep_regs_kernel<KIND, T, PERM8, 2, true, true> : act_prep_regs_kernel<KIND, T, PERM8, 2, false, true>;
+            auto prep = vec ? act_prep_regs_kernel<KIND, T, PERM8, 2, true, true, false>
+                            : act_prep_regs_kernel<KIND, T, PERM8, 2, false, true, false>;
             FNN_CUDA_CHECK(carve_out(prep), FNN_ERR_DISPATCH);
             FNN_CUDA_CHECK(launch_pdl_cluster(prep, M * blocks, blocks, 256, 0, ctx, a.a, M, K, Kp, blocks, bq, dq, rowsum),
                            FNN_ERR_DISPATCH);
@@ -896,7 +902,7 @@ int launch_prep(fnn_cuda_ctx *ctx, const QmmArgs &a, int Kp, uint8_t *bq, float 
             return FNN_OK;
         }
     }
-    auto prep = vec ? prep_kernel<KIND, T, PERM8, true>(K) : prep_kernel<KIND, T, PERM8, false>(K);
+    auto prep = vec ? prep_kernel<KIND, T, PERM8, true>(M, K) : prep_kernel<KIND, T, PERM8, false>(M, K);
     FNN_CUDA_CHECK(carve_out(prep), FNN_ERR_DISPATCH);
     FNN_CUDA_CHECK(launch_pdl(prep, M, 256, 0, ctx, a.a, M, K, Kp, 1, bq, dq, rowsum), FNN_ERR_DISPATCH);
     ctx->launches++;

@@ -62,13 +62,19 @@ def test_rewritten_rows_of_any_length(backend, fmt, k):
     check(backend, fmt, k, 40, [3, 9])
 
 
-# I4 rows of more than 4096 elements are shared by the blocks of a cluster up to a row per SM: both sides of that line, whole and
-# short last units, parts of unequal length
-@pytest.mark.parametrize("k", [4104, 8209])
+# I4 rows of more than 4096 elements are shared by the blocks of a cluster from 32 rows up to a row per SM: both sides of
+# those lines, whole and short last units, parts of unequal length; and up to 4096 the form of at most 32 rows
+@pytest.mark.parametrize("k", [4091, 4104, 8209])
 def test_rewritten_rows_by_cluster_or_by_block(backend, k):
     import torch
     sms = torch.cuda.get_device_properties(0).multi_processor_count
-    check(backend, orc.FMT_I4, k, 40, [sms, sms + 1])
+    check(backend, orc.FMT_I4, k, 40, [31, 32, 33, sms, sms + 1])
+
+
+# the cluster's longest rows: eight parts, and a last unit of one element
+@pytest.mark.parametrize("k", [14336, 20009, 32768])
+def test_long_rows_rewritten_by_clusters(backend, k):
+    check(backend, orc.FMT_I4, k, 40, [32, 40])
 
 
 def random_codes(fmt, k, n, seed):
