@@ -60,6 +60,14 @@ __device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
     return d;
 }
 
+// Contiguous bytes (a multiple of 16, both ends on 16) into shared memory; reports to `bar`.
+__device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t bytes, uint64_t *bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                     tc::smem_u32(dst)),
+                 "l"(src), "r"(bytes), "r"(tc::smem_u32(bar))
+                 : "memory");
+}
+
 // Eight 4-bit codes of one word -> the two A registers of one m16n8k32 MMA.
 //   I4: lo = 16*q of codes 0,2,4,6 ; hi = 16*q of codes 1,3,5,7 (the activations are staged in the
 //       matching order 0,2,4,6,1,3,5,7 of each 8-group)
@@ -147,6 +155,7 @@ struct P8 {
     const uint8_t *planes;
     const float *dq, *rowsum;
     int Kp;
+    int *err_flag;
     int gather_on;
     GatherArgs g;
 };
@@ -234,6 +243,13 @@ qmm_mma8_kernel(P8 p) {
     constexpr bool kCanHold = kHeld > 0;
     float hv[kCanHold ? kHeld : 1][8];
     bool held = false;
+    __shared__ uint64_t s_rows_bar[1];   // PLANES: the rows of a pass have landed
+    __shared__ volatile int s_abort[1];
+    if (PLANES && tid == 0) {
+        tc::mbar_init(s_rows_bar, 1);
+        *s_abort = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }   // (published by the barrier ahead of the first pass)
     for (int k0 = 0; k0 < Kpad; k0 += p.Kc) {
         const int kc_len = min(p.Kc, Kpad - k0);
         const int KBc = kc_len / KBLK;
@@ -340,15 +356,25 @@ qmm_mma8_kernel(P8 p) {
         __syncthreads();  // previous pass fully consumed
         // ---- stage the activation bytes of [k0, k0 + kc_len) --------------------------------
         if (PLANES) {
-            // copies of the rewritten rows, sixteen bytes at a time
-            const int pieces = kc_len / 16;
-            for (int i = tid; i < 2 * p.M * pieces; i += NT) {
-                const int r = i / pieces, k = (i - r * pieces) * 16;   // plane-major rows, as staged
-                const bool in = k0 + k < p.Kp;
-                frag::cp_async16(s_act + (size_t)r * RS + k, p.planes + (in ? (size_t)r * p.Kp + k0 + k : 0), in ? 16 : 0);
+            // One bulk copy per rewritten row (plane-major, as staged), issued by the lanes of a warp.  Sixteen bytes at a
+            // time through all threads the copies and their index arithmetic took 1.7 us, and waiting for them drained the
+            // weights' ring too (I4 M=8 K=4096 N=4096 7.75 -> 6.45 us).  What the last k-block has beyond the planes is cleared.
+            const int bytes = min(kc_len, p.Kp - k0);
+            if (warp == 0) {
+                if (lane == 0) {
+                    tc::fence_proxy_async();   // (an earlier pass read these rows)
+                    tc::mbar_expect_tx(s_rows_bar, (uint32_t)(cols * bytes));
+                }
+                __syncwarp();
+                if (lane < cols)
+                    bulk_load(s_act + (size_t)lane * RS, p.planes + (size_t)lane * p.Kp + k0, (uint32_t)bytes, s_rows_bar);
             }
-            cp_async_commit();
-            cp_async_wait<0>();
+            if (kc_len > bytes)
+                for (int i = tid; i < cols * (kc_len - bytes) / 16; i += NT) {
+                    const int pieces = (kc_len - bytes) / 16, r = i / pieces;
+                    *reinterpret_cast<uint4 *>(s_act + (size_t)r * RS + bytes + (i - r * pieces) * 16) = make_uint4(0u, 0u, 0u, 0u);
+                }
+            (void)tc::mbar_wait(s_rows_bar, (uint32_t)(k0 / p.Kc) & 1u, s_abort, p.err_flag, 0x1000);
         } else if (MULTI && vec_ok && (p.K % 8 == 0)) {
             // eight activations of four rows per thread and step: two 16-byte loads per row in flight,
             // one 8-byte store per (row, plane)
@@ -694,6 +720,7 @@ int launch8(fnn_cuda_ctx *ctx, const QmmArgs &a) {
             p.dq = dq;
             p.rowsum = rowsum;
             p.Kp = (int)lay.Kp;
+            p.err_flag = ctx->err_flag;
         }
     }
     const int cols = 2 * p.M;   // int8 pairs
