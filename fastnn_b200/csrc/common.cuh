@@ -97,7 +97,7 @@ struct fnn_cuda_qweight {
     uint4 *frag = nullptr;
     size_t frag_bytes = 0;
     float *frag_bs = nullptr;   // I4CB block scales in fragment order
-    uint4 *cb_tables = nullptr; // I4CB centroids as the 8-bit fragment kernel reads them
+    uint4 *cb_tables = nullptr; // I4CB centroids as the 8-bit fragment kernel reads them (behind frag_bs)
     bool fp16_ok = true;         // codebook format: false when block scales or centroids would leave the fp16 range
                                 // of the tcgen05 kernel's dequantized operand
 };

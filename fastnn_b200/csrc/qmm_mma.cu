@@ -619,8 +619,9 @@ int ensure_frag(fnn_cuda_ctx *ctx, fnn_cuda_qweight *w) {
     const size_t ntiles = div_ceil(w->N, 16);
     const size_t units = ntiles * KB * 64;
     if (w->fmt == FNN_FMT_I4CB) {   // before `frag`, whose presence says that all of them are there
-        if (!w->frag_bs) FNN_CUDA_CHECK(cudaMalloc((void **)&w->frag_bs, units * sizeof(float)), FNN_ERR_MEMORY);
-        if (!w->cb_tables) FNN_CUDA_CHECK(cudaMalloc((void **)&w->cb_tables, 3 * sizeof(uint4)), FNN_ERR_MEMORY);
+        if (!w->frag_bs)
+            FNN_CUDA_CHECK(cudaMalloc((void **)&w->frag_bs, units * sizeof(float) + 3 * sizeof(uint4)), FNN_ERR_MEMORY);
+        w->cb_tables = reinterpret_cast<uint4 *>(w->frag_bs + units);   // (units is a multiple of 64)
     }
     FNN_CUDA_CHECK(cudaMalloc((void **)&w->frag, units * sizeof(uint4)), FNN_ERR_MEMORY);
     w->frag_bytes = units * sizeof(uint4);

@@ -12,7 +12,6 @@ namespace fnn {
 void free_qweight_aux(fnn_cuda_qweight *w) {
     if (w->frag) cudaFree(w->frag);
     if (w->frag_bs) cudaFree(w->frag_bs);
-    if (w->cb_tables) cudaFree(w->cb_tables);
     w->frag = nullptr;
     w->frag_bs = nullptr;
     w->cb_tables = nullptr;
