@@ -551,13 +551,12 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
         const uint32_t t_dst = tmem_ops + ((uint32_t)(quad * 32) << 16);
         int s = 0;
         uint32_t phase = 0;
-        bool ok = true;
-        for (int tile = first_tile; tile < total_tiles && ok; tile += tile_step) {
+        bool filled = true;
+        for (int tile = first_tile; tile < total_tiles; tile += tile_step) {
             for (int kb = kb0; kb < kb1; ++kb) {
-                if (!mbar_wait(&rawfull[s], phase, s_abort, p.err_flag, 0x200)) {
-                    ok = false;
-                    break;
-                }
+                // (a lane that gives up stays with its warp through this step and the others, whatever the stages hold, and reports
+                // no stage any more: a vote, which ends the loop for all, cost 1 % of a decoder step)
+                filled = filled && mbar_wait(&rawfull[s], phase, s_abort, p.err_flag, 0x200);
                 tc_fence_after();   // the stage's columns were last read by MMAs another thread issued
                 const unsigned char *raw = s_raw + (size_t)s * raw_bytes + row * 64;
 #pragma unroll
@@ -577,7 +576,7 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
                 tmem_st_wait();
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&full[s]);
+                if (lane == 0 && filled) mbar_arrive(&full[s]);
                 if (++s == p.stages) {
                     s = 0;
                     phase ^= 1;
@@ -622,8 +621,7 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
             const float zero = (n_ok && has_zero) ? __ldg(p.zeros + n) : 0.0f;
             const float bias = (n_ok && p.bias) ? p.bias[n] : 0.0f;
             float fac = load_rowfac(mt, chunk0);
-            const bool ok = last ? mbar_wait(tlast, 0, s_abort, p.err_flag, 0x80)
-                                 : mbar_wait(&tfull[as], aphase, s_abort, p.err_flag, 0x80);
+            const bool ok = mbar_wait_warp(last ? tlast : &tfull[as], last ? 0u : aphase, s_abort, p.err_flag, 0x80);
             tc_fence_after();
             const uint32_t t_base = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(as * BNt);
             if (split) {

@@ -292,13 +292,12 @@ qmm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         const int xt = threadIdx.x - kXf0 * 32;
         int s = 0;
         uint32_t phase = 0;
-        bool ok = true;
-        for (int tile = pair; tile < total_tiles && ok; tile += pairs) {
+        bool filled = true;
+        for (int tile = pair; tile < total_tiles; tile += pairs) {
             for (int kb = 0; kb < p.kblocks; ++kb) {
-                if (!mbar_wait(&rawfull[s], phase, s_abort, p.err_flag, 0x200)) {
-                    ok = false;
-                    break;
-                }
+                // (a lane that gives up stays with its warp through this step and the others, whatever the stages hold, and reports
+                // no stage any more: a vote, which ends the loop for all, cost 1 % of a decoder step)
+                filled = filled && mbar_wait(&rawfull[s], phase, s_abort, p.err_flag, 0x200);
                 const unsigned char *raw = s_raw + (size_t)s * (kRawBytes + kScBytes);
                 unsigned char *dst = s_a + (size_t)s * a_bytes;
 #pragma unroll
@@ -320,7 +319,7 @@ qmm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                 }
                 fence_proxy_async();   // these stores are read by the tensor cores (async proxy)
                 __syncwarp();
-                if (lane == 0) mbar_arrive_cluster(mapa(&full[s], 0));
+                if (lane == 0 && filled) mbar_arrive_cluster(mapa(&full[s], 0));
                 if (++s == p.stages) {
                     s = 0;
                     phase ^= 1;
@@ -350,7 +349,7 @@ qmm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             const float zero = (n_ok && has_zero) ? __ldg(p.zeros + n) : 0.0f;
             const float bias = (n_ok && p.bias) ? p.bias[n] : 0.0f;
             float fac = load_rowfac(mt, chunk0);
-            if (!mbar_wait(&tfull[as], aphase, s_abort, p.err_flag, 0x80)) break;
+            if (!mbar_wait_warp(&tfull[as], aphase, s_abort, p.err_flag, 0x80)) break;
             tc_fence_after();
             const uint32_t t_base = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(as * acc_cols);
             for (int c0 = chunk0; c0 < p.Mb; c0 += kStep) {

@@ -80,6 +80,13 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, volati
         }
     }
 }
+// The same for a whole warp, with one answer for all of its lanes.  Each lane polls by itself, so one may see the phase
+// complete while another sees the abort flag, and what follows is for a converged warp: tcgen05 loads, and the
+// arrivals at a cluster barrier, of which every warp owes the same number on every path.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t *bar, uint32_t parity, volatile int *abort_flag, int *err_flag,
+                                               int code) {
+    return __all_sync(0xFFFFFFFFu, mbar_wait(bar, parity, abort_flag, err_flag, code));
+}
 __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, uint64_t *bar, int c0,
                                             int c1) {
     asm volatile(

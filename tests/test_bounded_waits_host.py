@@ -1,0 +1,44 @@
+"""How the kernels use their bounded waits, read from the sources: what happens when a wait gives up cannot be tried on a GPU
+(it would take a kernel that is broken on purpose)."""
+import os
+import re
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "fastnn_b200", "csrc")
+
+
+def code_of(name):
+    with open(os.path.join(CSRC, name)) as f:
+        return re.sub(r"//[^\n]*", "", f.read())
+
+
+def block_after(text, at):
+    """The span of the braces that open behind `at`."""
+    first = text.index("{", at)
+    depth = 0
+    for i in range(first, len(text)):
+        depth += {"{": 1, "}": -1}.get(text[i], 0)
+        if depth == 0:
+            return first, i
+    raise AssertionError("unbalanced braces")
+
+
+@pytest.mark.parametrize("name", ["qmm_tc.cu", "qmm_tc_pair.cu"])
+def test_waits_of_whole_warps_have_one_answer(name):
+    """Outside the blocks of an elected thread every lane of a warp waits by itself, and what follows is for converged warps:
+    tensor-memory accesses and cluster arrivals.  So either the wait votes, or its answer decides over nothing but one
+    lane's arrival, and the lanes stay together whatever it is."""
+    text = code_of(name)
+    elected = [block_after(text, m.start()) for m in re.finditer(r"if \(elect_one\(\)\)", text)]
+    assert elected
+    inside = lambda at: any(a <= at <= b for a, b in elected)
+    whole = [m.start() for m in re.finditer(r"\bmbar_wait_warp\(", text)]
+    assert whole and not any(inside(at) for at in whole)
+    lone = [m for m in re.finditer(r"(?:(\w+) = \1 && )?\bmbar_wait\(", text) if not inside(m.start())]
+    assert len(lone) == 1
+    answer = lone[0].group(1)   # once it is false it stays false
+    assert answer, text[lone[0].start():][:80]
+    uses = [u.strip() for u in re.findall(rf"[^;{{}}]*\b{answer}\b[^;]*;", text)]
+    assert len(uses) == 3 and uses[0] == f"bool {answer} = true;", uses
+    assert uses[2].startswith(f"if (lane == 0 && {answer}) mbar_arrive"), uses
