@@ -354,6 +354,7 @@ qmm_mma8_kernel(P8 p) {
         }
 
         __syncthreads();  // previous pass fully consumed
+        bool landed = true;
         // ---- stage the activation bytes of [k0, k0 + kc_len) --------------------------------
         if (PLANES) {
             // One bulk copy per rewritten row (plane-major, as staged), issued by the lanes of a warp.  Sixteen bytes at a
@@ -374,7 +375,7 @@ qmm_mma8_kernel(P8 p) {
                     const int pieces = (kc_len - bytes) / 16, r = i / pieces;
                     *reinterpret_cast<uint4 *>(s_act + (size_t)r * RS + bytes + (i - r * pieces) * 16) = make_uint4(0u, 0u, 0u, 0u);
                 }
-            (void)tc::mbar_wait(s_rows_bar, (uint32_t)(k0 / p.Kc) & 1u, s_abort, p.err_flag, 0x1000);
+            landed = tc::mbar_wait(s_rows_bar, (uint32_t)(k0 / p.Kc) & 1u, s_abort, p.err_flag, 0x1000);
         } else if (MULTI && vec_ok && (p.K % 8 == 0)) {
             // eight activations of four rows per thread and step: two 16-byte loads per row in flight,
             // one 8-byte store per (row, plane)
@@ -490,7 +491,16 @@ qmm_mma8_kernel(P8 p) {
                 for (int k = tid; k < kc_len; k += NT) put(k, (k0 + k < p.K) ? ld_after_wait(row + k0 + k) : 0.0f);
             }
         }
-        __syncthreads();
+        if (!PLANES) {
+            __syncthreads();
+        } else if (!__syncthreads_and(landed)) {
+            // The rows have not come: nothing is stored, the residual's slice least of all.  Copies already in flight land
+            // before the block's shared memory goes to another.
+            cp_async_wait<0>();
+            if (tid == 0)
+                for (int i = 0; i < 64; ++i) __nanosleep(1000);
+            return;
+        }
         if (CB && !(kCanHold && held)) {
             // -8192 * sum of each 32-element block of every staged column: the centroids are carried
             // with an offset of 8192, which the second MMA of a block takes back through its C operand

@@ -42,3 +42,25 @@ def test_waits_of_whole_warps_have_one_answer(name):
     uses = [u.strip() for u in re.findall(rf"[^;{{}}]*\b{answer}\b[^;]*;", text)]
     assert len(uses) == 3 and uses[0] == f"bool {answer} = true;", uses
     assert uses[2].startswith(f"if (lane == 0 && {answer}) mbar_arrive"), uses
+
+
+@pytest.mark.parametrize("name", ["qmm_mma8.cu", "qmm_tc.cu", "qmm_tc_pair.cu"])
+def test_no_answer_of_a_wait_is_dropped(name):
+    """What a wait was for is not there when it gives up: the kernel has to leave without using it."""
+    text = code_of(name)
+    calls = list(re.finditer(r"\bmbar_wait(?:_warp)?\(", text))
+    assert calls
+    for m in calls:
+        head = re.split(r"[;{}]", text[:m.start()])[-1].strip()
+        assert re.search(r"(=|&&|!|if \()\s*(tc::)?$", head), head
+
+
+def test_rows_that_never_came_end_the_fragment_kernel():
+    """The 8-bit fragment kernel: the block leaves as a whole between the wait for its rows and the first weight."""
+    text = code_of("qmm_mma8.cu")
+    wait = re.search(r"(\w+) = tc::mbar_wait\(s_rows_bar", text)
+    leave = re.search(rf"if \(!__syncthreads_and\({wait.group(1)}\)\) ", text)
+    assert leave and leave.start() > wait.start()
+    first, last = block_after(text, leave.end() - 1)
+    assert "cp_async_wait<0>()" in text[first:last] and "return;" in text[first:last]
+    assert last < text.index("for (int tl = 0; tl < tiles_here; ++tl)")
