@@ -653,8 +653,15 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
                 const float fac_next = load_rowfac(mt, c0 + parts * step);   // next chunk's
                 tmem_ld_wait();
                 if (split) {
-                    // The other shares in a fixed order, two of them in flight at once where the registers allow it (I8 M=16
-                    // K=11008 N=4096 in three parts 14.4 -> 13.5 us; FP8 in flight behind the arrival below 10.1 -> 9.4).
+                    // This CTA's share, then the others from the first on: the order decides the last bit of an f32 sum.  (Of
+                    // integers it does not, and every CTA begins with its neighbour.)  Several in flight at once, as far as the
+                    // registers go (I8 M=16 K=11008 N=4096 in three parts 14.4 -> 13.5 us; FP8 in flight behind the
+                    // arrival below 10.1 -> 9.4; six codebook pairs at 64 rows with two / three 154.2 / 153.1).
+                    constexpr int kFlight = T == 1 ? 3 : T == 2 ? 2 : 1;
+                    auto other = [&](int i) {   // i = 1 .. parts - 1
+                        if (KIND == KIND_I8) return part + i < parts ? part + i : part + i - parts;
+                        return i - 1 < part ? i - 1 : i;
+                    };
                     auto fetch = [&](int q, uint32_t (&x)[T][W]) {
                         const uint32_t src = mapa(s_dump + (size_t)c0 * kTileN + row, (uint32_t)q);
 #pragma unroll
@@ -670,26 +677,15 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
                                 r[t][j] = (KIND == KIND_I8) ? (uint32_t)((int)r[t][j] + (int)x[t][j])
                                                             : __float_as_uint(__uint_as_float(r[t][j]) + __uint_as_float(x[t][j]));
                     };
-                    if constexpr (T == 3) {   // (the registers of a second one cost more)
 #pragma unroll 1
-                        for (int q = part + 1 < parts ? part + 1 : 0; q != part; q = q + 1 < parts ? q + 1 : 0) {
-                            uint32_t x[T][W];
-                            fetch(q, x);
-                            add(x);
-                        }
-                    } else
-                    for (int i = 1; i < parts; i += 2) {
-                        uint32_t x[T][W], y[T][W];
-                        const int q0 = part + i < parts ? part + i : part + i - parts;
-                        const int q1 = q0 + 1 < parts ? q0 + 1 : 0;
-                        fetch(q0, x);
-                        if (i + 1 < parts) {
-                            fetch(q1, y);
-                            add(x);
-                            add(y);
-                        } else {
-                            add(x);
-                        }
+                    for (int i = 1; i < parts; i += kFlight) {
+                        uint32_t x[kFlight][T][W];
+#pragma unroll
+                        for (int f = 0; f < kFlight; ++f)
+                            if (i + f < parts) fetch(other(i + f), x[f]);
+#pragma unroll
+                        for (int f = 0; f < kFlight; ++f)
+                            if (i + f < parts) add(x[f]);
                     }
                     if (c0 + parts * step >= p.Mb) {   // this warp reads nothing more of the other CTAs
                         __syncwarp();
