@@ -163,48 +163,41 @@ act_prep_kernel(const float *act, int M, int K, int Kp, uint8_t *bq, float *dq, 
 // The same rewrite for rows of at most 32768 elements, read once: a thread holds HOLD units of eight consecutive elements
 // between the scan and the rewrite, with all loads in flight together, and every plane is written eight bytes at a
 // time.  (The loop above is a chain of two passes of 4-byte loads, about 8 us for K=11308.)
-// CLUSTER (I4 only): 32 rows to a row per SM, more than 4096 elements each.  The rewrite is then bound by latency, and a block
-// that holds up to 16 units a thread needs registers that the main kernel's 576 threads leave on no SM, so that the CTAs
-// which share an SM with one start when the rewrite is done.  The blocks of a cluster take an even part of a row
-// each and hand their maxima and sums round through distributed shared memory: two units a thread and 40 registers
-// whatever the length, which fit.  M=64 K=14336 N=4096 19.7 -> 18.4 us.  The main kernels of the other formats leave
-// room for the single block (I8, FP8, FP4: 320 threads) or for neither (codebook: 832); they lose the half microsecond that
-// the cluster's barriers take (FP8 M=32 K=11008 N=4096 16.6 / 17.5, FP4 M=4 K=8192 N=28672 29.4 / 30.1), and so do
-// more rows than SMs (M=4096 K=8192 N=1024 93.8 / 106) and few, whose blocks are on few SMs (I4 M=4 K=6000 N=4096 6.9 / 7.8,
-// three decoder layers at 16 rows 135.8 / 138.5).
-constexpr int kPrepCluster = 8;    // blocks of the longest rows
-constexpr int kPrepHold = 16;      // units a thread holds of the longest rows in one block
+// One block per row, whatever the format and the number of rows: the order in which a row is summed, and with it the last
+// bit of its outputs, does not depend on the batch.  A cluster that shares a row (4096 elements and 40 registers a thread to
+// a block, which find room beside the I4 kernel's 576 threads, and one block more that sums the row in this order) is
+// slower: us of a cluster / a block, I4 K=14336 N=4096 M=32 17.5 / 16.5, M=64 18.3 / 17.9, M=148 27.3 / 26.4; K=6000
+// N=4096 M=64 14.3 / 12.0; four decoder layers at 64 rows 300.2 / 298.2.
+constexpr int kPrepHold = 16;   // units of eight elements a thread can hold
+// HOLD: 2, 4, 8 or 16 units, the smallest that covers the row: fewer registers (more rows at once on an SM, and room
+// beside the main kernel before it) and less code to fetch, which a kernel of two microseconds notices.
 // VEC: rows of a multiple of four elements that start on 16 bytes (every layer of a real model); else 4-byte loads.
 // LEAN: 32 registers a thread instead of 40.  With a few rows the blocks then fit beside the fragment kernels' 512 threads of 112,
 // which leave 8192, and start before those end (I4 M=8 K=4096 N=6144 9.7 -> 8.2 us, N=22528 18.1 -> 15.4); from 33 rows on the
 // wider form is a little faster (four I4 decoder layers at 64 rows 302.0 lean, 299.1).
-template <int KIND, int T, bool PERM8, int HOLD, bool VEC, bool CLUSTER, bool LEAN>
+template <int KIND, int T, bool PERM8, int HOLD, bool VEC, bool LEAN>
 __global__ void __launch_bounds__(256, LEAN ? 8 : 1)
-act_prep_regs_kernel(const float *act, int M, int K, int Kp, int blocks, uint8_t *bq, float *dq, float *rowsum) {
-    __shared__ float2 s_part[8];                       // of this block's warps
-    __shared__ float2 s_all[kPrepCluster];             // of the row's blocks
-    if (CLUSTER) cluster_arrive();                     // (the others may be written to once they have started)
+act_prep_regs_kernel(const float *act, int M, int K, int Kp, uint8_t *bq, float *dq, float *rowsum) {
+    __shared__ float2 s_part[8];   // maximum and sum of the warps
     pdl_launch_dependents();
     pdl_wait();
-    const int tid = threadIdx.x;
-    const int m = CLUSTER ? blockIdx.x / blocks : blockIdx.x, part = CLUSTER ? blockIdx.x - m * blocks : 0;
+    const int m = blockIdx.x, tid = threadIdx.x;
     const float *row = act + (size_t)m * K;
     const float4 *row4 = reinterpret_cast<const float4 *>(row);
-    const int all_units = (K + 7) >> 3;   // the last one may be partly past the row: zeros there
-    const int u0 = CLUSTER ? all_units * part / blocks : 0, units = CLUSTER ? all_units * (part + 1) / blocks : all_units;
+    const int units = (K + 7) >> 3;   // the last one may be partly past the row: zeros there
     float v[HOLD][8];
 #pragma unroll
     for (int i = 0; i < HOLD; ++i) {
-        const int u = u0 + tid + i * 256;
+        const int u = tid + i * 256;
         if (VEC) {
             float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
-            if ((!CLUSTER || u < units) && 8 * u < K) a = ld_after_wait(row4 + 2 * u);
-            if ((!CLUSTER || u < units) && 8 * u + 4 < K) b = ld_after_wait(row4 + 2 * u + 1);
+            if (8 * u < K) a = ld_after_wait(row4 + 2 * u);
+            if (8 * u + 4 < K) b = ld_after_wait(row4 + 2 * u + 1);
             v[i][0] = a.x; v[i][1] = a.y; v[i][2] = a.z; v[i][3] = a.w;
             v[i][4] = b.x; v[i][5] = b.y; v[i][6] = b.z; v[i][7] = b.w;
         } else {
 #pragma unroll
-            for (int j = 0; j < 8; ++j) v[i][j] = (!CLUSTER || u < units) && 8 * u + j < K ? ld_after_wait(row + 8 * u + j) : 0.0f;
+            for (int j = 0; j < 8; ++j) v[i][j] = 8 * u + j < K ? ld_after_wait(row + 8 * u + j) : 0.0f;
         }
     }
     float mx = 0.0f, sum = 0.0f;
@@ -229,32 +222,19 @@ act_prep_regs_kernel(const float *act, int M, int K, int Kp, int blocks, uint8_t
         mx = fmaxf(mx, s_part[w].x);
         sum += s_part[w].y;
     }
-    if (CLUSTER) {
-        cluster_wait();
-        if (tid < blocks) st_cluster(mapa(&s_all[part], (uint32_t)tid), mx, sum);
-        __syncwarp();
-        cluster_sync();   // all parts are here, and nobody writes to a block that may have left
-        mx = 0.0f;
-        sum = 0.0f;
-        for (int q = 0; q < blocks; ++q) {
-            mx = fmaxf(mx, s_all[q].x);
-            sum += s_all[q].y;
-        }
-    }
-    const bool first = part == 0 && tid == 0;
     if (KIND == KIND_F16) {
         int ex = 15;
         if (mx > 0.0f && isfinite(mx)) (void)frexpf(mx, &ex);
         const int e = max(-120, min(120, 15 - ex));
         const float up = ldexpf(1.0f, e);
-        if (first) {
+        if (tid == 0) {
             dq[m] = ldexpf(1.0f, -e);
             rowsum[m] = sum;
         }
         uint4 *dst = reinterpret_cast<uint4 *>(bq + (size_t)m * Kp);   // Kp = 16 bytes per unit here
 #pragma unroll
         for (int i = 0; i < HOLD; ++i) {
-            const int u = u0 + tid + i * 256;
+            const int u = tid + i * 256;
             if (u >= units) continue;
             uint32_t h[4];
 #pragma unroll
@@ -269,18 +249,18 @@ act_prep_regs_kernel(const float *act, int M, int K, int Kp, int blocks, uint8_t
     const float full = (KIND == KIND_I8) ? 16256.0f : 448.0f;
     const float step = (mx > 0.0f && isfinite(mx)) ? mx / full : 1.0f;
     const float inv = 1.0f / step;
-    if (first) {
+    if (tid == 0) {
         dq[m] = step;
         rowsum[m] = sum;
-        if (Kp > 8 * all_units) {   // one more unit of zeros pads the row to 16 bytes
+        if (Kp > 8 * units) {   // one more unit of zeros pads the row to 16 bytes
 #pragma unroll
             for (int i = 0; i < T; ++i)
-                *reinterpret_cast<uint2 *>(bq + ((size_t)i * M + m) * Kp + 8 * all_units) = make_uint2(0u, 0u);
+                *reinterpret_cast<uint2 *>(bq + ((size_t)i * M + m) * Kp + 8 * units) = make_uint2(0u, 0u);
         }
     }
 #pragma unroll
     for (int i = 0; i < HOLD; ++i) {
-        const int u = u0 + tid + i * 256;
+        const int u = tid + i * 256;
         if (u >= units) continue;
         uint32_t w[T][2];
         float x[8];
@@ -860,11 +840,11 @@ namespace {
 
 template <int KIND, int T, bool PERM8, bool VEC>
 auto prep_kernel(int M, int K) {
-    return K <= 2 * 256 * 8   ? (M <= 32 ? act_prep_regs_kernel<KIND, T, PERM8, 2, VEC, false, true>
-                                         : act_prep_regs_kernel<KIND, T, PERM8, 2, VEC, false, false>)
-           : K <= 4 * 256 * 8 ? act_prep_regs_kernel<KIND, T, PERM8, 4, VEC, false, false>
-           : K <= 8 * 256 * 8 ? act_prep_regs_kernel<KIND, T, PERM8, 8, VEC, false, false>
-                              : act_prep_regs_kernel<KIND, T, PERM8, kPrepHold, VEC, false, false>;
+    return K <= 2 * 256 * 8   ? (M <= 32 ? act_prep_regs_kernel<KIND, T, PERM8, 2, VEC, true>
+                                         : act_prep_regs_kernel<KIND, T, PERM8, 2, VEC, false>)
+           : K <= 4 * 256 * 8 ? act_prep_regs_kernel<KIND, T, PERM8, 4, VEC, false>
+           : K <= 8 * 256 * 8 ? act_prep_regs_kernel<KIND, T, PERM8, 8, VEC, false>
+                              : act_prep_regs_kernel<KIND, T, PERM8, kPrepHold, VEC, false>;
 }
 
 template <int KIND, int T, bool PERM8>
@@ -873,32 +853,13 @@ int launch_prep(fnn_cuda_ctx *ctx, const QmmArgs &a, int Kp, uint8_t *bq, float 
     const bool vec = K % 4 == 0 && (reinterpret_cast<uintptr_t>(a.a) & 15) == 0;
     // same shared-memory carve-out as the main kernel: alternating carve-outs between consecutive
     // kernels makes every SM reconfigure (and drain) twice per call
-    auto carve_out = [](auto kern) {
-        return cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-    };
-    if (K > kPrepHold * 256 * 8) {
-        auto prep = act_prep_kernel<KIND, T, PERM8>;
-        FNN_CUDA_CHECK(carve_out(prep), FNN_ERR_DISPATCH);
-        FNN_CUDA_CHECK(launch_pdl(prep, M, 256, 0, ctx, a.a, M, K, Kp, bq, dq, rowsum), FNN_ERR_DISPATCH);
-        ctx->launches++;
-        return FNN_OK;
-    }
-    if constexpr (PERM8) {   // (I4)
-        if (K > 2 * 256 * 8 && M >= 32 && M <= ctx->sm_count) {
-            const int blocks = (K + 2 * 256 * 8 - 1) / (2 * 256 * 8);
-            static_assert(kPrepCluster * 2 >= kPrepHold, "a cluster covers the longest row");
-            auto prep = vec ? act_prep_regs_kernel<KIND, T, PERM8, 2, true, true, false>
-                            : act_prep_regs_kernel<KIND, T, PERM8, 2, false, true, false>;
-            FNN_CUDA_CHECK(carve_out(prep), FNN_ERR_DISPATCH);
-            FNN_CUDA_CHECK(launch_pdl_cluster(prep, M * blocks, blocks, 256, 0, ctx, a.a, M, K, Kp, blocks, bq, dq, rowsum),
-                           FNN_ERR_DISPATCH);
-            ctx->launches++;
-            return FNN_OK;
-        }
-    }
-    auto prep = vec ? prep_kernel<KIND, T, PERM8, true>(M, K) : prep_kernel<KIND, T, PERM8, false>(M, K);
-    FNN_CUDA_CHECK(carve_out(prep), FNN_ERR_DISPATCH);
-    FNN_CUDA_CHECK(launch_pdl(prep, M, 256, 0, ctx, a.a, M, K, Kp, 1, bq, dq, rowsum), FNN_ERR_DISPATCH);
+    auto prep = K > kPrepHold * 256 * 8 ? act_prep_kernel<KIND, T, PERM8>
+                : vec                   ? prep_kernel<KIND, T, PERM8, true>(M, K)
+                                        : prep_kernel<KIND, T, PERM8, false>(M, K);
+    FNN_CUDA_CHECK(cudaFuncSetAttribute(prep, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                        cudaSharedmemCarveoutMaxShared),
+                   FNN_ERR_DISPATCH);
+    FNN_CUDA_CHECK(launch_pdl(prep, M, 256, 0, ctx, a.a, M, K, Kp, bq, dq, rowsum), FNN_ERR_DISPATCH);
     ctx->launches++;
     return FNN_OK;
 }

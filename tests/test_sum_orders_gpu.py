@@ -28,3 +28,53 @@ def test_shares_of_a_cluster_meet_from_the_first_on(backend):
         assert (got == np.float32(2.0 ** 24)).all(), np.unique(got)
     finally:
         rig.close()
+
+
+def fold(partial):
+    """What the kernels make of the threads' sums: halves of a warp on one another down to one lane, then the warps in turn."""
+    lanes = partial.reshape(-1, 32)
+    for o in (16, 8, 4, 2, 1):
+        lanes = lanes + lanes[:, np.arange(32) ^ o]
+    total = np.float32(0.0)
+    for s in lanes[:, 0]:
+        total = np.float32(total + s)
+    return total
+
+
+def sum_of_units(row, threads):
+    """Thread t adds the elements of its units of eight (t, t + threads, ...) one after another."""
+    rounds = -(-len(row) // (8 * threads))
+    units = np.zeros((rounds, threads, 8), np.float32)
+    units.reshape(-1)[:len(row)] = row
+    s = np.zeros(threads, np.float32)
+    for i in range(rounds):
+        for j in range(8):
+            s = s + units[i, :, j]
+    return fold(s)
+
+
+def row_sums(backend, fmt, k, n, x, path, kernel):
+    """The row sums that a call used: codes of zero and zero points of one leave nothing else of the product."""
+    q = orc.QWeight(fmt, n, k, np.zeros(orc.packed_words(fmt, n, k), np.uint32), np.ones(n, np.float32),
+                    np.ones(n, np.float32))
+    rig = Rig(backend, q, len(x))
+    try:
+        got = rig.run(x, None, L.EPI_NONE, path)
+        assert backend.last_kernel().startswith(kernel), backend.last_kernel()
+        assert (got == got[:, :1]).all()
+        return got[:, 0]
+    finally:
+        rig.close()
+
+
+# whatever the number of rows, up to one per SM and more; every number of units that a thread holds; rows that start on 16
+# bytes and rows that do not
+@pytest.mark.parametrize("k", [4104, 6001, 14336, 20009, 28672, 28680, 32768])
+def test_row_sums_of_rewritten_rows(backend, k):
+    import torch
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    x = normal(930 + k, (sms + 1, k), 1.0)
+    want = np.array([sum_of_units(row, 256) for row in x])
+    for m in (31, 32, 64, sms, sms + 1):
+        got = row_sums(backend, orc.FMT_I4, k, 24, x[:m], L.PATH_TC, "tc")
+        assert (got == want[:m]).all(), (k, m)
