@@ -534,9 +534,9 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
         bool filled = true;
         for (int tile = first_tile; tile < total_tiles; tile += tile_step) {
             for (int kb = kb0; kb < kb1; ++kb) {
-                // (a lane that gives up stays with its warp through this step and the others, whatever the stages hold, and reports
-                // no stage any more: a vote, which ends the loop for all, cost 1 % of a decoder step)
-                filled = filled && mbar_wait(&rawfull[s], phase, s_abort, p.err_flag, 0x200);
+                // (A lane that gives up stays with its warp through this step and the others, whatever the stages hold, and reports
+                // no stage any more.  A vote, which ends the loop for all, cost 1 % of a decoder step, and so did a branch here.)
+                const bool here = mbar_wait(&rawfull[s], phase, s_abort, p.err_flag, 0x200);
                 tc_fence_after();   // the stage's columns were last read by MMAs another thread issued
                 const unsigned char *raw = s_raw + (size_t)s * raw_bytes + row * 64;
 #pragma unroll
@@ -556,6 +556,7 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
                 tmem_st_wait();
                 tc_fence_before();
                 __syncwarp();
+                filled &= here;
                 if (lane == 0 && filled) mbar_arrive(&full[s]);
                 if (++s == p.stages) {
                     s = 0;

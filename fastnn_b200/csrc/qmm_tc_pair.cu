@@ -295,9 +295,9 @@ qmm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         bool filled = true;
         for (int tile = pair; tile < total_tiles; tile += pairs) {
             for (int kb = 0; kb < p.kblocks; ++kb) {
-                // (a lane that gives up stays with its warp through this step and the others, whatever the stages hold, and reports
-                // no stage any more: a vote, which ends the loop for all, cost 1 % of a decoder step)
-                filled = filled && mbar_wait(&rawfull[s], phase, s_abort, p.err_flag, 0x200);
+                // (A lane that gives up stays with its warp through this step and the others, whatever the stages hold, and reports
+                // no stage any more.  A vote, which ends the loop for all, cost 1 % of a decoder step, and so did a branch here.)
+                const bool here = mbar_wait(&rawfull[s], phase, s_abort, p.err_flag, 0x200);
                 const unsigned char *raw = s_raw + (size_t)s * (kRawBytes + kScBytes);
                 unsigned char *dst = s_a + (size_t)s * a_bytes;
 #pragma unroll
@@ -319,6 +319,7 @@ qmm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                 }
                 fence_proxy_async();   // these stores are read by the tensor cores (async proxy)
                 __syncwarp();
+                filled &= here;
                 if (lane == 0 && filled) mbar_arrive_cluster(mapa(&full[s], 0));
                 if (++s == p.stages) {
                     s = 0;

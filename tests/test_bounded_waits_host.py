@@ -35,13 +35,17 @@ def test_waits_of_whole_warps_have_one_answer(name):
     inside = lambda at: any(a <= at <= b for a, b in elected)
     whole = [m.start() for m in re.finditer(r"\bmbar_wait_warp\(", text)]
     assert whole and not any(inside(at) for at in whole)
-    lone = [m for m in re.finditer(r"(?:(\w+) = \1 && )?\bmbar_wait\(", text) if not inside(m.start())]
+    lone = [m for m in re.finditer(r"(?:const bool (\w+) = )?\bmbar_wait\(", text) if not inside(m.start())]
     assert len(lone) == 1
-    answer = lone[0].group(1)   # once it is false it stays false
+    answer = lone[0].group(1)
     assert answer, text[lone[0].start():][:80]
-    uses = [u.strip() for u in re.findall(rf"[^;{{}}]*\b{answer}\b[^;]*;", text)]
-    assert len(uses) == 3 and uses[0] == f"bool {answer} = true;", uses
-    assert uses[2].startswith(f"if (lane == 0 && {answer}) mbar_arrive"), uses
+    def statements(word):
+        return [u.strip() for u in re.findall(rf"[^;{{}}]*\b{word}\b[^;]*;", text)]
+    kept = re.fullmatch(rf"(\w+) &= {answer};", statements(answer)[1])   # once it is false it stays false
+    assert kept and len(statements(answer)) == 2, statements(answer)
+    uses = statements(kept.group(1))
+    assert len(uses) == 3 and uses[0] == f"bool {kept.group(1)} = true;", uses
+    assert uses[2].startswith(f"if (lane == 0 && {kept.group(1)}) mbar_arrive"), uses
 
 
 @pytest.mark.parametrize("name", ["qmm_mma8.cu", "qmm_tc.cu", "qmm_tc_pair.cu"])
