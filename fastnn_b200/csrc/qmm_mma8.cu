@@ -241,6 +241,11 @@ qmm_mma8_kernel(P8 p) {
     const int Kpad = p.KB * KBLK;
     constexpr int kHeld = HELD;
     constexpr bool kCanHold = kHeld > 0;
+    // Long rows (more than 4096 elements of one group's, 8192 of two): a held group is two quads, one round of the block
+    // apart, as scan_rows walks a row, so that the sum of a row has the same last bit whether it is held or scanned.  us of
+    // groups of eight / of quads: I8 K=8192 N=2048 5.00 / 4.82, K=11008 N=4096 10.3 / 10.4; FP4 K=8192 N=2048 5.26 / 4.91; I4
+    // K=14336 N=2048 6.13 / 6.24, K=11008 N=4096 6.76 / 7.10 (scanned and read again: 7.5).
+    constexpr bool kQuads = kHeld >= 4 && !CB;   // (the codebook format takes no row sum, and block sums of its own)
     float hv[kCanHold ? kHeld : 1][8];
     bool held = false;
     __shared__ uint64_t s_rows_bar[1];   // PLANES: the rows of a pass have landed
@@ -314,15 +319,19 @@ qmm_mma8_kernel(P8 p) {
 #pragma unroll
                 for (int j = 0; j < kHeld; ++j) {
                     const int g8 = tid + j * NT;
+                    const int q0 = kQuads ? tid + 2 * j * NT : 2 * g8, q1 = kQuads ? q0 + NT : q0 + 1;   // its quads
                     if (vec_ok) {
                         float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
-                        if (g8 * 8 < p.K) a = ld_after_wait(reinterpret_cast<const float4 *>(p.act) + 2 * g8);
-                        if (g8 * 8 + 4 < p.K) b = ld_after_wait(reinterpret_cast<const float4 *>(p.act) + 2 * g8 + 1);
+                        if (q0 * 4 < p.K) a = ld_after_wait(reinterpret_cast<const float4 *>(p.act) + q0);
+                        if (q1 * 4 < p.K) b = ld_after_wait(reinterpret_cast<const float4 *>(p.act) + q1);
                         hv[j][0] = a.x; hv[j][1] = a.y; hv[j][2] = a.z; hv[j][3] = a.w;
                         hv[j][4] = b.x; hv[j][5] = b.y; hv[j][6] = b.z; hv[j][7] = b.w;
                     } else {
 #pragma unroll
-                        for (int q = 0; q < 8; ++q) hv[j][q] = g8 * 8 + q < p.K ? ld_after_wait(p.act + g8 * 8 + q) : 0.0f;
+                        for (int q = 0; q < 8; ++q) {
+                            const int k = (q < 4 ? q0 : q1) * 4 + (q & 3);
+                            hv[j][q] = k < p.K ? ld_after_wait(p.act + k) : 0.0f;
+                        }
                     }
                 }
 #pragma unroll
@@ -330,7 +339,8 @@ qmm_mma8_kernel(P8 p) {
 #pragma unroll
                     for (int q = 0; q < 8; ++q) {
                         mx = fmaxf(mx, fabsf(hv[j][q]));
-                        sum += hv[j][q];
+                        if (!kQuads) sum += hv[j][q];
+                        if (kQuads && (q & 3) == 3) sum += (hv[j][q - 3] + hv[j][q - 2]) + (hv[j][q - 1] + hv[j][q]);
                     }
 #pragma unroll
                 for (int o = 16; o > 0; o >>= 1) {
@@ -429,11 +439,35 @@ qmm_mma8_kernel(P8 p) {
 #pragma unroll
             for (int j = 0; j < kHeld; ++j) {
                 const int g8 = tid + j * NT;
-                if (g8 * 8 >= kc_len) continue;   // (beyond K the held values are zero: the padding of the last block)
                 float e[8];
 #pragma unroll
                 for (int q8 = 0; q8 < 8; ++q8) e[q8] = hv[j][q8] * inv;
                 uint32_t hi[2], lo[2];
+                if constexpr (kQuads) {
+                    int8_pairs<false>(e, hi, lo);   // a word of each plane per quad
+                    if constexpr (FMT == FNN_FMT_I4) {
+                        // I4 reorders inside a group of eight (inner_pos8).  The lanes of a pair hold the halves of two groups
+                        // and swap one each: the even lane stores the first round's group, the odd one the second's.
+                        const bool odd = lane & 1;
+                        const uint32_t h = __shfl_xor_sync(0xFFFFFFFFu, odd ? hi[0] : hi[1], 1);
+                        const uint32_t l = __shfl_xor_sync(0xFFFFFFFFu, odd ? lo[0] : lo[1], 1);
+                        const uint32_t h0 = odd ? h : hi[0], h1 = odd ? hi[1] : h, l0 = odd ? l : lo[0], l1 = odd ? lo[1] : l;
+                        const int k8 = ((tid + (2 * j + odd) * NT) >> 1) * 8;
+                        if (k8 >= kc_len) continue;
+                        *reinterpret_cast<uint2 *>(s_act + k8) = make_uint2(prmt(h0, h1, 0x6420), prmt(h0, h1, 0x7531));
+                        *reinterpret_cast<uint2 *>(s_act + (size_t)RS + k8) = make_uint2(prmt(l0, l1, 0x6420), prmt(l0, l1, 0x7531));
+                    } else {
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            const int k4 = (tid + (2 * j + h) * NT) * 4;
+                            if (k4 >= kc_len) continue;
+                            *reinterpret_cast<uint32_t *>(s_act + k4) = hi[h];
+                            *reinterpret_cast<uint32_t *>(s_act + (size_t)RS + k4) = lo[h];
+                        }
+                    }
+                    continue;
+                }
+                if (g8 * 8 >= kc_len) continue;   // (beyond K the held values are zero: the padding of the last block)
                 int8_pairs<FMT == FNN_FMT_I4>(e, hi, lo);   // (inner_pos8)
                 const int gp = group_pos8<FMT>(g8 * 8);
                 *reinterpret_cast<uint2 *>(s_act + gp) = make_uint2(hi[0], hi[1]);

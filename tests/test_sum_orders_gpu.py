@@ -78,3 +78,28 @@ def test_row_sums_of_rewritten_rows(backend, k):
     for m in (31, 32, 64, sms, sms + 1):
         got = row_sums(backend, orc.FMT_I4, k, 24, x[:m], L.PATH_TC, "tc")
         assert (got == want[:m]).all(), (k, m)
+
+
+def sum_of_quads(row, threads):
+    """Thread t adds the sums of its quads (t, t + threads, ...)."""
+    rounds = -(-len(row) // (4 * threads))
+    quads = np.zeros((rounds, threads, 4), np.float32)
+    quads.reshape(-1)[:len(row)] = row
+    s = np.zeros(threads, np.float32)
+    for i in range(rounds):
+        s = s + ((quads[i, :, 0] + quads[i, :, 1]) + (quads[i, :, 2] + quads[i, :, 3]))
+    return fold(s)
+
+
+# a single long row, held or scanned (from 16384 elements on): up to a tile of 16 channels per SM by one group of warps, with
+# two by two groups
+@pytest.mark.parametrize("fmt", [orc.FMT_I8, orc.FMT_I4, orc.FMT_F4])
+@pytest.mark.parametrize("k,tiles,threads", [(4104, 1, 256), (8192, 1, 256), (8196, 1, 256), (11008, 1, 256), (16384, 1, 256),
+                                             (16388, 1, 256), (8200, 2, 512), (11008, 2, 512), (12004, 2, 512), (16384, 2, 512),
+                                             (16388, 2, 512)])
+def test_row_sum_of_a_long_single_row(backend, fmt, k, tiles, threads):
+    import torch
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    x = normal(940 + k, (1, k), 1.0)
+    got = row_sums(backend, fmt, k, 16 * tiles * sms - 5, x, L.PATH_MMA, "mma8")
+    assert got[0] == sum_of_quads(x[0], threads), k
