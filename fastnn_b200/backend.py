@@ -269,7 +269,7 @@ class CudaBackend:
             following = next(todo, None)
             if (isinstance(instr, CallKernel) and instr.kernel_name in _QMATMUL_KERNELS
                     and isinstance(following, CallKernel) and following.kernel_name == "add_f32"):
-                residual = self._residual_of(instr, following, shape_env)
+                residual = self._residual_of(instr, following, arena, shape_env)
                 if residual is not None:
                     self._dispatch_qmatmul(instr, arena, shape_env, residual, following.output_slice)
                     instr = next(todo, None)
@@ -278,9 +278,10 @@ class CudaBackend:
             instr = following
 
     @staticmethod
-    def _residual_of(matmul: CallKernel, add: CallKernel, env: ShapeEnv) -> Optional[BufferSlice]:
+    def _residual_of(matmul: CallKernel, add: CallKernel, arena: CudaBuffer, env: ShapeEnv) -> Optional[BufferSlice]:
         """The other operand of an addition to the whole result of the MatMul before it, or None if it is anything
-        else (a broadcast, another slice, a symbolic size that differs): the two then run as they stand."""
+        else (a broadcast, another slice, a symbolic size that differs, no elements, an operand that the addition refuses because
+        its slice ends outside the arena): the two then run as they stand."""
         if len(add.input_slices) != 2 or len(matmul.input_slices) < 2:
             return None
         m, _, n = resolve_params(matmul.params, matmul.param_dims, env, 3)
@@ -293,8 +294,9 @@ class CudaBackend:
         x, y = add.input_slices
         if y.offset == matmul.output_slice.offset:
             x, y = y, x
-        if (x.offset != matmul.output_slice.offset or out_size != size
-                or min(x.size, y.size, add.output_slice.size) < size):
+        if (x.offset != matmul.output_slice.offset or size == 0 or out_size != size
+                or min(x.size, y.size, add.output_slice.size) < size
+                or max(s.offset + s.size // 4 * 4 for s in (x, y)) > arena.total_bytes):
             return None
         return y
 
