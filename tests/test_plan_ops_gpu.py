@@ -182,3 +182,29 @@ def test_elementwise_lengths(backend, op):
             assert (got[:n] == whole[:n]).all() and (got[n:] == 7).all(), n
     finally:
         arena.close()
+
+
+# f32 evaluation of the activations: the argument of the tanh carries four roundings of 2^-24, where its slope times itself is
+# at most 0.45, and tanhf and expf two units each, against a factor of |x| / 2 or |x|: below 5e-7 of max(1, |x|); twice that
+@pytest.mark.parametrize("op", [b | (a << 8) for b in (L.EW_ADD, L.EW_MUL, L.EW_SUB)
+                                for a in (L.EPI_NONE, L.EPI_RELU, L.EPI_GELU, L.EPI_SILU)] +
+                         [L.EW_RELU, L.EW_GELU, L.EW_SILU])
+def test_elementwise_results(backend, op):
+    """Every instantiation of the vector kernel against the function in 64 bits, behind the f32 rounding of the operation."""
+    n = 4104
+    x, y = normal(72, (n,), 1.0), normal(73, (n,), 1.0)
+    arena = backend.allocate_arena(3 * n * 4)
+    try:
+        backend.write_arena(arena, 0, np.concatenate([x, y, np.full(n, 7, np.float32)]).tobytes())
+        assert backend.lib.fnn_cuda_elementwise(backend.ctx, op, arena.handle, 0, n, 4 * n, n, 8 * n, n) == 0
+        got = np.frombuffer(backend.read_arena(arena, 8 * n, 4 * n), np.float32)
+    finally:
+        arena.close()
+    v = {L.EW_ADD: x + y, L.EW_MUL: x * y, L.EW_SUB: x - y}.get(op & 0xFF, x).astype(np.float64)
+    act = op >> 8 or {L.EW_RELU: L.EPI_RELU, L.EW_GELU: L.EPI_GELU, L.EW_SILU: L.EPI_SILU}.get(op, L.EPI_NONE)
+    want = {L.EPI_NONE: v, L.EPI_RELU: np.maximum(v, 0.0),
+            L.EPI_GELU: 0.5 * v * (1.0 + np.tanh(np.sqrt(2.0 / np.pi) * (v + 0.044715 * v ** 3))),
+            L.EPI_SILU: v / (1.0 + np.exp(-v))}[act]
+    assert np.max(np.abs(got - want) / np.maximum(1.0, np.abs(v))) <= 1e-6
+    if act in (L.EPI_NONE, L.EPI_RELU):
+        assert (got == want).all()

@@ -92,3 +92,64 @@ def test_plans_fuse_whole_residuals_only(backend):
         assert count == 2 and (got == y * r).all()
     finally:
         arena.close()
+
+
+# where the guards between the slices decide: one or two fragment rows, shared and whole tcgen05 tiles
+@pytest.mark.parametrize("m,k,n", [(1, 1024, 608), (4, 1024, 336), (20, 1280, 144), (64, 256, 19104)])
+def test_slices_that_may_not_be_written_by_one_epilogue(backend, m, k, n):
+    """One launch where the slices allow it; one more where the sum lies over something that the MatMul or the addition still
+    reads, or the residual over the result.  Both ways the bits are those of the two calls."""
+    q = orc.quantize_kn(orc.FMT_I8, normal(920 + k, (k, n), 0.02))
+    al = lambda x: -(-x // 64) * 64
+    size, payload = m * n, q.payload
+    a, out = 0, al(m * k)
+    add = out + al(size) + 64
+    total = add + al(size) + al(size) + 64
+    bias = total + al(size) + 64
+    weight = bias + al(size) + al(n)          # (a sum that begins over the bias ends ahead of the rows)
+    end = weight + max(len(payload) // 4, size + 64) + 64
+    arena = backend.allocate_arena(4 * end)
+    first = np.zeros(end, np.float32)
+    first[a:a + m * k], first[add:add + size] = normal(921, (m * k,), 1.0), normal(922, (size,), 1.0)
+    first[bias:bias + n] = normal(923, (n,), 0.1)
+    raw = bytearray(first.tobytes())
+    raw[4 * weight:4 * weight + len(payload)] = payload
+    raw = bytes(raw)
+    backend.write_arena(arena, 0, raw)
+    w = backend.upload_qweight(b"", meta_of(q), arena, 4 * weight, len(payload))   # (its rows stay where they are)
+    try:
+        def run(fused, add_at, sum_at):
+            backend.write_arena(arena, 0, raw)
+            before = backend.launch_count()
+            args = (backend.ctx, w.handle, arena.handle, 4 * a, 4 * out, 4 * bias, m, L.EPI_SILU, L.PATH_AUTO)
+            if fused:
+                assert backend.lib.fnn_cuda_qmatmul_add(*args, 4 * add_at, 4 * sum_at) == 0, L.last_error()
+            else:
+                assert backend.lib.fnn_cuda_qmatmul(*args) == 0, L.last_error()
+                assert backend.lib.fnn_cuda_elementwise(backend.ctx, L.EW_ADD, arena.handle, 4 * out, size, 4 * add_at, size,
+                                                        4 * sum_at, size) == 0
+            launches = backend.launch_count() - before
+            return launches, np.frombuffer(backend.read_arena(arena, 0, 4 * end), np.uint32).copy()
+
+        run(True, add, total)                      # first use: layouts, scratch
+        two = run(False, add, total)[0]
+        for add_at, sum_at, apart in [(add, total, False), (add, add, False),
+                                      (out, total, True), (out + 4, total, True),   # the residual over the result
+                                      (add, out, True),                             # the sum over the result
+                                      (add, bias, True), (add, bias + n - 4, True),
+                                      (add, weight, True), (add, weight + 8, True)] + (
+                                      [(add, a + 4, True)] if size + 4 <= out else []):
+            count, got = run(True, add_at, sum_at)
+            assert count == two - (not apart), (add_at, sum_at)
+            assert (got == run(False, add_at, sum_at)[1]).all(), (add_at, sum_at)
+        # half over the residual, ahead of it and behind it, and half over the result: an addition whose operand is overwritten
+        # as it runs, so what it makes of the overlap is open, but not what lies beside the two slices
+        for over, sum_at in ((add, add + 4), (add, add + size // 8 * 4), (add, add - 4), (out, out + 4)):
+            count, got = run(True, add, sum_at)
+            assert count == two, sum_at
+            plain = run(False, add, sum_at)[1]
+            lo, hi = min(over, sum_at), max(over, sum_at) + size
+            assert (got[:lo] == plain[:lo]).all() and (got[hi:] == plain[hi:]).all(), sum_at
+    finally:
+        w.close()
+        arena.close()

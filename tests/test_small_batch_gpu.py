@@ -12,7 +12,9 @@ import oracle as orc
 import fastnn_b200 as fnn
 from fastnn_b200 import _lib as L
 from helpers import max_err_vs_rms, normal
+from test_kernel_choice_gpu import columns
 from test_qmatmul_gpu import TOL_F32, Rig
+from test_tcgen05_tiles_gpu import random_codes
 
 pytestmark = pytest.mark.gpu
 
@@ -130,3 +132,22 @@ def test_own_stream_captured_without_scratch(fmt, k, n, m):
         del graph
         rig.close()
         fresh.close()
+
+
+# one FP8 row of at least eight tiles of 16 channels per SM and a ragged last one: two small blocks per SM up to 8192 elements,
+# one larger one beyond
+@pytest.mark.parametrize("k", [4104, 8192, 8200])
+def test_single_fp8_row_in_front_of_many_tiles(backend, k):
+    import torch
+    n = 8 * 16 * torch.cuda.get_device_properties(0).multi_processor_count + 5
+    q = random_codes(orc.FMT_F8, k, n, 860 + k)
+    x, bias = normal(861, (1, k), 1.0), normal(862, (n,), 0.01)
+    rig = Rig(backend, q, 1)
+    try:
+        got = rig.run(x, bias, L.EPI_NONE, L.PATH_MMA)
+        assert backend.last_kernel() == "mma"
+        for lo, hi in ((0, 130), (n - 150, n)):
+            err = max_err_vs_rms(got[:, lo:hi], orc.qmatmul(columns(q, lo, hi), x, bias[lo:hi], L.EPI_NONE))
+            assert err <= TOL_F32, (k, lo, err)
+    finally:
+        rig.close()
