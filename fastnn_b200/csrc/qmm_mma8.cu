@@ -802,24 +802,37 @@ int launch8(fnn_cuda_ctx *ctx, const QmmArgs &a) {
 // shared with the blocks of the next kernel on the stream, which prefetch their weights as soon as one fits, so smaller
 // blocks win where there are enough of them; every block stages the row, so a long one wants few of them; and up to one
 // tile per SM two blocks on an SM would leave another idle.  us, one group x 1 / x 2 / x 3 blocks per SM, two
-// groups x 1 (three groups x 1 are never the fastest):
+// groups x 1:
 //   up to a tile per SM        I8 K=8192 N=2048 6.18 / 6.72 / 8.35 / 6.57;  FP4 K=8192 N=2048 5.64 / 7.05 / 8.45 / 6.79;
 //                              codebook K=8192 N=2048 7.47 / 11.2 / - / 10.4
 //   K up to 4096               I4 K=4096 N=4096 - / 4.61 / 5.13 / 4.98;  FP4 K=4096 N=11008 - / 7.80 / 9.84 / 8.41;
 //                              I8 K=2048 N=8192 - / 5.05 / 5.65 / 5.70;  codebook K=2048 N=8192 7.77 / 6.60 / - / 7.56
 //   and I8 of four tiles a SM  K=4096 N=11008 11.1 / 10.0 / 9.84 / 9.88, N=14336 13.4 / 11.9 / 11.6 / 12.3
 //   longer                     I8 K=11008 N=4096 - / 11.1 / 15.8 / 10.7, K=8192 N=28672 - / 37.7 / 41.1 / 37.5; I4 K=14336 N=4096
-//                              - / 9.20 / 16.0 / 8.62; codebook, whose tables cost a second group its registers,
-//                              K=11008 N=4096 15.2 / 17.4 / - / 15.8
+//                              - / 9.20 / 16.0 / 8.62
+//   a little over a tile a SM  FP4 K=4096 N=2560 4.74 / 5.20, N=3584 4.91 / 4.89;  codebook K=4096 N=2560 6.6 / 7.2, N=3072 6.8 /
+//                              7.1, K=2048 N=2560 4.65 / 4.77, N=3072 4.76 / 4.61
+//   codebook, two to three     K=2048 N=5632 - / 6.5 / - / 5.9;  K=4096 N=6144 - / 9.5 / - / 8.7
+//   and by length              K=8192 N=4096 10.8 / - / - / 10.5, N=8192 17.9 / - / - / 17.3, N=28672 48.7 / - / - / 46.9;  K=11008
+//                              N=4096 15.0 / 17.4 / - / 15.3;  K=20000 N=4096 (not held) 28.0 / - / - / 25.3
 template <int FMT>
 int launch8_single(fnn_cuda_ctx *ctx, const QmmArgs &a, int ntiles) {
-    const int units = (int)div_ceil(a.w->K, 8);
-    if (ntiles > ctx->sm_count) {
-        if constexpr (FMT == FNN_FMT_I8)
-            if (units <= 512 && ntiles >= 4 * ctx->sm_count) return launch8<FMT, 1, 1, false, 3, 2>(ctx, a);
-        if (units <= 512) return launch8<FMT, 1, 1, false, 2, 2>(ctx, a);
-        if constexpr (!T8<FMT>::codebook)
+    const int units = (int)div_ceil(a.w->K, 8), sms = ctx->sm_count;
+    bool one = ntiles <= sms;   // a block of one group on an SM
+    if (FMT == FNN_FMT_F4 && units > 256 && units <= 512) one = 4 * ntiles < 5 * sms;
+    if (T8<FMT>::codebook && units <= 512) one = 4 * ntiles < (units > 256 ? 6 : 5) * sms;
+    if (!one) {
+        if constexpr (T8<FMT>::codebook) {
+            if (units <= 512 ? ntiles > 2 * sms && ntiles <= 3 * sms : units <= 1024)
+                return launch8<FMT, 1, 2, false, 1, 2>(ctx, a);
+            if (units <= 512) return launch8<FMT, 1, 1, false, 2, 2>(ctx, a);
+            if (units > 2048) return launch8<FMT, 1, 2, false>(ctx, a);
+        } else {
+            if constexpr (FMT == FNN_FMT_I8)
+                if (units <= 512 && ntiles >= 4 * sms) return launch8<FMT, 1, 1, false, 3, 2>(ctx, a);
+            if (units <= 512) return launch8<FMT, 1, 1, false, 2, 2>(ctx, a);
             return units <= 1024 ? launch8<FMT, 1, 2, false, 1, 2>(ctx, a) : launch8<FMT, 1, 2, false, 1, 4>(ctx, a);
+        }
     }
     return units <= 512    ? launch8<FMT, 1, 1, false, 1, 2>(ctx, a)
            : units <= 1024 ? launch8<FMT, 1, 1, false, 1, 4>(ctx, a)

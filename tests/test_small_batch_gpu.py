@@ -12,7 +12,7 @@ import oracle as orc
 import fastnn_b200 as fnn
 from fastnn_b200 import _lib as L
 from helpers import max_err_vs_rms, normal
-from test_kernel_choice_gpu import columns
+from test_kernel_choice_gpu import codes, columns
 from test_qmatmul_gpu import TOL_F32, Rig
 from test_tcgen05_tiles_gpu import random_codes
 
@@ -149,5 +149,27 @@ def test_single_fp8_row_in_front_of_many_tiles(backend, k):
         for lo, hi in ((0, 130), (n - 150, n)):
             err = max_err_vs_rms(got[:, lo:hi], orc.qmatmul(columns(q, lo, hi), x, bias[lo:hi], L.EPI_NONE))
             assert err <= TOL_F32, (k, lo, err)
+    finally:
+        rig.close()
+
+
+# launch shapes by tiles of 16 channels per SM and length: the codebook's single row on both sides of its lines, FP4 a little over
+# a tile per SM
+@pytest.mark.parametrize("fmt,m,k,tiles", [
+    (orc.FMT_I4CB, 1, 2048, 1.1), (orc.FMT_I4CB, 1, 4096, 1.45), (orc.FMT_I4CB, 1, 2080, 2.4), (orc.FMT_I4CB, 1, 4128, 1.7),
+    (orc.FMT_I4CB, 1, 8320, 1.2), (orc.FMT_I4CB, 1, 16416, 1.2), (orc.FMT_F4, 1, 4090, 1.1), (orc.FMT_F4, 1, 2056, 1.3)])
+def test_launch_shapes(backend, fmt, m, k, tiles):
+    import torch
+    n = int(tiles * torch.cuda.get_device_properties(0).multi_processor_count) * 16 - 5
+    q = codes(fmt, k, n, 870 + k)
+    x, bias = normal(871 + m, (m, k), 1.0), normal(872, (n,), 0.01)
+    rig = Rig(backend, q, m)
+    try:
+        got = rig.run(x, bias, L.EPI_NONE, L.PATH_MMA)
+        backend.synchronize()
+        assert backend.last_path() == "mma8"
+        for lo, hi in ((0, 130), (n - 150, n)):
+            err = max_err_vs_rms(got[:, lo:hi], orc.qmatmul(columns(q, lo, hi), x, bias[lo:hi], L.EPI_NONE))
+            assert err <= TOL_F32, (lo, err)
     finally:
         rig.close()
