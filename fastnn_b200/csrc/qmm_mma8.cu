@@ -162,14 +162,15 @@ struct P8 {
 
 // MULTI: more than one batch row (all rows scanned and staged together); the single-row instantiation
 // keeps the shortest prologue.  CG 8-column groups hold the (term, batch row) columns: up to 4 * CG rows.
-// PLANES: the rows arrive rewritten (p.planes); its own instantiation, since the branch and the longer code cost the
-// smallest calls 2 %.
+// PLANES: the rows arrive rewritten (p.planes), by bulk copies (kBulk) or by all threads (kThreads, see launch8); instantiations of
+// their own, since the branch and the longer code cost the smallest calls 2 %.
 // HELD: groups of eight activations a thread keeps of a single row between the scan and the rewrite, so that the row is read
 // once (0: never).  A row that is scanned and then read again behind two more block barriers costs 0.8 us (I8 K=11008 N=4096
 // 11.5 -> 10.7 us) to 2 us (I4 K=8192 N=2048 7.8 -> 5.6, one warp of byte stores per plane before).  As few groups as cover
 // the row: the prologue is straight-line code that every block runs once, and the instructions of groups
 // that are not there cost time too (I8 K=1024 N=2048 2.70 with 2, 3.46 with 8).
-template <int FMT, int CG, int kG8, bool MULTI, bool PLANES, int BPS, int HELD>
+enum Planes { kNoPlanes, kBulk, kThreads };
+template <int FMT, int CG, int kG8, bool MULTI, int PLANES, int BPS, int HELD>
 __global__ void __launch_bounds__(kG8 * kW8 * 32, BPS)
 qmm_mma8_kernel(P8 p) {
     using TT = T8<FMT>;
@@ -248,9 +249,9 @@ qmm_mma8_kernel(P8 p) {
     constexpr bool kQuads = kHeld >= 4 && !CB;   // (the codebook format takes no row sum, and block sums of its own)
     float hv[kCanHold ? kHeld : 1][8];
     bool held = false;
-    __shared__ uint64_t s_rows_bar[1];   // PLANES: the rows of a pass have landed
+    __shared__ uint64_t s_rows_bar[1];   // kBulk: the rows of a pass have landed
     __shared__ volatile int s_abort[1];
-    if (PLANES && tid == 0) {
+    if (PLANES == kBulk && tid == 0) {
         tc::mbar_init(s_rows_bar, 1);
         *s_abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -366,7 +367,16 @@ qmm_mma8_kernel(P8 p) {
         __syncthreads();  // previous pass fully consumed
         bool landed = true;
         // ---- stage the activation bytes of [k0, k0 + kc_len) --------------------------------
-        if (PLANES) {
+        if (PLANES == kThreads) {
+            const int pieces = kc_len / 16;   // of sixteen bytes
+            for (int i = tid; i < cols * pieces; i += NT) {
+                const int r = i / pieces, k = (i - r * pieces) * 16;   // plane-major rows, as staged
+                const bool in = k0 + k < p.Kp;
+                frag::cp_async16(s_act + (size_t)r * RS + k, p.planes + (in ? (size_t)r * p.Kp + k0 + k : 0), in ? 16 : 0);
+            }
+            cp_async_commit();
+            cp_async_wait<0>();
+        } else if (PLANES) {
             // One bulk copy per rewritten row (plane-major, as staged), issued by the lanes of a warp.  Sixteen bytes at a
             // time through all threads the copies and their index arithmetic took 1.7 us, and waiting for them drained the
             // weights' ring too (I4 M=8 K=4096 N=4096 7.75 -> 6.45 us).  What the last k-block has beyond the planes is cleared.
@@ -525,7 +535,7 @@ qmm_mma8_kernel(P8 p) {
                 for (int k = tid; k < kc_len; k += NT) put(k, (k0 + k < p.K) ? ld_after_wait(row + k0 + k) : 0.0f);
             }
         }
-        if (!PLANES) {
+        if (PLANES != kBulk) {
             __syncthreads();
         } else if (!__syncthreads_and(landed)) {
             // The rows have not come: nothing is stored, the residual's slice least of all.  Copies already in flight land
@@ -786,9 +796,15 @@ int launch8(fnn_cuda_ctx *ctx, const QmmArgs &a) {
                 "qmatmul: shared memory budget exceeded for M=%d on the 8-bit fragment kernel", p.M);
     p.tiles_per_group = sz.tiles_per_group;
     p.Kc = sz.Kc;
-    auto kern = qmm_mma8_kernel<FMT, CG, kG8, MULTI, false, BPS, HELD>;
+    auto kern = qmm_mma8_kernel<FMT, CG, kG8, MULTI, kNoPlanes, BPS, HELD>;
     if constexpr (MULTI && !TT::codebook)
-        if (p.planes) kern = qmm_mma8_kernel<FMT, CG, kG8, MULTI, true, BPS, HELD>;
+        if (p.planes) kern = qmm_mma8_kernel<FMT, CG, kG8, MULTI, kBulk, BPS, HELD>;
+    // Long I8 rows in front of more than a tile per SM: the weights are twice as many bytes, and behind bulk copies they start
+    // late.  us by bulk copies / by all threads: M=2 K=11008 N=4096 13.6 / 13.1, M=4 K=8192 N=4096 10.9 / 10.2, N=11008 21.1 /
+    // 19.4, M=3 K=8192 N=28672 46.3 / 40.2; but M=4 K=8192 N=2048 7.4 / 8.1, K=5000 N=4096 7.5 / 8.3, K=4104 N=11008 12.6 / 13.0,
+    // and of the 4-bit formats I4 M=4 K=11008 N=4096 9.4 / 10.8, M=8 K=4096 N=11008 10.2 / 10.5, FP4 M=4 K=11008 N=2048 8.8 / 10.6.
+    if constexpr (MULTI && FMT == FNN_FMT_I8)
+        if (p.planes && p.K >= 8192 && p.ntiles > ctx->sm_count) kern = qmm_mma8_kernel<FMT, CG, kG8, MULTI, kThreads, BPS, HELD>;
     FNN_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sz.smem),
                    FNN_ERR_DISPATCH);
     FNN_CUDA_CHECK(launch_pdl(kern, sz.grid, kG8 * kW8 * 32, sz.smem, ctx, p), FNN_ERR_DISPATCH);
