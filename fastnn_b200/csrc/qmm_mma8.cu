@@ -732,6 +732,11 @@ qmm_mma8_kernel(P8 p) {
     if (p.gather_on) gather_finish(p.g, step, p.M, p.N);
 }
 
+bool rewritten_once(const QmmArgs &a) {
+    const size_t elems = a.M * a.w->K;
+    return elems > 16384 || (a.M > 4 && elems >= 8192);
+}
+
 template <int FMT, int CG, int kG8, bool MULTI, int BPS = 1, int HELD = 0>
 int launch8(fnn_cuda_ctx *ctx, const QmmArgs &a) {
     using TT = T8<FMT>;
@@ -756,11 +761,10 @@ int launch8(fnn_cuda_ctx *ctx, const QmmArgs &a) {
     p.gather_on = a.gather != nullptr;
     if (a.gather) p.g = *a.gather;
     // Several rows: every block scans and rewrites all of them, which costs more than a kernel that does it once
-    // as soon as there is enough to rewrite.  us in the blocks / once: I4 K=4096 N=4096 M=2 6.3 / 6.3, M=4 7.3 / 6.7,
+    // as soon as there is enough to rewrite (rewritten_once).  us in the blocks / once: I4 K=4096 N=4096 M=2 6.3 / 6.3, M=4 7.3 / 6.7,
     // M=8 10.4 / 7.6; I8 K=11008 N=4096 M=2 13.6 / 12.8, M=4 16.3 / 13.5; I8 K=1024 N=2048 M=4 4.1 / 4.6, M=8 5.7 / 5.0;
     // I4 K=4096 N=28672 M=4 15.3 / 15.8.  (The codebook format stages groups of eight bytes: slower this way.)
-    const size_t elems = a.M * w->K;
-    if (MULTI && !TT::codebook && !a.gather && (elems > 16384 || (a.M > 4 && elems >= 8192))) {
+    if (MULTI && !TT::codebook && !a.gather && rewritten_once(a)) {
         const tc::PrepLayout lay = tc::prep_layout(2, 1, a.M, w->K);
         // (a capture that finds the scratch buffer too small keeps to the blocks)
         if (ctx->scratch_bytes >= lay.bytes || !stream_capturing(ctx)) {
@@ -856,12 +860,21 @@ int launch8_single(fnn_cuda_ctx *ctx, const QmmArgs &a, int ntiles) {
 }
 
 // Several batch rows: two groups per block while that still gives (nearly) every SM a block, else one, so that the tiles
-// spread over more SMs.  (us with three / two groups: I8 M=4 K=4096 N=11008 12.5 / 12.0, K=2048 N=8192 8.05 / 7.17.)
+// spread over more SMs.  (us with three / two groups: I8 M=4 K=4096 N=11008 12.4 / 12.3, K=2048 N=8192 6.8 / 6.5; I4 M=4 K=4096
+// N=11008 9.0 / 8.5, K=8192 N=28672 29.8 / 26.4.)  Three where the block itself scans two or three rows of more than 4096 elements,
+// which more threads do faster, and no round of tiles is added: M=2 K=5000 N=13001 I8 14.3 / 14.8, I4 10.4 / 10.8, FP4 13.3 / 13.6;
+// M=2 K=8192 N=28672 I8 40.8 / 41.4, I4 24.1 / 24.4; M=3 K=5000 N=13001 I8 15.3 / 15.7, I4 10.8 / 11.6, but FP4 14.7 / 14.2.  With
+// as many rounds either way two win again: I8 M=2 K=8192 N=8192 16.7 / 16.2.
 template <int FMT, int CG>
 int launch8_cg(fnn_cuda_ctx *ctx, const QmmArgs &a) {
     const int ntiles = (int)div_ceil(a.w->N, 16);
     if constexpr (CG == 1)
         if (a.M == 1) return launch8_single<FMT>(ctx, a, ntiles);
+    if constexpr (CG == 1 && !T8<FMT>::codebook) {
+        auto rounds = [&](int groups) { return div_ceil((size_t)ntiles, (size_t)groups * ctx->sm_count); };
+        if (a.w->K > 4096 && !rewritten_once(a) && (FMT != FNN_FMT_F4 || a.M == 2) && rounds(3) < rounds(2))
+            return launch8<FMT, 1, 3, true>(ctx, a);
+    }
     if ((ntiles + 1) / 2 >= ctx->sm_count * 4 / 5) return launch8<FMT, CG, 2, true>(ctx, a);
     return launch8<FMT, CG, 1, true>(ctx, a);
 }

@@ -154,12 +154,12 @@ def test_single_fp8_row_in_front_of_many_tiles(backend, k):
 
 
 # launch shapes by tiles of 16 channels per SM and length: the codebook's single row on both sides of its lines, FP4 a little over
-# a tile per SM; several I8 rows brought by all threads
+# a tile per SM; several I8 rows brought by all threads; two and three rows scanned by three groups of warps
 @pytest.mark.parametrize("fmt,m,k,tiles", [
     (orc.FMT_I4CB, 1, 2048, 1.1), (orc.FMT_I4CB, 1, 4096, 1.45), (orc.FMT_I4CB, 1, 2080, 2.4), (orc.FMT_I4CB, 1, 4128, 1.7),
     (orc.FMT_I4CB, 1, 8320, 1.2), (orc.FMT_I4CB, 1, 16416, 1.2), (orc.FMT_F4, 1, 4090, 1.1), (orc.FMT_F4, 1, 2056, 1.3),
     (orc.FMT_I8, 2, 8195, 1.2), (orc.FMT_I8, 4, 8208, 1.2), (orc.FMT_I8, 8, 8192, 1.9), (orc.FMT_I8, 13, 8200, 1.1),
-    (orc.FMT_I8, 4, 40000, 1.1)])
+    (orc.FMT_I8, 4, 40000, 1.1), (orc.FMT_I8, 2, 4104, 5.4), (orc.FMT_I4, 3, 5001, 5.4), (orc.FMT_F4, 2, 4104, 5.4)])
 def test_launch_shapes(backend, fmt, m, k, tiles):
     import torch
     n = int(tiles * torch.cuda.get_device_properties(0).multi_processor_count) * 16 - 5
