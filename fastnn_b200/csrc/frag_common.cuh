@@ -102,6 +102,62 @@ __device__ __forceinline__ void scan_rows(const float *act, int M, int K, bool v
     __syncthreads();
 }
 
+// A single batch row that is staged in one pass: every thread keeps HELD groups of eight activations in registers between
+// the scan and the rewrite, so the row is read once.  Thread t holds the groups t, t + NT, ... or, with QUADS, the quads
+// t, t + NT, ..., two to a group, as scan_rows walks a row (zeros beyond the row).  Each warp leaves its maximum and sum in s_part;
+// behind a block barrier every thread folds them itself, in a fixed order (fold_held): one barrier and a broadcast less than
+// handing the result round.
+template <int NT, int HELD, bool QUADS>
+__device__ __forceinline__ void hold_row(const float *act, int K, bool vec_ok, float (&hv)[HELD][8], float *s_part) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    float mx = 0.0f, sum = 0.0f;
+#pragma unroll
+    for (int j = 0; j < HELD; ++j) {
+        const int g8 = tid + j * NT;
+        const int q0 = QUADS ? tid + 2 * j * NT : 2 * g8, q1 = QUADS ? q0 + NT : q0 + 1;   // its quads
+        if (vec_ok) {
+            float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
+            if (q0 * 4 < K) a = ld_after_wait(reinterpret_cast<const float4 *>(act) + q0);
+            if (q1 * 4 < K) b = ld_after_wait(reinterpret_cast<const float4 *>(act) + q1);
+            hv[j][0] = a.x; hv[j][1] = a.y; hv[j][2] = a.z; hv[j][3] = a.w;
+            hv[j][4] = b.x; hv[j][5] = b.y; hv[j][6] = b.z; hv[j][7] = b.w;
+        } else {
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                const int k = (q < 4 ? q0 : q1) * 4 + (q & 3);
+                hv[j][q] = k < K ? ld_after_wait(act + k) : 0.0f;
+            }
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < HELD; ++j)
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            mx = fmaxf(mx, fabsf(hv[j][q]));
+            if (!QUADS) sum += hv[j][q];
+            if (QUADS && (q & 3) == 3) sum += (hv[j][q - 3] + hv[j][q - 2]) + (hv[j][q - 1] + hv[j][q]);
+        }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, o));
+        sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
+    }
+    if (lane == 0) {
+        s_part[warp * 2] = mx;
+        s_part[warp * 2 + 1] = sum;
+    }
+}
+template <int NT>
+__device__ __forceinline__ void fold_held(const float *s_part, float &mx, float &sum) {
+    mx = 0.0f;
+    sum = 0.0f;
+#pragma unroll
+    for (int w = 0; w < NT / 32; ++w) {
+        mx = fmaxf(mx, s_part[w * 2]);
+        sum += s_part[w * 2 + 1];
+    }
+}
+
 // The bias of a group's rows (tiles gg, gg + GG, ...), into the third word of their entries in `meta`.  A bias can be
 // an input that the kernel before this one writes, so it is read behind pdl_wait(), unlike the scales and
 // zero points of the weight, and not through the non-coherent path.  Asynchronous copies, issued behind the

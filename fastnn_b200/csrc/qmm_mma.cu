@@ -284,37 +284,7 @@ qmm_mma_kernel(MmaParams p) {
             // [2^14, 2^15): exact, inside the fp16 range whatever the magnitude of the activations
             if (HELD > 0 && p.K <= NT * 8 * HELD && kc_len >= Kpad) {
                 held = true;
-                float mx = 0.0f, sum = 0.0f;
-#pragma unroll
-                for (int j = 0; j < HELD; ++j) {
-                    const int g8 = tid + j * NT;
-                    if (vec_ok) {
-                        float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
-                        if (g8 * 8 < p.K) a = ld_after_wait(reinterpret_cast<const float4 *>(p.act) + 2 * g8);
-                        if (g8 * 8 + 4 < p.K) b = ld_after_wait(reinterpret_cast<const float4 *>(p.act) + 2 * g8 + 1);
-                        hv[j][0] = a.x; hv[j][1] = a.y; hv[j][2] = a.z; hv[j][3] = a.w;
-                        hv[j][4] = b.x; hv[j][5] = b.y; hv[j][6] = b.z; hv[j][7] = b.w;
-                    } else {
-#pragma unroll
-                        for (int q = 0; q < 8; ++q) hv[j][q] = g8 * 8 + q < p.K ? ld_after_wait(p.act + g8 * 8 + q) : 0.0f;
-                    }
-                }
-#pragma unroll
-                for (int j = 0; j < HELD; ++j)
-#pragma unroll
-                    for (int q = 0; q < 8; ++q) {
-                        mx = fmaxf(mx, fabsf(hv[j][q]));
-                        sum += hv[j][q];
-                    }
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) {
-                    mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, o));
-                    sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
-                }
-                if (lane == 0) {
-                    s_part[warp * 2] = mx;
-                    s_part[warp * 2 + 1] = sum;
-                }
+                if constexpr (HELD > 0) frag::hold_row<NT, HELD, false>(p.act, p.K, vec_ok, hv, s_part);
             } else {
                 frag::scan_rows<NT, (HELD > 0 ? 1 : 4)>(p.act, p.M, p.K, vec_ok, s_part, s_mx, s_rs);
             }
@@ -333,13 +303,8 @@ qmm_mma_kernel(MmaParams p) {
         // per lane, one 16-byte store per plane (an 8-group is contiguous in the staged order of every
         // format).  Two items are in flight per warp.
         if (HELD > 0 && held) {
-            // every thread folds the warps' partials itself, in the same fixed order
-            float bm = 0.0f, bs = 0.0f;
-#pragma unroll
-            for (int w = 0; w < NW; ++w) {
-                bm = fmaxf(bm, s_part[w * 2]);
-                bs += s_part[w * 2 + 1];
-            }
+            float bm, bs;
+            frag::fold_held<NT>(s_part, bm, bs);
             int ex = 15;
             if (bm > 0.0f && isfinite(bm)) (void)frexpf(bm, &ex);
             const int e = max(-120, min(120, 15 - ex));

@@ -312,46 +312,8 @@ qmm_mma8_kernel(P8 p) {
                     s_rs[tid] = __ldcg(p.rowsum + tid);
                 }
             } else if (kCanHold && p.K <= NT * 8 * kHeld && kc_len >= Kpad) {
-                // A single batch row that is staged in one pass: every thread keeps its groups of eight
-                // consecutive activations in registers between the scan and the rewrite, so the row is
-                // read once.
                 held = true;
-                float mx = 0.0f, sum = 0.0f;
-#pragma unroll
-                for (int j = 0; j < kHeld; ++j) {
-                    const int g8 = tid + j * NT;
-                    const int q0 = kQuads ? tid + 2 * j * NT : 2 * g8, q1 = kQuads ? q0 + NT : q0 + 1;   // its quads
-                    if (vec_ok) {
-                        float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
-                        if (q0 * 4 < p.K) a = ld_after_wait(reinterpret_cast<const float4 *>(p.act) + q0);
-                        if (q1 * 4 < p.K) b = ld_after_wait(reinterpret_cast<const float4 *>(p.act) + q1);
-                        hv[j][0] = a.x; hv[j][1] = a.y; hv[j][2] = a.z; hv[j][3] = a.w;
-                        hv[j][4] = b.x; hv[j][5] = b.y; hv[j][6] = b.z; hv[j][7] = b.w;
-                    } else {
-#pragma unroll
-                        for (int q = 0; q < 8; ++q) {
-                            const int k = (q < 4 ? q0 : q1) * 4 + (q & 3);
-                            hv[j][q] = k < p.K ? ld_after_wait(p.act + k) : 0.0f;
-                        }
-                    }
-                }
-#pragma unroll
-                for (int j = 0; j < kHeld; ++j)
-#pragma unroll
-                    for (int q = 0; q < 8; ++q) {
-                        mx = fmaxf(mx, fabsf(hv[j][q]));
-                        if (!kQuads) sum += hv[j][q];
-                        if (kQuads && (q & 3) == 3) sum += (hv[j][q - 3] + hv[j][q - 2]) + (hv[j][q - 1] + hv[j][q]);
-                    }
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) {
-                    mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, o));
-                    sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
-                }
-                if (lane == 0) {
-                    s_part[warp * 2] = mx;
-                    s_part[warp * 2 + 1] = sum;
-                }
+                if constexpr (kCanHold) frag::hold_row<NT, kHeld, kQuads>(p.act, p.K, vec_ok, hv, s_part);
             } else {
                 frag::scan_rows<NT, MULTI ? 4 : 1>(p.act, p.M, p.K, vec_ok, s_part, s_mx, s_rs);
             }
@@ -431,15 +393,8 @@ qmm_mma8_kernel(P8 p) {
                 }
             }
         } else if (kCanHold && held) {
-            // every thread folds the warps' partials itself, in the same fixed order: one barrier and a broadcast
-            // less than handing the result round
-            float bm = 0.0f, bs = 0.0f;
-#pragma unroll
-            for (int w = 0; w < NW; ++w) {
-                const float2 part = *reinterpret_cast<const float2 *>(s_part + w * 2);
-                bm = fmaxf(bm, part.x);
-                bs += part.y;
-            }
+            float bm, bs;
+            frag::fold_held<NT>(s_part, bm, bs);
             const float dq0 = (bm > 0.0f && isfinite(bm)) ? bm / 16256.0f : 1.0f;
             if (tid == 0) {   // (published by the barrier below, for the epilogue)
                 s_dq[0] = dq0;

@@ -679,24 +679,8 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
                 finish_chunk<KIND, T>(r, fac, scale, zero, bias, p.bias != nullptr, p.acc_scale, p.epilogue, v);
                 const int m0 = mt * p.Mb + c0;
                 const int jmax = n_ok ? min(W, min(p.Mb - c0, p.M - m0)) : 0;   // rows of this chunk that exist
-                if (p.ag.world == 0) {   // a warp writes 32 consecutive n
-                    float *dst = p.out + (size_t)m0 * p.N + n;
-#pragma unroll
-                    for (int j = 0; j < W; ++j)
-                        if (j < jmax) dst[(size_t)j * p.N] = v[j];
-                    if (p.sum) {   // the sums beside them, eight loads in flight together
-                        const float *ad = p.add + (size_t)m0 * p.N + n;
-                        float *sm = p.sum + (size_t)m0 * p.N + n;
-#pragma unroll
-                        for (int h = 0; h < W; h += 8) {
-                            float x[8];
-#pragma unroll
-                            for (int j = 0; j < 8; ++j) x[j] = h + j < jmax ? ld_after_wait(ad + (size_t)(h + j) * p.N) : 0.0f;
-#pragma unroll
-                            for (int j = 0; j < 8; ++j)
-                                if (h + j < jmax) sm[(size_t)(h + j) * p.N] = __fadd_rn(v[h + j], x[j]);
-                        }
-                    }
+                if (p.ag.world == 0) {
+                    store_chunk(p.out, p.add, p.sum, (size_t)m0 * p.N + n, p.N, jmax, v);
                 } else {   // plain peer stores over NVLink (and one local store)
                     const size_t at = (size_t)m0 * p.ag.n_total + p.ag.col0 + n;
                     for (int rk = 0; rk < p.ag.world; ++rk) {

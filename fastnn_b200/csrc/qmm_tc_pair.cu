@@ -363,23 +363,7 @@ qmm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                 finish_chunk<KIND, T>(r, fac, scale, zero, bias, p.bias != nullptr, p.acc_scale, p.epilogue, v);
                 const int m0 = mt * p.Mb + c0;
                 const int jmax = n_ok ? min(16, min(p.Mb - c0, p.M - m0)) : 0;   // rows of this chunk that exist
-                float *dst = p.out + (size_t)m0 * p.N + n;   // a warp writes 32 consecutive n
-#pragma unroll
-                for (int j = 0; j < 16; ++j)
-                    if (j < jmax) dst[(size_t)j * p.N] = v[j];
-                if (p.sum) {   // the sums beside them, eight loads in flight together
-                    const float *ad = p.add + (size_t)m0 * p.N + n;
-                    float *sm = p.sum + (size_t)m0 * p.N + n;
-#pragma unroll
-                    for (int h = 0; h < 16; h += 8) {
-                        float x[8];
-#pragma unroll
-                        for (int j = 0; j < 8; ++j) x[j] = h + j < jmax ? ld_after_wait(ad + (size_t)(h + j) * p.N) : 0.0f;
-#pragma unroll
-                        for (int j = 0; j < 8; ++j)
-                            if (h + j < jmax) sm[(size_t)(h + j) * p.N] = __fadd_rn(v[h + j], x[j]);
-                    }
-                }
+                store_chunk(p.out, p.add, p.sum, (size_t)m0 * p.N + n, p.N, jmax, v);
                 fac = fac_next;
             }
             tc_fence_before();

@@ -232,6 +232,26 @@ __host__ __device__ constexpr uint32_t make_idesc(int kind, int n_cols, int a_fm
 // generic-proxy writes to shared memory -> visible to the async proxy (the tensor core's reads)
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
+// One chunk of outputs: `rows` batch rows of one channel, `pitch` apart from `at` on (a warp writes 32 consecutive channels), and
+// where `sum` is given the sums with `add` beside them, eight loads in flight together.
+template <int W>
+__device__ __forceinline__ void store_chunk(float *out, const float *add, float *sum, size_t at, size_t pitch, int rows,
+                                            const float (&v)[W]) {
+#pragma unroll
+    for (int j = 0; j < W; ++j)
+        if (j < rows) out[at + (size_t)j * pitch] = v[j];
+    if (!sum) return;
+#pragma unroll
+    for (int h = 0; h < W; h += 8) {
+        float x[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) x[j] = h + j < rows ? ld_after_wait(add + at + (size_t)(h + j) * pitch) : 0.0f;
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+            if (h + j < rows) sum[at + (size_t)(h + j) * pitch] = __fadd_rn(v[h + j], x[j]);
+    }
+}
+
 // The epilogue arithmetic of one chunk: W batch rows (8 or 16) of one output channel.  `fac` carries the
 // rows' dq (lanes 0 .. W-1) and row sums (lanes 16 ..).  One branch per chunk, on the activation, behind the arithmetic that
 // all of them share: a branch per output ran the two warps of a scheduler one after another, and a copy of the whole
