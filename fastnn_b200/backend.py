@@ -303,7 +303,8 @@ class CudaBackend:
     def dispatch_profile(self, plan: ExecutablePlan, arena: CudaBuffer,
                          shape_env: ShapeEnv) -> List[ProfileEntry]:
         """Per-instruction device time from CUDA events (the trait default wall-clocks each
-        one-instruction plan, src/backend/mod.rs:178-211, which would time only the launch)."""
+        one-instruction plan, src/backend/mod.rs:178-211, which would time only the launch).  Every instruction runs by
+        itself here: an addition that ``dispatch`` takes into the MatMul before it is an entry of its own."""
         entries = []
         ms = ctypes.c_float()
         for i, instr in enumerate(plan.instructions):

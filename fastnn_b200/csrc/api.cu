@@ -506,12 +506,15 @@ static int qmatmul_impl(fnn_cuda_ctx *ctx, fnn_cuda_qweight *w, const float *a, 
         // quarter of the SMs), the codebook format the 8-bit fragment kernel up to 8 (12): there the tcgen05 kernel's
         // operands are narrower.  The other formats are as exact on the tcgen05 kernel, whose time does not depend
         // on the number of rows below 16; us fragment / tcgen05:
-        //   I8   K=4096 N=11008  M=4 12.8 / 12.2, M=8 13.8 / 12.1;  K=11008 N=4096 M=4 13.5 / 13.9, M=8 16.1 / 14.0;
-        //        K=1024 N=2048 M=8 5.0 / 5.4 (5 rows on, from 8 MB of weights)
-        //   FP4  K=8192 N=28672 (117 MB) M=1 30.4 / 30.8, M=2 32.1 / 30.4, M=4 36.5 / 31.4, M=8 43.5 / 31.4;
-        //        K=4096 N=11008 (22 MB) M=3 11.1 / 10.4;  K=4096 N=4096 (8 MB) M=2 6.9 / 8.4, M=4 7.4 / 8.5, M=8 8.6 / 8.7
-        //   I4   K=4096 N=4096 M=8 7.6 / 8.0, N=28672 18.3 / 19.3;  K=8192 N=8192 M=8 16.9 / 13.0, K=14336 N=4096 M=4
-        //        17.5 / 14.2: where the staged rows no longer fit beside the ring
+        //   I8   from 5 rows on, from 8 MB of weights: K=4096 N=11008 M=4 12.3 / 11.9, M=8 13.6 / 12.0;  K=11008 N=4096 M=4
+        //        13.7 / 13.8, M=8 16.3 / 14.0;  below 8 MB K=1024 N=2048 M=8 6.1 / 6.5
+        //   FP4  K=8192 N=28672 (117 MB) M=1 25.9 / 29.3, M=2 28.9 / 29.5, M=4 30.1 / 29.6, M=8 44.4 / 30.2;
+        //        K=4096 N=11008 (22 MB) M=3 9.5 / 10.6;  K=4096 N=4096 (8 MB) M=2 6.3 / 8.3, M=4 7.4 / 8.3, M=8 7.4 / 8.3
+        //   I4   K=4096 N=4096 M=8 6.6 / 8.2, N=28672 18.4 / 21.2;  K=8192 N=8192 M=8 18.0 / 14.0: where the staged rows no
+        //        longer fit beside the ring
+        // The lines were drawn before the fragment kernel's rows came by bulk copies.  By these figures FP4 would stay on it longer
+        // (2 rows at 117 MB, 3 at 22, 8 at 8) and I4 would too with few long rows (K=14336 N=4096 M=4 13.5 / 14.8), but leave it
+        // earlier in between (M=8 K=6144 N=4096 10.2 / 9.1, K=4096 N=14336 12.2 / 10.6).
         {
             const bool frag_ok = qmm_mma_supported(w, M) && auto_uses_mma(w);
             const size_t tiles128 = div_ceil(w->N, (size_t)128);

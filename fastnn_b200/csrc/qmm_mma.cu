@@ -662,8 +662,8 @@ int launch_mma_g(fnn_cuda_ctx *ctx, const QmmArgs &a, const float *act, float *o
 // A single batch row of FP8: groups per block and blocks per SM, by the same considerations as on the 8-bit kernel (launch8_single
 // there).  us, three groups x 1 that scanned and re-read the row / one group x 1 / x 2 / two groups x 1:
 //   up to a tile per SM             K=8192 N=2048 9.77 / 6.19 / 7.57 / 7.41
-//   K up to 4096, or eight tiles    K=4096 N=4096 6.94 / 6.03 / 5.54 / 6.18, N=28672 22.6 / 23.9 / 20.9 / 21.4;
-//   per SM                          K=8192 N=28672 40.4 / 42.9 / 37.7 / 38.3
+//   K up to 4096, and up to 8192    K=4096 N=4096 6.94 / 6.03 / 5.54 / 6.18, N=28672 22.6 / 23.9 / 20.9 / 21.4;
+//   from eight tiles per SM on      K=8192 N=28672 40.4 / 42.9 / 37.7 / 38.3
 //   longer                          K=8192 N=8192 16.1 / 15.8 / 14.3 / 13.9, K=11008 N=4096 12.6 / 12.3 / 11.9 / 10.8
 template <int FMT>
 int launch_mma_single(fnn_cuda_ctx *ctx, const QmmArgs &a, const float *act, float *out) {
@@ -681,8 +681,8 @@ int launch_mma_single(fnn_cuda_ctx *ctx, const QmmArgs &a, const float *act, flo
 }
 
 // Groups per block.  Single-column-group kernels: three where every SM has many tiles, two while that still gives (nearly) every
-// SM a block, else one, so that the tiles spread over more SMs (us with three / two groups: FP8 M=4 K=8192 N=28672
-// 46.2 / 46.8, K=4096 N=11008 15.2 / 12.7, M=3 K=2048 N=8192 8.3 / 7.4).  More columns: what the registers allow.
+// SM a block, else one, so that the tiles spread over more SMs (us with three / two groups, FP8 M=4: K=8192 N=28672
+// 46.2 / 46.8, K=3072 N=16384 13.0 / 13.0, K=4096 N=13001 16.2 / 13.8, N=11008 15.0 / 12.7, M=3 K=2048 N=8192 8.3 / 7.4).  More columns: what the registers allow.
 template <int FMT, int CG>
 int launch_mma(fnn_cuda_ctx *ctx, const QmmArgs &a, const float *act, float *out, int M, int split) {
     if constexpr (CG == 1) {

@@ -170,11 +170,14 @@ act_prep_kernel(const float *act, int M, int K, int Kp, uint8_t *bq, float *dq, 
 // N=4096 M=64 14.3 / 12.0; four decoder layers at 64 rows 300.2 / 298.2.
 constexpr int kPrepHold = 16;   // units of eight elements a thread can hold
 // HOLD: 2, 4, 8 or 16 units, the smallest that covers the row: fewer registers (more rows at once on an SM, and room
-// beside the main kernel before it) and less code to fetch, which a kernel of two microseconds notices.
+// beside the main kernel before it) and less code to fetch, which a kernel of two microseconds notices.  From four units on the
+// bound of one block per SM lets the compiler spend registers on loads in flight (64, 106 and 190 instead of 58, 80 and 152: I4
+// M=64 K=14336 N=4096 18.0 us instead of 20.1).
 // VEC: rows of a multiple of four elements that start on 16 bytes (every layer of a real model); else 4-byte loads.
 // LEAN: 32 registers a thread instead of 40.  With a few rows the blocks then fit beside the fragment kernels' 512 threads of 112,
-// which leave 8192, and start before those end (I4 M=8 K=4096 N=6144 9.7 -> 8.2 us, N=22528 18.1 -> 15.4); from 33 rows on the
-// wider form is a little faster (four I4 decoder layers at 64 rows 302.0 lean, 299.1).
+// which leave 8192, and start before those end (I4 M=8 K=4096 N=6144 9.7 -> 8.2 us, N=22528 18.1 -> 15.4); between 16 and 48
+// rows the two differ by less than 1.1 % either way, and at 64 the wider form is a little faster (four I4 decoder layers 302.0
+// lean, 299.1).
 template <int KIND, int T, bool PERM8, int HOLD, bool VEC, bool LEAN>
 __global__ void __launch_bounds__(256, LEAN ? 8 : 1)
 act_prep_regs_kernel(const float *act, int M, int K, int Kp, uint8_t *bq, float *dq, float *rowsum) {

@@ -46,8 +46,7 @@ def test_sum_and_result_are_those_of_two_calls(backend, fmt, m, k, n):
                                                         4 * sum_at, m * n) == 0
             return np.frombuffer(backend.read_arena(arena, 0, 4 * end), np.uint32).copy()
 
-        # a slice of its own; in place of the residual, of the result, of the activations (where they are large enough),
-        # and half over the residual
+        # a slice of its own; in place of the residual, of the result, of the activations (where they are large enough)
         for sum_at in (total, add, out) + ((a,) if k >= n else ()):
             assert (run(True, sum_at) == run(False, sum_at)).all(), sum_at
     finally:
