@@ -901,7 +901,10 @@ int split_parts(const fnn_cuda_ctx *ctx, int tiles, int kblocks, int cols, int w
     int best = 1;
     double best_cost = waves * kblocks * t_step;
     for (int q = 2; q <= 6 && q <= kblocks; ++q) {
-        if (tiles > kActive[q] * ctx->sm_count / 148) break;
+        // (the codebook kernel's 832 threads leave no room beside them: with the last two clusters of three taken a call waits for the
+        // SMs that the rewrite is on, M=48 K=2944 N=5732 14.1 us in three parts, 11.3 in two)
+        const int spare = wf == WF_CB && q == 3 ? 2 : 0;
+        if (tiles > (kActive[q] - spare) * ctx->sm_count / 148) break;
         const bool crowded = 4 * tiles * q > 3 * ctx->sm_count;
         const double cost = (kblocks + q - 1) / q * t_step + t_part * (q - 1) + (crowded ? 1.5 : 0.0);
         if (cost < best_cost) {

@@ -66,3 +66,20 @@ def test_kernel_and_result(backend, fmt, k, n, m, kernel):
         assert np.array_equal(rig.run(x, bias, L.EPI_NONE), got)
     finally:
         rig.close()
+
+
+# codebook tiles on both sides of the number that runs as clusters of three
+@pytest.mark.parametrize("n", [5500, 5504, 5505, 5700, 5769])
+def test_codebook_tiles_around_the_clusters_of_three(backend, n):
+    k, m = 2944, 48
+    q = codes(orc.FMT_I4CB, k, n, 1100)
+    x, bias = normal(1101, (m, k), 1.0), normal(1102, (n,), 0.01)
+    rig = Rig(backend, q, m)
+    try:
+        got = rig.run(x, bias, L.EPI_NONE, L.PATH_TC)
+        backend.synchronize()
+        for lo, hi in ((0, 130), (n - 150, n)):
+            err = max_err_vs_rms(got[:, lo:hi], orc.qmatmul(columns(q, lo, hi), x, bias[lo:hi], L.EPI_NONE))
+            assert err <= TOL_TC, (lo, err)
+    finally:
+        rig.close()
